@@ -1,6 +1,6 @@
 // Batched in-place 3D FFT building blocks on [nt][n0][n1][n2] complex64 grids: one
 // kernel per axis, built on the team engine of fft.cuh (unnormalised, DIR = -1 forward,
-// +1 inverse).  Used by the NUFFT's fine grid.
+// +1 inverse).  Used by the Toeplitz diagonal and the circulant preconditioner.
 //
 //   fft_lines_contig   : lines along the contiguous axis (n2); a team of S lanes loads
 //                        its line directly (S consecutive values per load).

@@ -1,6 +1,6 @@
 // Host launchers of the batched 3D FFT (fft3_kernels.cuh) on [nt][n0][n1][n2] complex64
-// grids, in place, for every team length the library compiles; shared by the NUFFT and
-// the circulant preconditioner.
+// grids, in place, for the lengths of images and doubled grids; shared by the Toeplitz diagonal
+// and the circulant preconditioner.  (The NUFFT's fine grid has its own passes.)
 #pragma once
 
 #include <cuda_runtime.h>
@@ -82,7 +82,6 @@ cudaError_t contig_any(int L, float2* d, long long nlines, const float2* tw, cud
     case 160: return lines_contig<160, DIR>(d, nlines, tw, st, kind);
     case 192: return lines_contig<192, DIR>(d, nlines, tw, st, kind);
     case 320: return lines_contig<320, DIR>(d, nlines, tw, st, kind);
-    case 512: return lines_contig<512, DIR>(d, nlines, tw, st, kind);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -101,7 +100,6 @@ cudaError_t strided_any(int L, float2* d, long long rs, int ncols, int ny, long 
     case 160: return lines_strided<160, DIR>(d, rs, ncols, ny, oy, nz, oz, tw, st, kind);
     case 192: return lines_strided<192, DIR>(d, rs, ncols, ny, oy, nz, oz, tw, st, kind);
     case 320: return lines_strided<320, DIR>(d, rs, ncols, ny, oy, nz, oz, tw, st, kind);
-    case 512: return lines_strided<512, DIR>(d, rs, ncols, ny, oy, nz, oz, tw, st, kind);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -12,6 +12,7 @@
 #include "../../include/hasty_b200.h"
 #include "fft3_launch.cuh"
 #include "nufft_kernels.cuh"
+#include "nufft_pass_kernels.cuh"
 #include "runtime.cuh"
 
 using namespace hb;
@@ -22,22 +23,16 @@ using hb::fftl::team_tables;
 struct hb_nufft {
   int device;
   NufftGeom g;
-  int maxbatch;
+  int group;                // transforms interleaved in the grid at once: 1, 2, 4 or 8
   float* coords = nullptr;  // [3][K] (a copy)
   int* perm = nullptr;      // [K] samples in bin order
   float* corr = nullptr;    // [N0 | N1 | N2] 1 / phi_hat
   float2* tw = nullptr;     // team twiddle tables of n0, n1, n2 (offsets 0, n0, n0 + n1)
-  float2* grid = nullptr;   // [maxbatch][n0][n1][n2]
-  float2* modes = nullptr;  // [maxbatch][N0][N1][N2] (SENSE temporaries)
-  float2* kbuf = nullptr;   // [maxbatch][K] (SENSE normal temporaries)
+  float2* grid = nullptr;   // [n0][n1][n2][group]
+  float2* kbuf = nullptr;   // [group][K] (SENSE normal temporaries)
 };
 
 namespace {
-
-template <int DIR>
-cudaError_t fft3(const hb_nufft* p, float2* grid, int nt, cudaStream_t st) {
-  return fft3_grid<DIR>(p->g.n[0], p->g.n[1], p->g.n[2], p->tw, grid, nt, st);
-}
 
 // Kernel width for a requested tolerance (upsampling 2): w = ceil(log10(1/tol)) + 1.
 int width_for_tol(double tol) {
@@ -88,22 +83,36 @@ double phi_hat(int k, int n, int w, double beta) {
   return 2.0 * 0.5 * hw * acc;
 }
 
+// Transforms of one group: nact <= NB = 1 << lgnb interleaved grids.  Sizes that are not a
+// power of two are padded, except 5, which runs as 4 + 1 (padding it to 8 moves 1.6 times the
+// bytes); at 3, 6 and 7 the padding costs at most a third and saves a second set of launches.
+struct Group {
+  int nact, lgnb;
+};
+Group next_group(const hb_nufft* p, int64_t left) {
+  int n = (int)(left < p->group ? left : p->group);
+  if (n == 5) n = 4;
+  return {n, n > 4 ? 3 : n > 2 ? 2 : n - 1};
+}
+
 template <int W>
-cudaError_t spread_w(const hb_nufft* p, const float2* c, long long c_ld, int nb, cudaStream_t st) {
-  dim3 grid((unsigned)((p->g.K + 255) / 256), nb);
+cudaError_t spread_w(const hb_nufft* p, const float2* c, long long c_ld, Group q, float csgn, cudaStream_t st) {
+  const unsigned grid = (unsigned)(((p->g.K << q.lgnb) + 255) / 256);
   LaunchScope ls(HB_KERNEL_NUFFT, st);
-  if (p->g.dim == 3) nufft_spread_kernel<W, 3><<<grid, 256, 0, st>>>(p->g, p->coords, p->perm, c, c_ld, p->grid);
-  else if (p->g.dim == 2) nufft_spread_kernel<W, 2><<<grid, 256, 0, st>>>(p->g, p->coords, p->perm, c, c_ld, p->grid);
-  else nufft_spread_kernel<W, 1><<<grid, 256, 0, st>>>(p->g, p->coords, p->perm, c, c_ld, p->grid);
+  auto go = [&](auto kernel) { kernel<<<grid, 256, 0, st>>>(p->g, p->coords, p->perm, c, c_ld, q.lgnb, q.nact, csgn, p->grid); };
+  if (p->g.dim == 3) go(nufft_spread_kernel<W, 3>);
+  else if (p->g.dim == 2) go(nufft_spread_kernel<W, 2>);
+  else go(nufft_spread_kernel<W, 1>);
   return cudaGetLastError();
 }
 template <int W>
-cudaError_t interp_w(const hb_nufft* p, float2* c, long long c_ld, int nb, cudaStream_t st) {
-  dim3 grid((unsigned)((p->g.K + 255) / 256), nb);
+cudaError_t interp_w(const hb_nufft* p, float2* c, long long c_ld, Group q, float csgn, cudaStream_t st) {
+  const unsigned grid = (unsigned)(((p->g.K << q.lgnb) + 255) / 256);
   LaunchScope ls(HB_KERNEL_NUFFT, st);
-  if (p->g.dim == 3) nufft_interp_kernel<W, 3><<<grid, 256, 0, st>>>(p->g, p->coords, p->perm, p->grid, c, c_ld);
-  else if (p->g.dim == 2) nufft_interp_kernel<W, 2><<<grid, 256, 0, st>>>(p->g, p->coords, p->perm, p->grid, c, c_ld);
-  else nufft_interp_kernel<W, 1><<<grid, 256, 0, st>>>(p->g, p->coords, p->perm, p->grid, c, c_ld);
+  auto go = [&](auto kernel) { kernel<<<grid, 256, 0, st>>>(p->g, p->coords, p->perm, p->grid, q.lgnb, q.nact, csgn, c, c_ld); };
+  if (p->g.dim == 3) go(nufft_interp_kernel<W, 3>);
+  else if (p->g.dim == 2) go(nufft_interp_kernel<W, 2>);
+  else go(nufft_interp_kernel<W, 1>);
   return cudaGetLastError();
 }
 
@@ -120,44 +129,110 @@ cudaError_t interp_w(const hb_nufft* p, float2* c, long long c_ld, int nb, cudaS
     default: return cudaErrorInvalidValue;                                                           \
   }
 
-cudaError_t spread(const hb_nufft* p, const float2* c, long long c_ld, int nb, cudaStream_t st) {
-  HB_W_DISPATCH(spread_w, p, c, c_ld, nb, st)
+cudaError_t spread(const hb_nufft* p, const float2* c, long long c_ld, Group q, float csgn, cudaStream_t st) {
+  HB_W_DISPATCH(spread_w, p, c, c_ld, q, csgn, st)
 }
-cudaError_t interp(const hb_nufft* p, float2* c, long long c_ld, int nb, cudaStream_t st) {
-  HB_W_DISPATCH(interp_w, p, c, c_ld, nb, st)
+cudaError_t interp(const hb_nufft* p, float2* c, long long c_ld, Group q, float csgn, cudaStream_t st) {
+  HB_W_DISPATCH(interp_w, p, c, c_ld, q, csgn, st)
 }
 
 long long nmodes(const hb_nufft* p) { return (long long)p->g.N[0] * p->g.N[1] * p->g.N[2]; }
 long long nfine(const hb_nufft* p) { return (long long)p->g.n[0] * p->g.n[1] * p->g.n[2]; }
 
-// nb <= maxbatch transforms: c [nb][K] (row pitch c_ld) -> f [nb][modes] (row pitch f_ld)
-int type1_batch(const hb_nufft* p, const float2* c, long long c_ld, float2* f, long long f_ld, int nb, int isign,
-                cudaStream_t st) {
-  HB_CUDA(cudaMemsetAsync(p->grid, 0, (size_t)nb * nfine(p) * sizeof(float2), st));
-  HB_CUDA(spread(p, c, c_ld, nb, st));
-  HB_CUDA(isign > 0 ? fft3<1>(p, p->grid, nb, st) : fft3<-1>(p, p->grid, nb, st));
-  dim3 grid((unsigned)((nmodes(p) + 255) / 256), nb);
-  {
-    LaunchScope ls(HB_KERNEL_NUFFT, st);
-    nufft_deconv_kernel<<<grid, 256, 0, st>>>(p->g, p->grid, p->corr, f, f_ld);
+// ---- fine-grid passes (nufft_pass_kernels.cuh); axis twiddles at tw + {0, n0, n0 + n1} ----
+template <int L, bool PAD>
+cudaError_t axis_pass_l(const hb_nufft* p, int axis, int lgnb, cudaStream_t st) {
+  using C = TilePassCfg<L>;
+  constexpr size_t smem = C::SMEM * sizeof(float2);
+  cudaError_t e = hb::fftl::allow_smem<nufft_axis_pass_kernel<L, PAD>>(smem);
+  if (e != cudaSuccess) return e;
+  const NufftGeom& g = p->g;
+  LaunchScope ls(HB_KERNEL_NUFFT, st);
+  if (axis == 0) {  // z: every (y, x) column
+    const long long ncols = (long long)g.n[1] * g.n[2] << lgnb;
+    nufft_axis_pass_kernel<L, PAD><<<dim3((unsigned)((ncols + 15) / 16), 1), C::THREADS, smem, st>>>(
+        p->grid, ncols, (int)ncols, 1, 1, 0, p->tw);
+  } else {  // y: the kept z planes
+    const int ncols = g.n[2] << lgnb;
+    nufft_axis_pass_kernel<L, PAD><<<dim3((ncols + 15) / 16, g.N[0]), C::THREADS, smem, st>>>(
+        p->grid, ncols, ncols, g.N[0], g.n[0], (long long)ncols * L, p->tw + g.n[0]);
   }
-  HB_CHECK_LAUNCH();
+  return cudaGetLastError();
+}
+// to_grid: modes -> grid (type 2), else grid -> modes (type 1)
+template <int L>
+cudaError_t mode_pass_l(const hb_nufft* p, const NufftModeOp& op, Group q, float sgn, bool to_grid, cudaStream_t st) {
+  using C = TilePassCfg<L>;
+  constexpr size_t smem = C::SMEM * sizeof(float2);
+  const NufftGeom& g = p->g;
+  const int nl = 16 >> q.lgnb;
+  const unsigned grid = (unsigned)((g.N[0] * g.N[1] + nl - 1) / nl);
+  const float2* tw = p->tw + g.n[0] + g.n[1];
+  cudaError_t e;
+  if (to_grid) {
+    if ((e = hb::fftl::allow_smem<nufft_modes_to_grid_kernel<L>>(smem)) != cudaSuccess) return e;
+    LaunchScope ls(HB_KERNEL_NUFFT, st);
+    nufft_modes_to_grid_kernel<L><<<grid, C::THREADS, smem, st>>>(g, op, q.lgnb, q.nact, sgn, p->corr, tw, p->grid);
+  } else {
+    if ((e = hb::fftl::allow_smem<nufft_grid_to_modes_kernel<L>>(smem)) != cudaSuccess) return e;
+    LaunchScope ls(HB_KERNEL_NUFFT, st);
+    nufft_grid_to_modes_kernel<L><<<grid, C::THREADS, smem, st>>>(g, op, q.lgnb, q.nact, sgn, p->corr, tw, p->grid);
+  }
+  return cudaGetLastError();
+}
+
+#define HB_L_DISPATCH(n, CALL)                                                        \
+  switch (n) {                                                                        \
+    case 8: { constexpr int L = 8; return CALL; }     case 16: { constexpr int L = 16; return CALL; }   \
+    case 32: { constexpr int L = 32; return CALL; }   case 64: { constexpr int L = 64; return CALL; }   \
+    case 128: { constexpr int L = 128; return CALL; } case 256: { constexpr int L = 256; return CALL; } \
+    case 512: { constexpr int L = 512; return CALL; } case 96: { constexpr int L = 96; return CALL; }   \
+    case 160: { constexpr int L = 160; return CALL; } case 192: { constexpr int L = 192; return CALL; } \
+    case 320: { constexpr int L = 320; return CALL; }                                 \
+    default: return cudaErrorInvalidValue;                                            \
+  }
+cudaError_t axis_pass(const hb_nufft* p, int axis, bool pad, int lgnb, cudaStream_t st) {
+  if (p->g.n[axis] == 1) return cudaSuccess;  // a degenerate axis of a 1-D or 2-D plan
+  HB_L_DISPATCH(p->g.n[axis], (pad ? axis_pass_l<L, true>(p, axis, lgnb, st) : axis_pass_l<L, false>(p, axis, lgnb, st)))
+}
+cudaError_t mode_pass(const hb_nufft* p, const NufftModeOp& op, Group q, float sgn, bool to_grid, cudaStream_t st) {
+  HB_L_DISPATCH(p->g.n[2], (mode_pass_l<L>(p, op, q, sgn, to_grid, st)))
+}
+
+// One group of transforms: c [nact][K] (row pitch c_ld) -> modes (op)
+int type1_group(const hb_nufft* p, const float2* c, long long c_ld, const NufftModeOp& op, Group q, int isign,
+                cudaStream_t st) {
+  const float sgn = isign > 0 ? -1.f : 1.f;  // the passes transform forward
+  HB_CUDA(cudaMemsetAsync(p->grid, 0, ((size_t)nfine(p) << q.lgnb) * sizeof(float2), st));
+  HB_CUDA(spread(p, c, c_ld, q, sgn, st));
+  HB_CUDA(axis_pass(p, 0, false, q.lgnb, st));
+  HB_CUDA(axis_pass(p, 1, false, q.lgnb, st));
+  HB_CUDA(mode_pass(p, op, q, sgn, false, st));
   return HB_OK;
 }
 
-// nb <= maxbatch transforms: f [nb][modes] -> c [nb][K]
-int type2_batch(const hb_nufft* p, const float2* f, long long f_ld, float2* c, long long c_ld, int nb, int isign,
+// One group of transforms: modes (op) -> c [nact][K]
+int type2_group(const hb_nufft* p, const NufftModeOp& op, float2* c, long long c_ld, Group q, int isign,
                 cudaStream_t st) {
-  HB_CUDA(cudaMemsetAsync(p->grid, 0, (size_t)nb * nfine(p) * sizeof(float2), st));
-  dim3 grid((unsigned)((nmodes(p) + 255) / 256), nb);
-  {
-    LaunchScope ls(HB_KERNEL_NUFFT, st);
-    nufft_precorrect_kernel<<<grid, 256, 0, st>>>(p->g, f, f_ld, p->corr, p->grid);
-  }
-  HB_CHECK_LAUNCH();
-  HB_CUDA(isign > 0 ? fft3<1>(p, p->grid, nb, st) : fft3<-1>(p, p->grid, nb, st));
-  HB_CUDA(interp(p, c, c_ld, nb, st));
+  const float sgn = isign > 0 ? -1.f : 1.f;
+  HB_CUDA(mode_pass(p, op, q, sgn, true, st));
+  HB_CUDA(axis_pass(p, 1, true, q.lgnb, st));
+  HB_CUDA(axis_pass(p, 0, true, q.lgnb, st));
+  HB_CUDA(interp(p, c, c_ld, q, sgn, st));
   return HB_OK;
+}
+
+NufftModeOp plain_modes(const float2* f, long long f_ld) {
+  NufftModeOp op{};
+  op.f = const_cast<float2*>(f);
+  op.f_ld = f_ld;
+  return op;
+}
+// Coil form of the mode side for coils [b0, b0 + n)
+NufftModeOp coil_modes(const void* smaps, const int64_t* coils, int64_t b0, int n, long long nm) {
+  NufftModeOp op{};
+  for (int b = 0; b < n; ++b) op.maps.s[b] = (const float2*)smaps + coils[b0 + b] * nm;
+  return op;
 }
 
 void free_plan(hb_nufft* p) {
@@ -167,7 +242,6 @@ void free_plan(hb_nufft* p) {
   cudaFree(p->corr);
   cudaFree(p->tw);
   cudaFree(p->grid);
-  cudaFree(p->modes);
   cudaFree(p->kbuf);
   delete p;
 }
@@ -182,19 +256,20 @@ int nufft_psf_circulant(const int* M, const float* coords, int64_t nsamples, dou
   hb_nufft* np = nullptr;
   // type 1 over the grid's modes: sum_j exp(+i c_j . d), d in [-M/2, M/2)
   if (int r = hb_nufft_create(&np, M[0], M[1], M[2], coords, nsamples, tol, 1, device, st)) return r;
-  float2* ones = nullptr;
+  float2 *ones = nullptr, *modes = nullptr;
   int rc = HB_OK;
   cudaError_t e = cudaMalloc(&ones, nsamples * sizeof(float2));
+  if (e == cudaSuccess) e = cudaMalloc(&modes, vol * sizeof(float2));
   if (e == cudaSuccess) {
     {
       LaunchScope ls(HB_KERNEL_DIAG, st);
       fill_c64_kernel<<<(unsigned)((nsamples + 255) / 256), 256, 0, st>>>(ones, nsamples, make_float2(1.f, 0.f),
                                                                           weights);
     }
-    rc = type1_batch(np, ones, nsamples, np->modes, vol, 1, +1, st);
+    rc = type1_group(np, ones, nsamples, plain_modes(modes, vol), {1, 0}, +1, st);
     if (rc == HB_OK) {
       LaunchScope ls(HB_KERNEL_DIAG, st);
-      ifftshift3_scale_kernel<<<(unsigned)((vol + 255) / 256), 256, 0, st>>>(np->modes, M[0], M[1], M[2],
+      ifftshift3_scale_kernel<<<(unsigned)((vol + 255) / 256), 256, 0, st>>>(modes, M[0], M[1], M[2],
                                                                              (float)(1.0 / (double)vol), out);
     }
     if (rc == HB_OK && (e = cudaGetLastError()) != cudaSuccess)
@@ -206,6 +281,7 @@ int nufft_psf_circulant(const int* M, const float* coords, int64_t nsamples, dou
   }
   if (rc != HB_OK) cudaStreamSynchronize(st);
   cudaFree(ones);
+  cudaFree(modes);
   hb_nufft_destroy(np);
   return rc;
 }
@@ -251,10 +327,9 @@ int hb_nufft_create(hb_nufft** out, int64_t nz, int64_t ny, int64_t nx, const fl
   hb_nufft* p = new hb_nufft();
   p->device = device;
   p->g = g;
-  p->maxbatch = maxbatch;
+  p->group = maxbatch > 4 ? 8 : maxbatch > 2 ? 4 : maxbatch;
   const long long nbins = (long long)g.nb[0] * g.nb[1] * g.nb[2];
   const long long vol = (long long)g.n[0] * g.n[1] * g.n[2];
-  const long long nm = (long long)g.N[0] * g.N[1] * g.N[2];
   int* bin_of = nullptr;
   int* counts = nullptr;
   auto bail = [&](cudaError_t e, const char* what) {
@@ -268,9 +343,8 @@ int hb_nufft_create(hb_nufft** out, int64_t nz, int64_t ny, int64_t nx, const fl
   if ((e = cudaMalloc(&p->perm, nsamples * sizeof(int))) != cudaSuccess) return bail(e, "perm");
   if ((e = cudaMalloc(&p->corr, (g.N[0] + g.N[1] + g.N[2]) * sizeof(float))) != cudaSuccess) return bail(e, "corr");
   if ((e = cudaMalloc(&p->tw, (g.n[0] + g.n[1] + g.n[2]) * sizeof(float2))) != cudaSuccess) return bail(e, "tables");
-  if ((e = cudaMalloc(&p->grid, (size_t)maxbatch * vol * sizeof(float2))) != cudaSuccess) return bail(e, "fine grid");
-  if ((e = cudaMalloc(&p->modes, (size_t)maxbatch * nm * sizeof(float2))) != cudaSuccess) return bail(e, "modes");
-  if ((e = cudaMalloc(&p->kbuf, (size_t)maxbatch * nsamples * sizeof(float2))) != cudaSuccess) return bail(e, "kbuf");
+  if ((e = cudaMalloc(&p->grid, (size_t)p->group * vol * sizeof(float2))) != cudaSuccess) return bail(e, "fine grid");
+  if ((e = cudaMalloc(&p->kbuf, (size_t)p->group * nsamples * sizeof(float2))) != cudaSuccess) return bail(e, "kbuf");
   if ((e = cudaMalloc(&bin_of, nsamples * sizeof(int))) != cudaSuccess) return bail(e, "bins");
   if ((e = cudaMalloc(&counts, 2 * nbins * sizeof(int))) != cudaSuccess) return bail(e, "bins");
 
@@ -328,11 +402,12 @@ int hb_nufft_type1(const hb_nufft* plan, const void* c, void* f, int64_t ntransf
     return fail(HB_ERR_INVALID, "hb_nufft_type1: null argument, negative ntransf or isign not +-1");
   DeviceGuard dg(plan->device);
   const long long K = plan->g.K, nm = nmodes(plan);
-  for (int64_t t0 = 0; t0 < ntransf; t0 += plan->maxbatch) {
-    const int nb = (int)((ntransf - t0) < plan->maxbatch ? (ntransf - t0) : plan->maxbatch);
-    if (int r = type1_batch(plan, (const float2*)c + t0 * K, K, (float2*)f + t0 * nm, nm, nb, isign,
+  for (int64_t t0 = 0; t0 < ntransf;) {
+    const Group q = next_group(plan, ntransf - t0);
+    if (int r = type1_group(plan, (const float2*)c + t0 * K, K, plain_modes((const float2*)f + t0 * nm, nm), q, isign,
                             (cudaStream_t)stream))
       return r;
+    t0 += q.nact;
   }
   return HB_OK;
 }
@@ -342,11 +417,12 @@ int hb_nufft_type2(const hb_nufft* plan, const void* f, void* c, int64_t ntransf
     return fail(HB_ERR_INVALID, "hb_nufft_type2: null argument, negative ntransf or isign not +-1");
   DeviceGuard dg(plan->device);
   const long long K = plan->g.K, nm = nmodes(plan);
-  for (int64_t t0 = 0; t0 < ntransf; t0 += plan->maxbatch) {
-    const int nb = (int)((ntransf - t0) < plan->maxbatch ? (ntransf - t0) : plan->maxbatch);
-    if (int r = type2_batch(plan, (const float2*)f + t0 * nm, nm, (float2*)c + t0 * K, K, nb, isign,
+  for (int64_t t0 = 0; t0 < ntransf;) {
+    const Group q = next_group(plan, ntransf - t0);
+    if (int r = type2_group(plan, plain_modes((const float2*)f + t0 * nm, nm), (float2*)c + t0 * K, K, q, isign,
                             (cudaStream_t)stream))
       return r;
+    t0 += q.nact;
   }
   return HB_OK;
 }
@@ -360,10 +436,11 @@ int hb_sense_adjoint_nufft(const hb_nufft* plan, const void* kdata, const void* 
   DeviceGuard dg(plan->device);
   cudaStream_t st = (cudaStream_t)stream;
   const long long K = plan->g.K, nm = nmodes(plan);
-  const unsigned vb = (unsigned)((nm + 255) / 256), kb = (unsigned)((K + 255) / 256);
+  const unsigned kb = (unsigned)((K + 255) / 256);
   if (ncoil == 0 && !accumulate) HB_CUDA(cudaMemsetAsync(out, 0, nm * sizeof(float2), st));
-  for (int64_t b0 = 0; b0 < ncoil; b0 += plan->maxbatch) {
-    const int nb = (int)((ncoil - b0) < plan->maxbatch ? (ncoil - b0) : plan->maxbatch);
+  for (int64_t b0 = 0; b0 < ncoil;) {
+    const Group q = next_group(plan, ncoil - b0);
+    const int nb = q.nact;
     const float2* src = (const float2*)kdata + b0 * K;
     if (weights) {  // w * kdata rows into the plan's k-space temporaries
       KdataPtrs ys{};
@@ -375,15 +452,11 @@ int hb_sense_adjoint_nufft(const hb_nufft* plan, const void* kdata, const void* 
       HB_CHECK_LAUNCH();
       src = plan->kbuf;
     }
-    if (int r = type1_batch(plan, src, K, plan->modes, nm, nb, +1, st)) return r;
-    CoilMaps maps{};
-    for (int b = 0; b < nb; ++b) maps.s[b] = (const float2*)smaps + coils[b0 + b] * nm;
-    {
-      LaunchScope ls(HB_KERNEL_NUFFT, st);
-      sense_coil_combine_kernel<<<vb, 256, 0, st>>>(plan->modes, nb, nm, maps, (float2*)out,
-                                                    (b0 > 0 || accumulate) ? 1 : 0);
-    }
-    HB_CHECK_LAUNCH();
+    NufftModeOp op = coil_modes(smaps, coils, b0, nb, nm);
+    op.out = (float2*)out;
+    op.accumulate = (b0 > 0 || accumulate) ? 1 : 0;
+    if (int r = type1_group(plan, src, K, op, q, +1, st)) return r;
+    b0 += nb;
   }
   return HB_OK;
 }
@@ -397,17 +470,13 @@ int hb_sense_forward_nufft(const hb_nufft* plan, const void* x, const void* smap
   DeviceGuard dg(plan->device);
   cudaStream_t st = (cudaStream_t)stream;
   const long long K = plan->g.K, nm = nmodes(plan);
-  const unsigned vb = (unsigned)((nm + 255) / 256);
-  for (int64_t b0 = 0; b0 < ncoil; b0 += plan->maxbatch) {
-    const int nb = (int)((ncoil - b0) < plan->maxbatch ? (ncoil - b0) : plan->maxbatch);
-    CoilMaps maps{};
-    for (int b = 0; b < nb; ++b) maps.s[b] = (const float2*)smaps + coils[b0 + b] * nm;
-    {
-      LaunchScope ls(HB_KERNEL_NUFFT, st);
-      sense_coil_expand_kernel<<<vb, 256, 0, st>>>((const float2*)x, nb, nm, maps, plan->modes);
-    }
-    HB_CHECK_LAUNCH();
-    if (int r = type2_batch(plan, plan->modes, nm, (float2*)kdata + b0 * K, K, nb, -1, st)) return r;
+  for (int64_t b0 = 0; b0 < ncoil;) {
+    const Group q = next_group(plan, ncoil - b0);
+    const int nb = q.nact;
+    NufftModeOp op = coil_modes(smaps, coils, b0, nb, nm);
+    op.x = (const float2*)x;
+    if (int r = type2_group(plan, op, (float2*)kdata + b0 * K, K, q, -1, st)) return r;
+    b0 += nb;
   }
   return HB_OK;
 }
@@ -421,34 +490,25 @@ int hb_sense_normal_nufft(const hb_nufft* plan, const void* x, const void* smaps
   DeviceGuard dg(plan->device);
   cudaStream_t st = (cudaStream_t)stream;
   const long long K = plan->g.K, nm = nmodes(plan);
-  const unsigned vb = (unsigned)((nm + 255) / 256), kb = (unsigned)((K + 255) / 256);
+  const unsigned kb = (unsigned)((K + 255) / 256);
   if (ncoil == 0 && !accumulate) HB_CUDA(cudaMemsetAsync(out, 0, nm * sizeof(float2), st));
-  for (int64_t b0 = 0; b0 < ncoil; b0 += plan->maxbatch) {
-    const int nb = (int)((ncoil - b0) < plan->maxbatch ? (ncoil - b0) : plan->maxbatch);
-    CoilMaps maps{};
+  for (int64_t b0 = 0; b0 < ncoil;) {
+    const Group q = next_group(plan, ncoil - b0);
+    const int nb = q.nact;
     KdataPtrs ys{};
-    for (int b = 0; b < nb; ++b) {
-      maps.s[b] = (const float2*)smaps + coils[b0 + b] * nm;
-      ys.y[b] = kdata ? (const float2*)kdata + coils[b0 + b] * K : nullptr;
-    }
-    {
-      LaunchScope ls(HB_KERNEL_NUFFT, st);
-      sense_coil_expand_kernel<<<vb, 256, 0, st>>>((const float2*)x, nb, nm, maps, plan->modes);
-    }
-    HB_CHECK_LAUNCH();
-    if (int r = type2_batch(plan, plan->modes, nm, plan->kbuf, K, nb, -1, st)) return r;
+    for (int b = 0; b < nb; ++b) ys.y[b] = kdata ? (const float2*)kdata + coils[b0 + b] * K : nullptr;
+    NufftModeOp op = coil_modes(smaps, coils, b0, nb, nm);
+    op.x = (const float2*)x;
+    op.out = (float2*)out;
+    op.accumulate = (b0 > 0 || accumulate) ? 1 : 0;
+    if (int r = type2_group(plan, op, plan->kbuf, K, q, -1, st)) return r;
     if (kdata || weights) {
       LaunchScope ls(HB_KERNEL_NUFFT, st);
       sense_kspace_mid_kernel<<<kb, 256, 0, st>>>(plan->kbuf, nb, K, ys, weights);
     }
     HB_CHECK_LAUNCH();
-    if (int r = type1_batch(plan, plan->kbuf, K, plan->modes, nm, nb, +1, st)) return r;
-    {
-      LaunchScope ls(HB_KERNEL_NUFFT, st);
-      sense_coil_combine_kernel<<<vb, 256, 0, st>>>(plan->modes, nb, nm, maps, (float2*)out,
-                                                    (b0 > 0 || accumulate) ? 1 : 0);
-    }
-    HB_CHECK_LAUNCH();
+    if (int r = type1_group(plan, plan->kbuf, K, op, q, +1, st)) return r;
+    b0 += nb;
   }
   return HB_OK;
 }

@@ -123,61 +123,67 @@ __device__ __forceinline__ int nufft_axis(const NufftGeom& g, const float* coord
   }
 }
 
-// ---- type 1: spread (grid pre-zeroed); grid y = transform within the batch ----
+// ---- type 1: spread into a zeroed grid [n0][n1][n2][NB], NB = 1 << lgnb interleaved
+// transforms; one thread per (sample, transform), transform fastest; csgn = -1 conjugates c ----
 template <int W, int DIM>
 __global__ void __launch_bounds__(256) nufft_spread_kernel(NufftGeom g, const float* coords, const int* perm,
-                                                           const float2* c, long long c_ld, float2* grid) {
+                                                           const float2* c, long long c_ld, int lgnb, int nact,
+                                                           float csgn, float2* grid) {
   constexpr int W0 = DIM >= 3 ? W : 1, W1 = DIM >= 2 ? W : 1;
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= g.K) return;
+  const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int bt = (int)(id & ((1 << lgnb) - 1));
+  const long long i = id >> lgnb;
+  if (i >= g.K || bt >= nact) return;
   const int j = perm[i];
-  const float2 cj = c[(long long)blockIdx.y * c_ld + j];
+  float2 cj = c[bt * c_ld + j];
+  cj.y *= csgn;
   float w0[W0], w1[W1], w2[W];
   const int i0 = nufft_axis<W, W0>(g, coords, 0, j, w0);
   const int i1 = nufft_axis<W, W1>(g, coords, 1, j, w1);
   const int i2 = nufft_axis<W, W>(g, coords, 2, j, w2);
-  float2* G = grid + (long long)blockIdx.y * g.n[0] * g.n[1] * g.n[2];
   int x2[W];
 #pragma unroll
-  for (int m = 0; m < W; ++m) x2[m] = wrap(i2 + m, g.n[2]);
+  for (int m = 0; m < W; ++m) x2[m] = wrap(i2 + m, g.n[2]) << lgnb;
 #pragma unroll 1
   for (int a = 0; a < W0; ++a) {
     const float2 ca = cscale(cj, w0[a]);
-    float2* Ga = G + (long long)wrap(i0 + a, g.n[0]) * g.n[1] * g.n[2];
+    float2* Ga = grid + ((long long)wrap(i0 + a, g.n[0]) * g.n[1] * g.n[2] << lgnb) + bt;
 #pragma unroll
     for (int b = 0; b < W1; ++b) {
       const float2 cab = cscale(ca, w1[b]);
-      float2* Gab = Ga + (long long)wrap(i1 + b, g.n[1]) * g.n[2];
+      float2* Gab = Ga + ((long long)wrap(i1 + b, g.n[1]) * g.n[2] << lgnb);
 #pragma unroll
       for (int m = 0; m < W; ++m) red_add(Gab + x2[m], cscale(cab, w2[m]));
     }
   }
 }
 
-// ---- type 2: interpolate ----
+// ---- type 2: interpolate (same thread mapping; csgn = -1 conjugates the result) ----
 template <int W, int DIM>
 __global__ void __launch_bounds__(256) nufft_interp_kernel(NufftGeom g, const float* coords, const int* perm,
-                                                           const float2* grid, float2* c, long long c_ld) {
+                                                           const float2* grid, int lgnb, int nact, float csgn,
+                                                           float2* c, long long c_ld) {
   constexpr int W0 = DIM >= 3 ? W : 1, W1 = DIM >= 2 ? W : 1;
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= g.K) return;
+  const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int bt = (int)(id & ((1 << lgnb) - 1));
+  const long long i = id >> lgnb;
+  if (i >= g.K || bt >= nact) return;
   const int j = perm[i];
   float w0[W0], w1[W1], w2[W];
   const int i0 = nufft_axis<W, W0>(g, coords, 0, j, w0);
   const int i1 = nufft_axis<W, W1>(g, coords, 1, j, w1);
   const int i2 = nufft_axis<W, W>(g, coords, 2, j, w2);
-  const float2* G = grid + (long long)blockIdx.y * g.n[0] * g.n[1] * g.n[2];
   int x2[W];
 #pragma unroll
-  for (int m = 0; m < W; ++m) x2[m] = wrap(i2 + m, g.n[2]);
+  for (int m = 0; m < W; ++m) x2[m] = wrap(i2 + m, g.n[2]) << lgnb;
   float2 acc = make_float2(0.f, 0.f);
 #pragma unroll 1
   for (int a = 0; a < W0; ++a) {
-    const float2* Ga = G + (long long)wrap(i0 + a, g.n[0]) * g.n[1] * g.n[2];
+    const float2* Ga = grid + ((long long)wrap(i0 + a, g.n[0]) * g.n[1] * g.n[2] << lgnb) + bt;
     float2 sa = make_float2(0.f, 0.f);
 #pragma unroll
     for (int b = 0; b < W1; ++b) {
-      const float2* Gab = Ga + (long long)wrap(i1 + b, g.n[1]) * g.n[2];
+      const float2* Gab = Ga + ((long long)wrap(i1 + b, g.n[1]) * g.n[2] << lgnb);
       float2 sb = make_float2(0.f, 0.f);
 #pragma unroll
       for (int m = 0; m < W; ++m) {
@@ -191,40 +197,8 @@ __global__ void __launch_bounds__(256) nufft_interp_kernel(NufftGeom g, const fl
     acc.x = fmaf(w0[a], sa.x, acc.x);
     acc.y = fmaf(w0[a], sa.y, acc.y);
   }
-  c[(long long)blockIdx.y * c_ld + j] = acc;
-}
-
-// ---- mode <-> fine-grid maps with the kernel correction 1/phi_hat (corr: [N0 | N1 | N2]) ----
-__device__ __forceinline__ long long nufft_mode_cell(const NufftGeom& g, long long m, float* scale,
-                                                     const float* corr) {
-  const int i2 = (int)(m % g.N[2]);
-  const int i1 = (int)((m / g.N[2]) % g.N[1]);
-  const int i0 = (int)(m / ((long long)g.N[2] * g.N[1]));
-  const int k0 = i0 - g.N[0] / 2, k1 = i1 - g.N[1] / 2, k2 = i2 - g.N[2] / 2;
-  *scale = corr[i0] * corr[g.N[0] + i1] * corr[g.N[0] + g.N[1] + i2];
-  const int c0 = k0 < 0 ? k0 + g.n[0] : k0, c1 = k1 < 0 ? k1 + g.n[1] : k1, c2 = k2 < 0 ? k2 + g.n[2] : k2;
-  return ((long long)c0 * g.n[1] + c1) * g.n[2] + c2;
-}
-
-// type 1: f[t][mode] = grid[t][cell(mode)] / phi_hat(mode)
-__global__ void nufft_deconv_kernel(NufftGeom g, const float2* grid, const float* corr, float2* f, long long f_ld) {
-  const long long nm = (long long)g.N[0] * g.N[1] * g.N[2];
-  const long long m = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= nm) return;
-  float s;
-  const long long cell = nufft_mode_cell(g, m, &s, corr);
-  const float2 v = grid[(long long)blockIdx.y * g.n[0] * g.n[1] * g.n[2] + cell];
-  f[(long long)blockIdx.y * f_ld + m] = cscale(v, s);
-}
-
-// type 2: grid[t][cell(mode)] = f[t][mode] / phi_hat(mode)  (grid pre-zeroed)
-__global__ void nufft_precorrect_kernel(NufftGeom g, const float2* f, long long f_ld, const float* corr, float2* grid) {
-  const long long nm = (long long)g.N[0] * g.N[1] * g.N[2];
-  const long long m = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= nm) return;
-  float s;
-  const long long cell = nufft_mode_cell(g, m, &s, corr);
-  grid[(long long)blockIdx.y * g.n[0] * g.n[1] * g.n[2] + cell] = cscale(f[(long long)blockIdx.y * f_ld + m], s);
+  acc.y *= csgn;
+  c[bt * c_ld + j] = acc;
 }
 
 // ---- Toeplitz diagonal through the NUFFT ----
@@ -246,25 +220,16 @@ __global__ void ifftshift3_scale_kernel(const float2* in, int M0, int M1, int M2
 }
 
 // ---- SENSE around the NUFFT ----
-constexpr int kNufftMaxBatch = 32;  // transforms per batch (coil-map pointers by value)
-struct CoilMaps {
-  const float2* s[kNufftMaxBatch];
+constexpr int kNufftMaxBatch = 32;  // largest maxbatch of a plan
+constexpr int kNufftGroup = 8;      // transforms interleaved in one grid
+struct CoilMaps {  // coil-map pointers by value
+  const float2* s[kNufftGroup];
 };
-
-// out (+)= sum_b conj(S_b) * f[b]   (f: [nb][nvox]); accumulate = 0 overwrites
-__global__ void sense_coil_combine_kernel(const float2* f, int nb, long long nvox, CoilMaps maps, float2* out,
-                                          int accumulate) {
-  const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= nvox) return;
-  float2 acc = accumulate ? out[v] : make_float2(0.f, 0.f);
-  for (int b = 0; b < nb; ++b) acc = cadd(acc, cmulc(f[b * nvox + v], maps.s[b][v]));
-  out[v] = acc;
-}
 
 // k-space step of the SENSE normal operator (the reference's mid-appliers):
 // k[b][j] = (k[b][j] - y_b[j]) * w[j]  (y_b and w nullable)
 struct KdataPtrs {
-  const float2* y[kNufftMaxBatch];
+  const float2* y[kNufftGroup];
 };
 __global__ void sense_kspace_mid_kernel(float2* k, int nb, long long K, KdataPtrs y, const float* w) {
   const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -283,14 +248,6 @@ __global__ void sense_kspace_weight_kernel(float2* k, int nb, long long K, Kdata
   if (j >= K) return;
   const float wj = w[j];
   for (int b = 0; b < nb; ++b) k[b * K + j] = cscale(y.y[b][j], wj);
-}
-
-// f[b] = S_b * x
-__global__ void sense_coil_expand_kernel(const float2* x, int nb, long long nvox, CoilMaps maps, float2* f) {
-  const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= nvox) return;
-  const float2 xv = x[v];
-  for (int b = 0; b < nb; ++b) f[b * nvox + v] = cmul(xv, maps.s[b][v]);
 }
 
 }  // namespace hb

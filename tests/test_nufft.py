@@ -200,3 +200,22 @@ def test_diagonal_through_the_nufft_rejects_unsupported_grids(cuda, shape):
     with pytest.raises(capi.HastyError) as e:
         plan.build_diagonal(coords, method="nufft")
     assert e.value.code == capi.HB_ERR_UNSUPPORTED
+
+
+@pytest.mark.parametrize("shape,nt", [((256, 8, 8), 1), ((8, 256, 8), 3), ((8, 8, 256), 5), ((160, 8, 16), 2),
+                                      ((48, 80, 8), 7), ((96, 8, 48), 9), ((80, 96), 6), ((128, 32), 8), ((160,), 4)])
+def test_every_pass_length_and_group_of_transforms(cuda, shape, nt):
+    """Each compiled line length on each axis, and batches that fill, pad and split the interleaved
+    groups (1, 2, 4, 8; 5 = 4 + 1).  Bound: 10 x tol plus the worst phase error of a float32 grid
+    position, pi/2 * n * 1.5 * 2^-24 at the highest mode."""
+    d, K = len(shape), 400
+    bound = 1e-5 + 1.41e-7 * 2 * max(shape)
+    rng = np.random.default_rng(29)
+    coords = rng.uniform(-np.pi, np.pi, (d, K)).astype(np.float32)
+    plan = NufftPlan(torch.from_numpy(coords).to(cuda), shape, tol=1e-6, maxbatch=min(nt, 8))
+    c, fm = _rand((nt, K), 30), _rand((nt,) + shape, 31)
+    for sign in (+1, -1):
+        f, ref = _np(plan.type1(_c64(c, cuda), isign=sign)), O.nudft_type1(coords, c, shape, sign)
+        y, ref2 = _np(plan.type2(_c64(fm, cuda), isign=sign)), O.nudft_type2(coords, fm, sign)
+        for t in range(nt):
+            assert O.rel_l2(f[t], ref[t]) < bound and O.rel_l2(y[t], ref2[t]) < bound
