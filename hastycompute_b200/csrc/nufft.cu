@@ -13,6 +13,7 @@
 #include "fft3_launch.cuh"
 #include "nufft_kernels.cuh"
 #include "nufft_pass_kernels.cuh"
+#include "nufft_spread_kernels.cuh"
 #include "runtime.cuh"
 
 using namespace hb;
@@ -24,12 +25,18 @@ struct hb_nufft {
   int device;
   NufftGeom g;
   int group;                // transforms interleaved in the grid at once: 1, 2, 4 or 8
-  float* coords = nullptr;  // [3][K] (a copy)
-  int* perm = nullptr;      // [K] samples in bin order
-  float* corr = nullptr;    // [N0 | N1 | N2] 1 / phi_hat
-  float2* tw = nullptr;     // team twiddle tables of n0, n1, n2 (offsets 0, n0, n0 + n1)
-  float2* grid = nullptr;   // [n0][n1][n2][group]
-  float2* kbuf = nullptr;   // [group][K] (SENSE normal temporaries)
+  void* mem = nullptr;        // one allocation: the arrays below up to vals
+  float4* pts = nullptr;      // [K] grid positions and sample numbers in bin order
+  int* start = nullptr;       // [bins + 1] first position of every bin
+  float* corr = nullptr;      // [N0 | N1 | N2] 1 / phi_hat
+  float2* tw = nullptr;       // team twiddle tables of n0, n1, n2 (offsets 0, n0, n0 + n1)
+  float2* grid = nullptr;     // [n0][n1][n2][group]
+  float2* vals = nullptr;     // [K][group] values to spread, in sorted order
+  // spreading (2-D and 3-D): pieces of tile work and the tiles cut into several
+  void* items_mem = nullptr;
+  SpreadItem* items = nullptr;
+  int* split_tiles = nullptr;
+  int nitems = 0, nsplit = 0;
 };
 
 namespace {
@@ -96,23 +103,46 @@ Group next_group(const hb_nufft* p, int64_t left) {
 }
 
 template <int W>
-cudaError_t spread_w(const hb_nufft* p, const float2* c, long long c_ld, Group q, float csgn, cudaStream_t st) {
+cudaError_t spread_reductions_w(const hb_nufft* p, Group q, cudaStream_t st) {
   const unsigned grid = (unsigned)(((p->g.K << q.lgnb) + 255) / 256);
   LaunchScope ls(HB_KERNEL_NUFFT, st);
-  auto go = [&](auto kernel) { kernel<<<grid, 256, 0, st>>>(p->g, p->coords, p->perm, c, c_ld, q.lgnb, q.nact, csgn, p->grid); };
-  if (p->g.dim == 3) go(nufft_spread_kernel<W, 3>);
-  else if (p->g.dim == 2) go(nufft_spread_kernel<W, 2>);
-  else go(nufft_spread_kernel<W, 1>);
+  if (p->g.dim == 3) nufft_spread_reductions_kernel<W, 3><<<grid, 256, 0, st>>>(p->g, p->pts, p->vals, q.lgnb, p->grid);
+  else nufft_spread_reductions_kernel<W, 1><<<grid, 256, 0, st>>>(p->g, p->pts, p->vals, q.lgnb, p->grid);
   return cudaGetLastError();
 }
 template <int W>
-cudaError_t interp_w(const hb_nufft* p, float2* c, long long c_ld, Group q, float csgn, cudaStream_t st) {
+cudaError_t interp_w(const hb_nufft* p, const InterpDest& dst, Group q, float csgn, cudaStream_t st) {
   const unsigned grid = (unsigned)(((p->g.K << q.lgnb) + 255) / 256);
   LaunchScope ls(HB_KERNEL_NUFFT, st);
-  auto go = [&](auto kernel) { kernel<<<grid, 256, 0, st>>>(p->g, p->coords, p->perm, p->grid, q.lgnb, q.nact, csgn, c, c_ld); };
+  auto go = [&](auto kernel) { kernel<<<grid, 256, 0, st>>>(p->g, p->pts, p->grid, q.lgnb, q.nact, csgn, dst); };
   if (p->g.dim == 3) go(nufft_interp_kernel<W, 3>);
   else if (p->g.dim == 2) go(nufft_interp_kernel<W, 2>);
   else go(nufft_interp_kernel<W, 1>);
+  return cudaGetLastError();
+}
+
+// p->vals = the values to spread
+cudaError_t gather_values(const hb_nufft* p, const SpreadSource& src, Group q, float csgn, cudaStream_t st) {
+  const unsigned grid = (unsigned)(((p->g.K << q.lgnb) + 255) / 256);
+  LaunchScope ls(HB_KERNEL_NUFFT, st);
+  nufft_gather_values_kernel<<<grid, 256, 0, st>>>(p->g.K, p->pts, src, q.lgnb, q.nact, csgn, p->vals);
+  return cudaGetLastError();
+}
+
+template <int DIM>
+cudaError_t spread_tiles(const hb_nufft* p, Group q, cudaStream_t st) {
+  if (p->nsplit > 0) {
+    LaunchScope ls(HB_KERNEL_NUFFT, st);
+    nufft_zero_tiles_kernel<DIM><<<p->nsplit, 128, 0, st>>>(p->g, p->split_tiles, q.lgnb, p->grid);
+  }
+  LaunchScope ls(HB_KERNEL_NUFFT, st);
+  auto go = [&](auto kernel) {
+    kernel<<<p->nitems, 32, 0, st>>>(p->g, p->pts, p->start, p->items, p->vals, p->grid);
+  };
+  if (q.lgnb == 3) go(nufft_spread_tiles_kernel<DIM, 8>);
+  else if (q.lgnb == 2) go(nufft_spread_tiles_kernel<DIM, 4>);
+  else if (q.lgnb == 1) go(nufft_spread_tiles_kernel<DIM, 2>);
+  else go(nufft_spread_tiles_kernel<DIM, 1>);
   return cudaGetLastError();
 }
 
@@ -129,11 +159,11 @@ cudaError_t interp_w(const hb_nufft* p, float2* c, long long c_ld, Group q, floa
     default: return cudaErrorInvalidValue;                                                           \
   }
 
-cudaError_t spread(const hb_nufft* p, const float2* c, long long c_ld, Group q, float csgn, cudaStream_t st) {
-  HB_W_DISPATCH(spread_w, p, c, c_ld, q, csgn, st)
+cudaError_t spread_reductions(const hb_nufft* p, Group q, cudaStream_t st) {
+  HB_W_DISPATCH(spread_reductions_w, p, q, st)
 }
-cudaError_t interp(const hb_nufft* p, float2* c, long long c_ld, Group q, float csgn, cudaStream_t st) {
-  HB_W_DISPATCH(interp_w, p, c, c_ld, q, csgn, st)
+cudaError_t interp(const hb_nufft* p, const InterpDest& dst, Group q, float csgn, cudaStream_t st) {
+  HB_W_DISPATCH(interp_w, p, dst, q, csgn, st)
 }
 
 long long nmodes(const hb_nufft* p) { return (long long)p->g.N[0] * p->g.N[1] * p->g.N[2]; }
@@ -199,27 +229,44 @@ cudaError_t mode_pass(const hb_nufft* p, const NufftModeOp& op, Group q, float s
   HB_L_DISPATCH(p->g.n[2], (mode_pass_l<L>(p, op, q, sgn, to_grid, st)))
 }
 
-// One group of transforms: c [nact][K] (row pitch c_ld) -> modes (op)
-int type1_group(const hb_nufft* p, const float2* c, long long c_ld, const NufftModeOp& op, Group q, int isign,
-                cudaStream_t st) {
-  const float sgn = isign > 0 ? -1.f : 1.f;  // the passes transform forward
-  HB_CUDA(cudaMemsetAsync(p->grid, 0, ((size_t)nfine(p) << q.lgnb) * sizeof(float2), st));
-  HB_CUDA(spread(p, c, c_ld, q, sgn, st));
-  HB_CUDA(axis_pass(p, 0, false, q.lgnb, st));
-  HB_CUDA(axis_pass(p, 1, false, q.lgnb, st));
-  HB_CUDA(mode_pass(p, op, q, sgn, false, st));
-  return HB_OK;
+// The passes transform forward; the other sign conjugates what enters and leaves the chain.
+float conj_sign(int isign) { return isign > 0 ? -1.f : 1.f; }
+
+// The whole grid = the spread values p->vals
+cudaError_t spread(const hb_nufft* p, Group q, cudaStream_t st) {
+  if (p->nitems > 0) return p->g.dim == 3 ? spread_tiles<3>(p, q, st) : spread_tiles<2>(p, q, st);
+  cudaError_t e = cudaMemsetAsync(p->grid, 0, ((size_t)nfine(p) << q.lgnb) * sizeof(float2), st);
+  return e != cudaSuccess ? e : spread_reductions(p, q, st);
 }
 
-// One group of transforms: modes (op) -> c [nact][K]
-int type2_group(const hb_nufft* p, const NufftModeOp& op, float2* c, long long c_ld, Group q, int isign,
-                cudaStream_t st) {
-  const float sgn = isign > 0 ? -1.f : 1.f;
+// One group of transforms: p->vals (already conjugated for isign) -> modes (op)
+int type1_from_vals(const hb_nufft* p, const NufftModeOp& op, Group q, int isign, cudaStream_t st) {
+  HB_CUDA(spread(p, q, st));
+  HB_CUDA(axis_pass(p, 0, false, q.lgnb, st));
+  HB_CUDA(axis_pass(p, 1, false, q.lgnb, st));
+  HB_CUDA(mode_pass(p, op, q, conj_sign(isign), false, st));
+  return HB_OK;
+}
+// One group of transforms: samples (src) -> modes (op)
+int type1_group(const hb_nufft* p, const SpreadSource& src, const NufftModeOp& op, Group q, int isign, cudaStream_t st) {
+  HB_CUDA(gather_values(p, src, q, conj_sign(isign), st));
+  return type1_from_vals(p, op, q, isign, st);
+}
+
+// One group of transforms: modes (op) -> samples (dst)
+int type2_group(const hb_nufft* p, const NufftModeOp& op, const InterpDest& dst, Group q, int isign, cudaStream_t st) {
+  const float sgn = conj_sign(isign);
   HB_CUDA(mode_pass(p, op, q, sgn, true, st));
   HB_CUDA(axis_pass(p, 1, true, q.lgnb, st));
   HB_CUDA(axis_pass(p, 0, true, q.lgnb, st));
-  HB_CUDA(interp(p, c, c_ld, q, sgn, st));
+  HB_CUDA(interp(p, dst, q, sgn, st));
   return HB_OK;
+}
+InterpDest rows_dest(float2* c, long long c_ld) {
+  InterpDest d{};
+  d.c = c;
+  d.c_ld = c_ld;
+  return d;
 }
 
 NufftModeOp plain_modes(const float2* f, long long f_ld) {
@@ -237,61 +284,14 @@ NufftModeOp coil_modes(const void* smaps, const int64_t* coils, int64_t b0, int 
 
 void free_plan(hb_nufft* p) {
   if (!p) return;
-  cudaFree(p->coords);
-  cudaFree(p->perm);
-  cudaFree(p->corr);
-  cudaFree(p->tw);
-  cudaFree(p->grid);
-  cudaFree(p->kbuf);
+  cudaFree(p->mem);
+  cudaFree(p->items_mem);
   delete p;
 }
 
-}  // namespace
-
-namespace hb {
-
-int nufft_psf_circulant(const int* M, const float* coords, int64_t nsamples, double tol, const float* weights,
-                        int device, float2* out, cudaStream_t st) {
-  const long long vol = (long long)M[0] * M[1] * M[2];
-  hb_nufft* np = nullptr;
-  // type 1 over the grid's modes: sum_j exp(+i c_j . d), d in [-M/2, M/2)
-  if (int r = hb_nufft_create(&np, M[0], M[1], M[2], coords, nsamples, tol, 1, device, st)) return r;
-  float2 *ones = nullptr, *modes = nullptr;
-  int rc = HB_OK;
-  cudaError_t e = cudaMalloc(&ones, nsamples * sizeof(float2));
-  if (e == cudaSuccess) e = cudaMalloc(&modes, vol * sizeof(float2));
-  if (e == cudaSuccess) {
-    {
-      LaunchScope ls(HB_KERNEL_DIAG, st);
-      fill_c64_kernel<<<(unsigned)((nsamples + 255) / 256), 256, 0, st>>>(ones, nsamples, make_float2(1.f, 0.f),
-                                                                          weights);
-    }
-    rc = type1_group(np, ones, nsamples, plain_modes(modes, vol), {1, 0}, +1, st);
-    if (rc == HB_OK) {
-      LaunchScope ls(HB_KERNEL_DIAG, st);
-      ifftshift3_scale_kernel<<<(unsigned)((vol + 255) / 256), 256, 0, st>>>(modes, M[0], M[1], M[2],
-                                                                             (float)(1.0 / (double)vol), out);
-    }
-    if (rc == HB_OK && (e = cudaGetLastError()) != cudaSuccess)
-      rc = fail(HB_ERR_CUDA, std::string("psf: ") + cudaGetErrorString(e));
-    if (rc == HB_OK && (e = cudaStreamSynchronize(st)) != cudaSuccess)
-      rc = fail(HB_ERR_CUDA, std::string("psf: ") + cudaGetErrorString(e));
-  } else {
-    rc = fail(HB_ERR_CUDA, std::string("psf: ") + cudaGetErrorString(e));
-  }
-  if (rc != HB_OK) cudaStreamSynchronize(st);
-  cudaFree(ones);
-  cudaFree(modes);
-  hb_nufft_destroy(np);
-  return rc;
-}
-
-}  // namespace hb
-
-extern "C" {
-
-int hb_nufft_create(hb_nufft** out, int64_t nz, int64_t ny, int64_t nx, const float* coords, int64_t nsamples,
-                    double tol, int maxbatch, int device, void* stream) {
+// hb_nufft_create; tiles = false leaves out the tile work lists (spread by reductions only)
+int create_plan(hb_nufft** out, int64_t nz, int64_t ny, int64_t nx, const float* coords, int64_t nsamples, double tol,
+                int maxbatch, int device, void* stream, bool tiles) {
   if (!out) return fail(HB_ERR_INVALID, "hb_nufft_create: null output");
   *out = nullptr;
   if (!coords || nsamples < 1 || nsamples > (int64_t)0x7fffffff)
@@ -308,7 +308,7 @@ int hb_nufft_create(hb_nufft** out, int64_t nz, int64_t ny, int64_t nx, const fl
   g.dim = nz != 1 ? 3 : (ny != 1 ? 2 : 1);
   for (int a = 0; a < 3; ++a) {
     if (a < 3 - g.dim) {  // degenerate leading axis
-      g.N[a] = g.n[a] = g.nb[a] = 1;
+      g.N[a] = g.n[a] = g.nb[a] = g.bin[a] = 1;
       continue;
     }
     int E = 0, S = 0;
@@ -319,7 +319,8 @@ int hb_nufft_create(hb_nufft** out, int64_t nz, int64_t ny, int64_t nx, const fl
                                           "and >= 2w)");
     g.N[a] = (int)Nv[a];
     g.n[a] = (int)n;
-    g.nb[a] = (g.n[a] + kNufftBin - 1) / kNufftBin;
+    g.bin[a] = g.dim == 3 && a < 2 ? 4 : 8;  // every fine-grid length is a multiple of 8
+    g.nb[a] = g.n[a] / g.bin[a];
   }
   DeviceGuard dg(device);
   if (!dg.ok) return fail(HB_ERR_CUDA, "hb_nufft_create: cannot select device");
@@ -328,25 +329,90 @@ int hb_nufft_create(hb_nufft** out, int64_t nz, int64_t ny, int64_t nx, const fl
   p->device = device;
   p->g = g;
   p->group = maxbatch > 4 ? 8 : maxbatch > 2 ? 4 : maxbatch;
-  const long long nbins = (long long)g.nb[0] * g.nb[1] * g.nb[2];
+  const int nbins = g.nb[0] * g.nb[1] * g.nb[2];
   const long long vol = (long long)g.n[0] * g.n[1] * g.n[2];
-  int* bin_of = nullptr;
-  int* counts = nullptr;
+  const int ntiles = !tiles       ? 0
+                     : g.dim == 3 ? (g.n[0] / SpreadTile<3>::T0) * (g.n[1] / SpreadTile<3>::T1) * (g.n[2] / SpreadTile<3>::T2)
+                     : g.dim == 2 ? ((g.n[1] + SpreadTile<2>::T1 - 1) / SpreadTile<2>::T1) * (g.n[2] / SpreadTile<2>::T2)
+                                  : 0;
+  void* tmp = nullptr;
   auto bail = [&](cudaError_t e, const char* what) {
-    cudaFree(bin_of);
-    cudaFree(counts);
+    cudaFree(tmp);
     free_plan(p);
     return fail(HB_ERR_CUDA, std::string("hb_nufft_create: ") + what + ": " + cudaGetErrorString(e));
   };
+  // one allocation for the plan's arrays, one for the temporaries of the sort (a cudaMalloc
+  // and its cudaFree cost as much as the kernels between them)
+  auto carve = [&](Arena& ar) {
+    p->pts = ar.take<float4>(nsamples);
+    p->start = ar.take<int>(nbins + 1);
+    p->corr = ar.take<float>(g.N[0] + g.N[1] + g.N[2]);
+    p->tw = ar.take<float2>(g.n[0] + g.n[1] + g.n[2]);
+    p->grid = ar.take<float2>((size_t)p->group * vol);
+    p->vals = ar.take<float2>((size_t)p->group * nsamples);
+  };
+  int2* bin_rank;
+  int *counts, *sums, *candidates;
+  SpreadCounts* nwork;
+  auto carve_tmp = [&](Arena& ar) {
+    bin_rank = ar.take<int2>(nsamples);
+    counts = ar.take<int>(nbins);
+    sums = ar.take<int>((nbins + kScanBlock - 1) / kScanBlock);
+    candidates = ar.take<int>(ntiles);
+    nwork = ar.take<SpreadCounts>(1);
+  };
+  Arena size(nullptr), size_tmp(nullptr);
+  carve(size);
+  carve_tmp(size_tmp);
   cudaError_t e;
-  if ((e = cudaMalloc(&p->coords, 3 * nsamples * sizeof(float))) != cudaSuccess) return bail(e, "coords");
-  if ((e = cudaMalloc(&p->perm, nsamples * sizeof(int))) != cudaSuccess) return bail(e, "perm");
-  if ((e = cudaMalloc(&p->corr, (g.N[0] + g.N[1] + g.N[2]) * sizeof(float))) != cudaSuccess) return bail(e, "corr");
-  if ((e = cudaMalloc(&p->tw, (g.n[0] + g.n[1] + g.n[2]) * sizeof(float2))) != cudaSuccess) return bail(e, "tables");
-  if ((e = cudaMalloc(&p->grid, (size_t)p->group * vol * sizeof(float2))) != cudaSuccess) return bail(e, "fine grid");
-  if ((e = cudaMalloc(&p->kbuf, (size_t)p->group * nsamples * sizeof(float2))) != cudaSuccess) return bail(e, "kbuf");
-  if ((e = cudaMalloc(&bin_of, nsamples * sizeof(int))) != cudaSuccess) return bail(e, "bins");
-  if ((e = cudaMalloc(&counts, 2 * nbins * sizeof(int))) != cudaSuccess) return bail(e, "bins");
+  if ((e = cudaMalloc(&p->mem, size.off)) != cudaSuccess) return bail(e, "plan arrays and fine grid");
+  if ((e = cudaMalloc(&tmp, size_tmp.off)) != cudaSuccess) return bail(e, "sort temporaries");
+  Arena ar(p->mem), ar_tmp(tmp);
+  carve(ar);
+  carve_tmp(ar_tmp);
+
+  // counting sort of the samples by bin, while the host fills its tables
+  const unsigned blocks = (unsigned)((nsamples + 255) / 256);
+  if ((e = cudaMemsetAsync(counts, 0, nbins * sizeof(int), st)) != cudaSuccess) return bail(e, "memset");
+  {
+    LaunchScope ls(HB_KERNEL_NUFFT, st);
+    nufft_bin_count_kernel<<<blocks, 256, 0, st>>>(g, coords, bin_rank, counts);
+  }
+  const unsigned sb = (unsigned)((nbins + kScanBlock - 1) / kScanBlock);
+  {
+    LaunchScope ls(HB_KERNEL_NUFFT, st);
+    nufft_scan_block_kernel<<<sb, 1024, 0, st>>>(counts, p->start, sums, nbins);
+  }
+  {
+    LaunchScope ls(HB_KERNEL_NUFFT, st);
+    nufft_scan_sums_kernel<<<1, 1024, 0, st>>>(sums, (int)sb);
+  }
+  {
+    LaunchScope ls(HB_KERNEL_NUFFT, st);
+    nufft_scan_add_kernel<<<sb, 1024, 0, st>>>(counts, p->start, sums, nbins);
+  }
+  {
+    LaunchScope ls(HB_KERNEL_NUFFT, st);
+    nufft_bin_scatter_kernel<<<blocks, 256, 0, st>>>(g, coords, bin_rank, p->start, p->pts);
+  }
+  // Spreading: cut the tiles' candidates into pieces of at most `cap`, about 32 pieces per SM
+  // sub-partition over the whole plan (a sample is a candidate of up to 27 tiles of 4 x 4 x 8 or 6
+  // of 16 x 8).  Measured, 8 transforms: 64^3 modes with 524 k radial samples 632 / 555 / 542 /
+  // 551 us at cap 128 / 256 / 512 / 1024 (a piece re-adds its tile; one of 1024 is the tail), 201 x
+  // 256 samples on 128^2 modes 37 / 28 / 29 / 40 us at 32 / 64 / 128 / 256.
+  const long long per_sample = g.dim == 3 ? 27 : 6;
+  const long long want = nsamples * per_sample / (148 * 4 * 32);
+  const int cap = (int)(want < 64 ? 64 : want > 512 ? 512 : want);
+  const unsigned tb = (unsigned)((ntiles + 255) / 256);
+  if (ntiles > 0) {
+    if ((e = cudaMemsetAsync(nwork, 0, sizeof(SpreadCounts), st)) != cudaSuccess) return bail(e, "memset");
+    {
+      LaunchScope ls(HB_KERNEL_NUFFT, st);
+      if (g.dim == 3) nufft_tile_count_kernel<3><<<tb, 256, 0, st>>>(g, p->start, ntiles, cap, candidates, nwork);
+      else nufft_tile_count_kernel<2><<<tb, 256, 0, st>>>(g, p->start, ntiles, cap, candidates, nwork);
+    }
+  }
+  if ((e = cudaGetLastError()) != cudaSuccess) return bail(e, "binning");
 
   // host tables: 1/phi_hat per axis and the team twiddles of each fine-grid length
   std::vector<float> corr;
@@ -358,36 +424,74 @@ int hb_nufft_create(hb_nufft** out, int64_t nz, int64_t ny, int64_t nx, const fl
     return bail(e, "upload");
   if ((e = cudaMemcpyAsync(p->tw, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice, st)) != cudaSuccess)
     return bail(e, "upload");
-  // the caller's [dim][K] rows become the trailing rows of [3][K]; degenerate rows are 0
-  const int lead = 3 - g.dim;
-  if (lead > 0 && (e = cudaMemsetAsync(p->coords, 0, lead * nsamples * sizeof(float), st)) != cudaSuccess)
-    return bail(e, "coords copy");
-  if ((e = cudaMemcpyAsync(p->coords + lead * nsamples, coords, g.dim * nsamples * sizeof(float),
-                           cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
-    return bail(e, "coords copy");
-  // counting sort of the samples by bin
-  if ((e = cudaMemsetAsync(counts, 0, nbins * sizeof(int), st)) != cudaSuccess) return bail(e, "memset");
-  const unsigned blocks = (unsigned)((nsamples + 255) / 256);
-  {
-    LaunchScope ls(HB_KERNEL_NUFFT, st);
-    nufft_bin_count_kernel<<<blocks, 256, 0, st>>>(g, p->coords, bin_of, counts);
+  if (ntiles > 0) {
+    if ((e = cudaMemcpyAsync(&p->nitems, &nwork->items, sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(st)) != cudaSuccess)
+      return bail(e, "binning");
+    // at most every piece beyond the first of its tile belongs to a split tile
+    const int most_split = p->nitems - ntiles;
+    if ((e = cudaMalloc(&p->items_mem, p->nitems * sizeof(SpreadItem) + most_split * sizeof(int) + 16)) != cudaSuccess)
+      return bail(e, "spread items");
+    p->items = (SpreadItem*)p->items_mem;
+    p->split_tiles = (int*)(p->items + p->nitems);
+    {
+      LaunchScope ls(HB_KERNEL_NUFFT, st);
+      if (g.dim == 3)
+        nufft_tile_items_kernel<3><<<tb, 256, 0, st>>>(g, ntiles, cap, candidates, p->items, p->split_tiles, nwork);
+      else
+        nufft_tile_items_kernel<2><<<tb, 256, 0, st>>>(g, ntiles, cap, candidates, p->items, p->split_tiles, nwork);
+    }
+    if ((e = cudaGetLastError()) != cudaSuccess) return bail(e, "spread items");
+    if ((e = cudaMemcpyAsync(&p->nsplit, &nwork->split_tiles, sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
+      return bail(e, "spread items");
   }
-  {
-    LaunchScope ls(HB_KERNEL_NUFFT, st);
-    nufft_scan_kernel<<<1, 1024, 0, st>>>(counts, counts + nbins, (int)nbins);
-  }
-  {
-    LaunchScope ls(HB_KERNEL_NUFFT, st);
-    nufft_bin_scatter_kernel<<<blocks, 256, 0, st>>>(nsamples, bin_of, counts + nbins, p->perm);
-  }
-  if ((e = cudaGetLastError()) != cudaSuccess) return bail(e, "binning");
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return bail(e, "binning");
-  cudaFree(bin_of);
-  cudaFree(counts);
+  cudaFree(tmp);
   *out = p;
   return HB_OK;
 }
 
+}  // namespace
+
+namespace hb {
+
+int nufft_psf_circulant(const int* M, const float* coords, int64_t nsamples, double tol, const float* weights,
+                        int device, float2* out, cudaStream_t st) {
+  const long long vol = (long long)M[0] * M[1] * M[2];
+  hb_nufft* np = nullptr;
+  // type 1 over the grid's modes: sum_j exp(+i c_j . d), d in [-M/2, M/2)
+  if (int r = create_plan(&np, M[0], M[1], M[2], coords, nsamples, tol, 1, device, st, false)) return r;
+  float2* modes = nullptr;
+  int rc = HB_OK;
+  cudaError_t e = cudaMalloc(&modes, vol * sizeof(float2));
+  if (e == cudaSuccess) {
+    rc = type1_group(np, {nullptr, 0, weights}, plain_modes(modes, vol), {1, 0}, +1, st);
+    if (rc == HB_OK) {
+      LaunchScope ls(HB_KERNEL_DIAG, st);
+      ifftshift3_scale_kernel<<<(unsigned)((vol + 255) / 256), 256, 0, st>>>(modes, M[0], M[1], M[2],
+                                                                             (float)(1.0 / (double)vol), out);
+    }
+    if (rc == HB_OK && (e = cudaGetLastError()) != cudaSuccess)
+      rc = fail(HB_ERR_CUDA, std::string("psf: ") + cudaGetErrorString(e));
+    if (rc == HB_OK && (e = cudaStreamSynchronize(st)) != cudaSuccess)
+      rc = fail(HB_ERR_CUDA, std::string("psf: ") + cudaGetErrorString(e));
+  } else {
+    rc = fail(HB_ERR_CUDA, std::string("psf: ") + cudaGetErrorString(e));
+  }
+  if (rc != HB_OK) cudaStreamSynchronize(st);
+  cudaFree(modes);
+  hb_nufft_destroy(np);
+  return rc;
+}
+
+}  // namespace hb
+
+extern "C" {
+
+int hb_nufft_create(hb_nufft** out, int64_t nz, int64_t ny, int64_t nx, const float* coords, int64_t nsamples,
+                    double tol, int maxbatch, int device, void* stream) {
+  return create_plan(out, nz, ny, nx, coords, nsamples, tol, maxbatch, device, stream, true);
+}
 int hb_nufft_destroy(hb_nufft* plan) {
   if (!plan) return HB_OK;
   DeviceGuard dg(plan->device);
@@ -404,8 +508,8 @@ int hb_nufft_type1(const hb_nufft* plan, const void* c, void* f, int64_t ntransf
   const long long K = plan->g.K, nm = nmodes(plan);
   for (int64_t t0 = 0; t0 < ntransf;) {
     const Group q = next_group(plan, ntransf - t0);
-    if (int r = type1_group(plan, (const float2*)c + t0 * K, K, plain_modes((const float2*)f + t0 * nm, nm), q, isign,
-                            (cudaStream_t)stream))
+    if (int r = type1_group(plan, {(const float2*)c + t0 * K, K, nullptr}, plain_modes((const float2*)f + t0 * nm, nm), q,
+                            isign, (cudaStream_t)stream))
       return r;
     t0 += q.nact;
   }
@@ -419,8 +523,8 @@ int hb_nufft_type2(const hb_nufft* plan, const void* f, void* c, int64_t ntransf
   const long long K = plan->g.K, nm = nmodes(plan);
   for (int64_t t0 = 0; t0 < ntransf;) {
     const Group q = next_group(plan, ntransf - t0);
-    if (int r = type2_group(plan, plain_modes((const float2*)f + t0 * nm, nm), (float2*)c + t0 * K, K, q, isign,
-                            (cudaStream_t)stream))
+    if (int r = type2_group(plan, plain_modes((const float2*)f + t0 * nm, nm), rows_dest((float2*)c + t0 * K, K), q,
+                            isign, (cudaStream_t)stream))
       return r;
     t0 += q.nact;
   }
@@ -436,26 +540,14 @@ int hb_sense_adjoint_nufft(const hb_nufft* plan, const void* kdata, const void* 
   DeviceGuard dg(plan->device);
   cudaStream_t st = (cudaStream_t)stream;
   const long long K = plan->g.K, nm = nmodes(plan);
-  const unsigned kb = (unsigned)((K + 255) / 256);
   if (ncoil == 0 && !accumulate) HB_CUDA(cudaMemsetAsync(out, 0, nm * sizeof(float2), st));
   for (int64_t b0 = 0; b0 < ncoil;) {
     const Group q = next_group(plan, ncoil - b0);
     const int nb = q.nact;
-    const float2* src = (const float2*)kdata + b0 * K;
-    if (weights) {  // w * kdata rows into the plan's k-space temporaries
-      KdataPtrs ys{};
-      for (int b = 0; b < nb; ++b) ys.y[b] = src + b * K;
-      {
-        LaunchScope ls(HB_KERNEL_NUFFT, st);
-        sense_kspace_weight_kernel<<<kb, 256, 0, st>>>(plan->kbuf, nb, K, ys, weights);
-      }
-      HB_CHECK_LAUNCH();
-      src = plan->kbuf;
-    }
     NufftModeOp op = coil_modes(smaps, coils, b0, nb, nm);
     op.out = (float2*)out;
     op.accumulate = (b0 > 0 || accumulate) ? 1 : 0;
-    if (int r = type1_group(plan, src, K, op, q, +1, st)) return r;
+    if (int r = type1_group(plan, {(const float2*)kdata + b0 * K, K, weights}, op, q, +1, st)) return r;
     b0 += nb;
   }
   return HB_OK;
@@ -475,7 +567,7 @@ int hb_sense_forward_nufft(const hb_nufft* plan, const void* x, const void* smap
     const int nb = q.nact;
     NufftModeOp op = coil_modes(smaps, coils, b0, nb, nm);
     op.x = (const float2*)x;
-    if (int r = type2_group(plan, op, (float2*)kdata + b0 * K, K, q, -1, st)) return r;
+    if (int r = type2_group(plan, op, rows_dest((float2*)kdata + b0 * K, K), q, -1, st)) return r;
     b0 += nb;
   }
   return HB_OK;
@@ -490,24 +582,21 @@ int hb_sense_normal_nufft(const hb_nufft* plan, const void* x, const void* smaps
   DeviceGuard dg(plan->device);
   cudaStream_t st = (cudaStream_t)stream;
   const long long K = plan->g.K, nm = nmodes(plan);
-  const unsigned kb = (unsigned)((K + 255) / 256);
   if (ncoil == 0 && !accumulate) HB_CUDA(cudaMemsetAsync(out, 0, nm * sizeof(float2), st));
   for (int64_t b0 = 0; b0 < ncoil;) {
     const Group q = next_group(plan, ncoil - b0);
     const int nb = q.nact;
-    KdataPtrs ys{};
-    for (int b = 0; b < nb; ++b) ys.y[b] = kdata ? (const float2*)kdata + coils[b0 + b] * K : nullptr;
+    InterpDest mid{};
+    for (int b = 0; b < nb; ++b) mid.y[b] = kdata ? (const float2*)kdata + coils[b0 + b] * K : nullptr;
+    mid.w = weights;
+    mid.vals = plan->vals;
+    mid.vsgn = conj_sign(+1);
     NufftModeOp op = coil_modes(smaps, coils, b0, nb, nm);
     op.x = (const float2*)x;
     op.out = (float2*)out;
     op.accumulate = (b0 > 0 || accumulate) ? 1 : 0;
-    if (int r = type2_group(plan, op, plan->kbuf, K, q, -1, st)) return r;
-    if (kdata || weights) {
-      LaunchScope ls(HB_KERNEL_NUFFT, st);
-      sense_kspace_mid_kernel<<<kb, 256, 0, st>>>(plan->kbuf, nb, K, ys, weights);
-    }
-    HB_CHECK_LAUNCH();
-    if (int r = type1_group(plan, plan->kbuf, K, op, q, +1, st)) return r;
+    if (int r = type2_group(plan, op, mid, q, -1, st)) return r;
+    if (int r = type1_from_vals(plan, op, q, +1, st)) return r;
     b0 += nb;
   }
   return HB_OK;

@@ -13,17 +13,22 @@
 // beta = 2.30 w.  Type 1 = spread c_j * phi(g - u_j) onto the fine grid (u_j = x_j n/(2pi)),
 // FFT with sign isign, divide by phi_hat(k) and crop; type 2 = the transpose.
 //
-// Samples are bucketed by fine-grid bin once per plan (counting sort), so that spreading
-// (vector reductions into global memory) and interpolation (gathers) walk the grid with
-// locality.  The atomics make type 1 bitwise non-deterministic, as the reference's
-// cufinufft is.
+// Samples are bucketed by fine-grid bin once per plan (counting sort into an array of grid
+// positions), so that spreading (nufft_spread_kernels.cuh) finds the samples near a tile and
+// interpolation walks the grid with locality.  The order of a bin's samples comes from
+// atomics, so type 1 is not bitwise reproducible across plans, as the reference's cufinufft
+// is not.
 #pragma once
 
 #include "common.cuh"
 
 namespace hb {
 
-constexpr int kNufftBin = 8;  // fine-grid cells per bin edge
+constexpr int kNufftMaxBatch = 32;  // largest maxbatch of a plan
+constexpr int kNufftGroup = 8;      // transforms interleaved in one grid
+struct CoilMaps {  // coil-map pointers by value
+  const float2* s[kNufftGroup];
+};
 constexpr float kNufftInvTwoPi = 0.159154943091895336f;
 
 // A plan of dimension d < 3 keeps the 3-axis layout with its leading 3 - d axes
@@ -31,6 +36,7 @@ constexpr float kNufftInvTwoPi = 0.159154943091895336f;
 struct NufftGeom {
   int N[3];          // modes per axis
   int n[3];          // fine grid per axis (2 N; 1 on a degenerate axis)
+  int bin[3];        // cells per bin: (4, 4, 8), (1, 8, 8) in 2-D, (1, 1, 8) in 1-D
   int nb[3];         // bins per axis
   int w;             // kernel width (cells)
   float beta;        // kernel shape
@@ -44,10 +50,22 @@ __device__ __forceinline__ float nufft_grid_pos(float x, int n) {
   return u < (float)n ? u : 0.f;  // rounding may land exactly on n
 }
 
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float y;
+  asm("rsqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// Branch-free, so that a lane's evaluations overlap: the square root is the approximate
+// reciprocal root with one Newton correction of the root itself (within an ulp; s = 0 is
+// kept off the reciprocal).
 __device__ __forceinline__ float es_kernel(float z, float beta, float inv_hw) {
   const float t = z * inv_hw;
-  const float s = 1.f - t * t;
-  return s > 0.f ? expf(beta * (sqrtf(s) - 1.f)) : 0.f;
+  const float s = 1.f - t * t, sp = fmaxf(s, 1e-30f);
+  const float y = rsqrt_approx(sp);
+  float r = sp * y;
+  r = fmaf(0.5f * y, fmaf(-r, r, sp), r);
+  const float e = expf(beta * (r - 1.f));
+  return s > 0.f ? e : 0.f;
 }
 
 // First cell and the W kernel values of one axis.
@@ -68,79 +86,132 @@ __device__ __forceinline__ void red_add(float2* p, float2 v) {
   asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(v.x), "f"(v.y) : "memory");
 }
 
-// ---- binning (once per plan) ----
-__global__ void nufft_bin_count_kernel(NufftGeom g, const float* coords, int* sample_bin, int* bin_count) {
-  const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= g.K) return;
-  int b[3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    const float u = nufft_grid_pos(coords[a * g.K + j], g.n[a]);
-    const int bi = (int)u / kNufftBin;
-    b[a] = bi < g.nb[a] ? bi : g.nb[a] - 1;
-  }
-  const int bin = (b[0] * g.nb[1] + b[1]) * g.nb[2] + b[2];
-  sample_bin[j] = bin;
-  atomicAdd(&bin_count[bin], 1);
+// The values to spread: transform b of sample j is c[b * c_ld + j] (1 when c is null), times w[j].
+struct SpreadSource {
+  const float2* c;
+  long long c_ld;
+  const float* w;  // nullable
+};
+__device__ __forceinline__ float2 spread_value(const SpreadSource& src, int b, int j, float csgn) {
+  float2 v = src.c ? src.c[b * src.c_ld + j] : make_float2(1.f, 0.f);
+  if (src.w) v = cscale(v, src.w[j]);
+  v.y *= csgn;
+  return v;
 }
 
-// Exclusive prefix sum of n ints by one CTA of 1024 threads (bin counts -> offsets).
-__global__ void __launch_bounds__(1024) nufft_scan_kernel(const int* count, int* offset, int n) {
-  __shared__ int part[1024];
-  const int per = (n + 1023) / 1024;
-  const int lo = threadIdx.x * per, hi = (lo + per) < n ? (lo + per) : n;
-  int s = 0;
-  for (int i = lo; i < hi; ++i) s += count[i];
+// ---- binning (once per plan): coords [dim][K] pair with the trailing axes ----
+__device__ __forceinline__ float nufft_coord_pos(const NufftGeom& g, const float* coords, int a, long long j) {
+  return a < 3 - g.dim ? 0.f : nufft_grid_pos(coords[(a - (3 - g.dim)) * g.K + j], g.n[a]);
+}
+// bin of every sample and its rank within the bin
+__global__ void nufft_bin_count_kernel(NufftGeom g, const float* coords, int2* bin_rank, int* bin_count) {
+  const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= g.K) return;
+  int bin = 0;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const int bi = (int)nufft_coord_pos(g, coords, a, j) / g.bin[a];
+    bin = bin * g.nb[a] + (bi < g.nb[a] ? bi : g.nb[a] - 1);
+  }
+  bin_rank[j] = make_int2(bin, atomicAdd(&bin_count[bin], 1));
+}
+
+// Exclusive prefix sum of n ints: per block of 4096 (block totals to `sums`), a one-block scan
+// of the totals, and their addition; out[n] = total.  (A single CTA took 524 us for the
+// 262144 bins of a 512^3 grid; this form takes 3 launches of a few us.)
+constexpr int kScanBlock = 4096;
+__device__ __forceinline__ int block_scan_exclusive(int s, int* part) {  // 1024 threads; part[1024]
   part[threadIdx.x] = s;
   __syncthreads();
-  for (int d = 1; d < 1024; d <<= 1) {  // inclusive Hillis-Steele scan of the parts
+  for (int d = 1; d < 1024; d <<= 1) {
     const int v = threadIdx.x >= d ? part[threadIdx.x - d] : 0;
     __syncthreads();
     part[threadIdx.x] += v;
     __syncthreads();
   }
-  int run = part[threadIdx.x] - s;
-  for (int i = lo; i < hi; ++i) {
-    offset[i] = run;
-    run += count[i];
+  return part[threadIdx.x] - s;
+}
+__global__ void __launch_bounds__(1024) nufft_scan_block_kernel(const int* in, int* out, int* sums, int n) {
+  __shared__ int part[1024];
+  const int lo = blockIdx.x * kScanBlock + threadIdx.x * 4;
+  int v[4], s = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    v[i] = lo + i < n ? in[lo + i] : 0;
+    s += v[i];
+  }
+  int run = block_scan_exclusive(s, part);
+  if (threadIdx.x == 1023) sums[blockIdx.x] = run + s;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (lo + i < n) out[lo + i] = run;
+    run += v[i];
   }
 }
-
-__global__ void nufft_bin_scatter_kernel(long long K, const int* sample_bin, int* cursor, int* perm) {
-  const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= K) return;
-  perm[atomicAdd(&cursor[sample_bin[j]], 1)] = (int)j;
+__global__ void __launch_bounds__(1024) nufft_scan_sums_kernel(int* sums, int nblocks) {  // in place
+  __shared__ int part[1024];
+  const int per = (nblocks + 1023) / 1024;
+  const int lo = threadIdx.x * per, hi = (lo + per) < nblocks ? (lo + per) : nblocks;
+  int s = 0;
+  for (int i = lo; i < hi; ++i) s += sums[i];
+  int run = block_scan_exclusive(s, part);
+  for (int i = lo; i < hi; ++i) {
+    const int v = sums[i];
+    sums[i] = run;
+    run += v;
+  }
+}
+__global__ void __launch_bounds__(1024) nufft_scan_add_kernel(const int* in, int* out, const int* sums, int n) {
+  const int lo = blockIdx.x * kScanBlock + threadIdx.x * 4, add = sums[blockIdx.x];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (lo + i < n) {
+      out[lo + i] += add;
+      if (lo + i == n - 1) out[n] = out[n - 1] + in[n - 1];
+    }
 }
 
-// Kernel weights of axis a, or the single weight 1 at cell 0 on a degenerate axis
+// pts[position] = (u0, u1, u2, sample number), in bin order
+__global__ void nufft_bin_scatter_kernel(NufftGeom g, const float* coords, const int2* bin_rank, const int* start,
+                                         float4* pts) {
+  const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= g.K) return;
+  const int2 br = bin_rank[j];
+  pts[start[br.x] + br.y] = make_float4(nufft_coord_pos(g, coords, 0, j), nufft_coord_pos(g, coords, 1, j),
+                                        nufft_coord_pos(g, coords, 2, j), __int_as_float((int)j));
+}
+
+// Kernel weights of an axis at position u, or the single weight 1 at cell 0 on a degenerate axis
 template <int W, int WA>
-__device__ __forceinline__ int nufft_axis(const NufftGeom& g, const float* coords, int a, int j, float* wt) {
+__device__ __forceinline__ int nufft_axis(const NufftGeom& g, float u, float* wt) {
   if constexpr (WA == 1) {
     wt[0] = 1.f;
     return 0;
   } else {
-    return nufft_axis_weights<W>(nufft_grid_pos(coords[a * g.K + j], g.n[a]), g.beta, wt);
+    return nufft_axis_weights<W>(u, g.beta, wt);
   }
 }
 
-// ---- type 1: spread into a zeroed grid [n0][n1][n2][NB], NB = 1 << lgnb interleaved
-// transforms; one thread per (sample, transform), transform fastest; csgn = -1 conjugates c ----
+// ---- type 1 by vector reductions into a zeroed grid [n0][n1][n2][NB], NB = 1 << lgnb: one thread
+// per (sample, transform), transform fastest.  Used where the tile form (nufft_spread_kernels.cuh)
+// is not: 1-D plans (a sample has only W cells, fewer than a tile's tests would cost) and the
+// point-spread function, whose thousands of equal terms at the centre of a trajectory round
+// differently when they are summed tile by tile (2e-3 of the diagonal's rms at single
+// entries). ----
 template <int W, int DIM>
-__global__ void __launch_bounds__(256) nufft_spread_kernel(NufftGeom g, const float* coords, const int* perm,
-                                                           const float2* c, long long c_ld, int lgnb, int nact,
-                                                           float csgn, float2* grid) {
+__global__ void __launch_bounds__(256) nufft_spread_reductions_kernel(NufftGeom g, const float4* pts, const float2* vals,
+                                                                      int lgnb, float2* grid) {
   constexpr int W0 = DIM >= 3 ? W : 1, W1 = DIM >= 2 ? W : 1;
   const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int bt = (int)(id & ((1 << lgnb) - 1));
   const long long i = id >> lgnb;
-  if (i >= g.K || bt >= nact) return;
-  const int j = perm[i];
-  float2 cj = c[bt * c_ld + j];
-  cj.y *= csgn;
+  if (i >= g.K) return;
+  const float2 cj = vals[id];
+  const float4 p = pts[i];
   float w0[W0], w1[W1], w2[W];
-  const int i0 = nufft_axis<W, W0>(g, coords, 0, j, w0);
-  const int i1 = nufft_axis<W, W1>(g, coords, 1, j, w1);
-  const int i2 = nufft_axis<W, W>(g, coords, 2, j, w2);
+  const int i0 = nufft_axis<W, W0>(g, p.x, w0);
+  const int i1 = nufft_axis<W, W1>(g, p.y, w1);
+  const int i2 = nufft_axis<W, W>(g, p.z, w2);
   int x2[W];
 #pragma unroll
   for (int m = 0; m < W; ++m) x2[m] = wrap(i2 + m, g.n[2]) << lgnb;
@@ -158,21 +229,38 @@ __global__ void __launch_bounds__(256) nufft_spread_kernel(NufftGeom g, const fl
   }
 }
 
+// Where interpolated values go: to the caller's rows c[b * c_ld + j], or (c null) through the
+// k-space step of the SENSE normal operator, v = (v - y_b[j]) * w[j] (the reference's
+// mid-appliers; y and w nullable), to vals[i][NB] in sorted order, where spreading reads them.
+struct InterpDest {
+  float2* c;
+  long long c_ld;
+  const float2* y[kNufftGroup];
+  const float* w;
+  float2* vals;
+  float vsgn;  // -1 conjugates vals
+};
+
 // ---- type 2: interpolate (same thread mapping; csgn = -1 conjugates the result) ----
 template <int W, int DIM>
-__global__ void __launch_bounds__(256) nufft_interp_kernel(NufftGeom g, const float* coords, const int* perm,
-                                                           const float2* grid, int lgnb, int nact, float csgn,
-                                                           float2* c, long long c_ld) {
+__global__ void __launch_bounds__(256) nufft_interp_kernel(NufftGeom g, const float4* pts, const float2* grid, int lgnb,
+                                                           int nact, float csgn,
+                                                           const __grid_constant__ InterpDest dst) {
   constexpr int W0 = DIM >= 3 ? W : 1, W1 = DIM >= 2 ? W : 1;
   const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int bt = (int)(id & ((1 << lgnb) - 1));
   const long long i = id >> lgnb;
-  if (i >= g.K || bt >= nact) return;
-  const int j = perm[i];
+  if (i >= g.K) return;
+  if (bt >= nact) {
+    if (!dst.c) dst.vals[id] = make_float2(0.f, 0.f);
+    return;
+  }
+  const float4 p = pts[i];
+  const int j = __float_as_int(p.w);
   float w0[W0], w1[W1], w2[W];
-  const int i0 = nufft_axis<W, W0>(g, coords, 0, j, w0);
-  const int i1 = nufft_axis<W, W1>(g, coords, 1, j, w1);
-  const int i2 = nufft_axis<W, W>(g, coords, 2, j, w2);
+  const int i0 = nufft_axis<W, W0>(g, p.x, w0);
+  const int i1 = nufft_axis<W, W1>(g, p.y, w1);
+  const int i2 = nufft_axis<W, W>(g, p.z, w2);
   int x2[W];
 #pragma unroll
   for (int m = 0; m < W; ++m) x2[m] = wrap(i2 + m, g.n[2]) << lgnb;
@@ -198,16 +286,17 @@ __global__ void __launch_bounds__(256) nufft_interp_kernel(NufftGeom g, const fl
     acc.y = fmaf(w0[a], sa.y, acc.y);
   }
   acc.y *= csgn;
-  c[bt * c_ld + j] = acc;
+  if (dst.c) {
+    dst.c[bt * dst.c_ld + j] = acc;
+  } else {
+    if (dst.y[bt]) acc = csub(acc, dst.y[bt][j]);
+    if (dst.w) acc = cscale(acc, dst.w[j]);
+    acc.y *= dst.vsgn;
+    dst.vals[id] = acc;
+  }
 }
 
 // ---- Toeplitz diagonal through the NUFFT ----
-// a[i] = v, times w[i] when w is given
-__global__ void fill_c64_kernel(float2* a, long long n, float2 v, const float* w) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) a[i] = w ? cscale(v, w[i]) : v;
-}
-
 // Circulant (ifftshift) layout of a centred [M0][M1][M2] array, scaled:
 // out[n] = s * in[(n + M/2) mod M] per axis (offset d = n for n < M/2, n - M otherwise).
 __global__ void ifftshift3_scale_kernel(const float2* in, int M0, int M1, int M2, float s, float2* out) {
@@ -217,37 +306,6 @@ __global__ void ifftshift3_scale_kernel(const float2* in, int M0, int M1, int M2
   const int n2 = (int)(i % M2), n1 = (int)((i / M2) % M1), n0 = (int)(i / ((long long)M1 * M2));
   const int c0 = (n0 + M0 / 2) % M0, c1 = (n1 + M1 / 2) % M1, c2 = (n2 + M2 / 2) % M2;
   out[i] = cscale(in[((long long)c0 * M1 + c1) * M2 + c2], s);
-}
-
-// ---- SENSE around the NUFFT ----
-constexpr int kNufftMaxBatch = 32;  // largest maxbatch of a plan
-constexpr int kNufftGroup = 8;      // transforms interleaved in one grid
-struct CoilMaps {  // coil-map pointers by value
-  const float2* s[kNufftGroup];
-};
-
-// k-space step of the SENSE normal operator (the reference's mid-appliers):
-// k[b][j] = (k[b][j] - y_b[j]) * w[j]  (y_b and w nullable)
-struct KdataPtrs {
-  const float2* y[kNufftGroup];
-};
-__global__ void sense_kspace_mid_kernel(float2* k, int nb, long long K, KdataPtrs y, const float* w) {
-  const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= K) return;
-  const float wj = w ? w[j] : 1.f;
-  for (int b = 0; b < nb; ++b) {
-    float2 v = k[b * K + j];
-    if (y.y[b]) v = csub(v, y.y[b][j]);
-    k[b * K + j] = cscale(v, wj);
-  }
-}
-
-// k[b][j] = y_b[j] * w[j]  (weighted copy of k-space rows)
-__global__ void sense_kspace_weight_kernel(float2* k, int nb, long long K, KdataPtrs y, const float* w) {
-  const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= K) return;
-  const float wj = w[j];
-  for (int b = 0; b < nb; ++b) k[b * K + j] = cscale(y.y[b][j], wj);
 }
 
 }  // namespace hb

@@ -219,3 +219,24 @@ def test_every_pass_length_and_group_of_transforms(cuda, shape, nt):
         y, ref2 = _np(plan.type2(_c64(fm, cuda), isign=sign)), O.nudft_type2(coords, fm, sign)
         for t in range(nt):
             assert O.rel_l2(f[t], ref[t]) < bound and O.rel_l2(y[t], ref2[t]) < bound
+
+
+@pytest.mark.parametrize("shape,tol,nt", [((16, 16, 16), 1e-6, 8), ((32, 8, 48), 1e-4, 3), ((4, 4, 4), 1e-3, 2),
+                                          ((16, 32, 16), 1e-9, 1), ((64, 32), 1e-6, 8), ((4, 64), 1e-3, 4),
+                                          ((80, 16), 1e-5, 1)])
+def test_spreading_crowded_and_empty_tiles(cuda, shape, tol, nt):
+    """Tiles with thousands of samples (cut into pieces), with a few, and with none; samples on tile
+    and grid edges; kernels from narrower to wider than a tile.  Bound: 10 x tol, and not below the
+    float32 floor of test_every_pass_length_and_group_of_transforms."""
+    d = len(shape)
+    rng = np.random.default_rng(41)
+    crowd = rng.normal(0.0, 0.02, (d, 3000))                          # around the origin (a grid corner)
+    same = np.full((d, 700), 0.6)                                     # one position many times
+    cell = 2 * np.pi / (2 * np.array(shape, float))[:, None]
+    edge = cell * rng.integers(0, 2 * min(shape), (d, 60))            # on grid cells
+    coords = np.concatenate([crowd, same, edge, rng.uniform(-np.pi, np.pi, (d, 20))], 1).astype(np.float32)
+    plan = NufftPlan(torch.from_numpy(coords).to(cuda), shape, tol=tol, maxbatch=nt)
+    c = _rand((nt, coords.shape[1]), 42)
+    f, ref = _np(plan.type1(_c64(c, cuda))), O.nudft_type1(coords, c, shape, +1)
+    for t in range(nt):
+        assert O.rel_l2(f[t], ref[t]) < max(10 * tol, 1e-5 + 1.41e-7 * 2 * max(shape))
