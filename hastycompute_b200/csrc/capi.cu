@@ -14,6 +14,7 @@
 #include "cg_kernels.cuh"
 #include "diag_kernels.cuh"
 #include "fft3_launch.cuh"
+#include "plane_odd_kernels.cuh"
 #include "runtime.cuh"
 #include "tc_kernels.cuh"
 #include "toeplitz_kernels.cuh"
@@ -207,14 +208,13 @@ cudaError_t launch_b(const PassArgs& a, int nslots, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-template <int N0, int N1, int K, int THREADS>
-cudaError_t launch_bmod(const PassArgs& a, int nslots, cudaStream_t st) {
-  using C = PlaneModCfg<N0, N1, K, THREADS>;
-  const size_t smem = C::SMEM_F2 * sizeof(float2);
-  cudaError_t e = ensure_smem<plane_mod_kernel<N0, N1, K, THREADS>>(smem);
+// Launches one cluster per (slot, kx) plane, with the L2 prefetch one wave of clusters ahead
+// (as many clusters as can be co-resident, cached per kernel and device).
+template <auto kernel>
+cudaError_t launch_plane_clusters(const PassArgs& a, int nslots, int cluster, int threads, size_t smem, cudaStream_t st) {
+  cudaError_t e = ensure_smem<kernel>(smem);
   if (e != cudaSuccess) return e;
-  dim3 grid(K, nslots, 2 * a.N2);
-  // one wave of clusters ahead: as many clusters as can be co-resident
+  dim3 grid(cluster, nslots, 2 * a.N2);
   static std::atomic<int> ahead[64];
   int dev = 0;
   e = cudaGetDevice(&dev);
@@ -222,11 +222,11 @@ cudaError_t launch_bmod(const PassArgs& a, int nslots, cudaStream_t st) {
   int pa = ahead[dev & 63].load();
   if (pa <= 0) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(K, 1, 1);
-    cfg.blockDim = dim3(THREADS, 1, 1);
+    cfg.gridDim = dim3(cluster, 1, 1);
+    cfg.blockDim = dim3(threads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     int ncl = 0;
-    e = cudaOccupancyMaxActiveClusters(&ncl, plane_mod_kernel<N0, N1, K, THREADS>, &cfg);
+    e = cudaOccupancyMaxActiveClusters(&ncl, kernel, &cfg);
     if (e != cudaSuccess) return e;
     pa = ncl < 1 ? 1 : ncl;
     ahead[dev & 63].store(pa);
@@ -234,8 +234,18 @@ cudaError_t launch_bmod(const PassArgs& a, int nslots, cudaStream_t st) {
   PassArgs b = a;
   b.prefetch_ahead = getenv("HB_NO_L2_PREFETCH") ? 0 : pa;
   LaunchScope ls(HB_KERNEL_PLANE_YZ, st);
-  plane_mod_kernel<N0, N1, K, THREADS><<<grid, THREADS, smem, st>>>(b);
+  kernel<<<grid, threads, smem, st>>>(b);
   return cudaGetLastError();
+}
+template <int N0, int N1, int K, int THREADS>
+cudaError_t launch_bmod(const PassArgs& a, int nslots, cudaStream_t st) {
+  constexpr size_t smem = PlaneModCfg<N0, N1, K, THREADS>::SMEM_F2 * sizeof(float2);
+  return launch_plane_clusters<plane_mod_kernel<N0, N1, K, THREADS>>(a, nslots, K, THREADS, smem, st);
+}
+template <int K, int THREADS>
+cudaError_t launch_bodd(const PassArgs& a, int nslots, cudaStream_t st) {
+  constexpr size_t smem = PlaneOddCfg<K, THREADS>::SMEM_F2 * sizeof(float2);
+  return launch_plane_clusters<plane_odd_kernel<K, THREADS>>(a, nslots, K, THREADS, smem, st);
 }
 
 // Plane-pass schedules (cluster split Q x CTA size) per plane size; hb_plan_autotune
@@ -257,20 +267,15 @@ const PlaneVariant kPlane64[] = {
     {"mod4t256", &launch_bmod<64, 64, 4, 256>}, {"mod4t128", &launch_bmod<64, 64, 4, 128>},
     {"mod8t128", &launch_bmod<64, 64, 8, 128>},
 };
-const PlaneVariant kPlane96[] = {
-    {"q1t256", &launch_b<96, 96, 1, 256>}, {"q2t128", &launch_b<96, 96, 2, 128>},
-    {"q2t256", &launch_b<96, 96, 2, 256>},
-};
-const PlaneVariant kPlane160[] = {
-    {"q2t128", &launch_b<160, 160, 2, 128>}, {"q4t128", &launch_b<160, 160, 4, 128>},
-};
+const PlaneVariant kPlane96[] = {{"odd3t128", &launch_bodd<3, 128>}};
+const PlaneVariant kPlane160[] = {{"odd5t256", &launch_bodd<5, 256>}};
 
 const PlaneVariant* plane_variants(int N0, int N1, int* n) {
   *n = 0;
   if (N0 == 128 && N1 == 128) { *n = 10; return kPlane128; }
   if (N0 == 64 && N1 == 64) { *n = 7; return kPlane64; }
-  if (N0 == 96 && N1 == 96) { *n = 3; return kPlane96; }
-  if (N0 == 160 && N1 == 160) { *n = 2; return kPlane160; }
+  if (N0 == 96 && N1 == 96) { *n = 1; return kPlane96; }
+  if (N0 == 160 && N1 == 160) { *n = 1; return kPlane160; }
   return nullptr;
 }
 

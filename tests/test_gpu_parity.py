@@ -306,6 +306,26 @@ def test_sense_normal_non_power_of_two(cuda, shape, ncoil):
     assert O.rel_l2(_np(out), ref) < TOL
 
 
+@pytest.mark.parametrize("shape", [(96, 96, 8), (160, 160, 16)])
+def test_odd_planes_with_a_diagonal_per_system(cuda, shape):
+    """The 96- and 160-point planes (frequency residues mod 3 and mod 5) with several systems, each its
+    own diagonal: one with a single frequency, which a wrong residue would miss."""
+    plan = ToeplitzPlan(shape, cuda)
+    rng = np.random.default_rng(51)
+    grid = tuple(2 * n for n in shape)
+    T = np.stack([rng.standard_normal(grid) + 1.5, np.zeros(grid), rng.standard_normal(grid)])
+    T[1, -1, 1, 3] = 2.0
+    packed = torch.stack([plan.pack_diagonal(_c64(t, cuda)) for t in T])
+    sm = synth.coil_maps(2, shape, seed=52)
+    x = np.stack([synth.gaussian_image(shape, seed=s) for s in (53, 54, 55)])
+    out = torch.empty(x.shape, dtype=torch.complex64, device=cuda)
+    plan.sense_normal(_c64(x, cuda), out, _c64(sm, cuda), packed, diag_index=[2, 1, 0], lam=0.1)
+    for i, d in enumerate((2, 1, 0)):
+        ref = O.sense_normal_toeplitz_t(_c64(x[i], cuda), _c64(sm, cuda), torch.from_numpy(T[d]).to(cuda)) + \
+            0.1 * _c64(x[i], cuda).to(torch.complex128)
+        assert O.rel_l2(out[i], ref) < TOL, i
+
+
 def _mixed_jobs(plan, cuda, seeds, ncoils, lam=1e-3):
     from hastycompute_b200.toeplitz import System
     shape = plan.shape
