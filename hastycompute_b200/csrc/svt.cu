@@ -12,6 +12,22 @@
 
 using namespace hb;
 
+namespace {
+
+template <int NT>
+cudaError_t launch_svt(const SvtArgs& a, int64_t nblocks, cudaStream_t st) {
+  constexpr size_t smem = SvtCfg<NT>::SMEM;
+  if (smem > 48 * 1024) {  // per device; cheap next to the launch
+    cudaError_t e = cudaFuncSetAttribute(svt_blocks_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  LaunchScope ls(HB_KERNEL_CG_UPDATE, st);
+  svt_blocks_kernel<NT><<<(unsigned)nblocks, kSvtThreads, smem, st>>>(a);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
 extern "C" {
 
 int hb_svt_blocks(void* x, int64_t d0, int64_t d1, int64_t S0, int64_t S1, int64_t S2, int64_t b0, int64_t b1,
@@ -36,11 +52,16 @@ int hb_svt_blocks(void* x, int64_t d0, int64_t d1, int64_t S0, int64_t S1, int64
   a.thresh = (float)thresh;
   a.rank = soft ? 0 : (int)(thresh + 0.5);
   cudaStream_t st = (cudaStream_t)stream;
-  {
-    LaunchScope ls(HB_KERNEL_CG_UPDATE, st);
-    svt_blocks_kernel<<<(unsigned)nblocks, kSvtThreads, 0, st>>>(a);
+  switch ((d0 + 3) / 4) {
+    case 1: HB_CUDA(launch_svt<1>(a, nblocks, st)); break;
+    case 2: HB_CUDA(launch_svt<2>(a, nblocks, st)); break;
+    case 3: HB_CUDA(launch_svt<3>(a, nblocks, st)); break;
+    case 4: HB_CUDA(launch_svt<4>(a, nblocks, st)); break;
+    case 5: HB_CUDA(launch_svt<5>(a, nblocks, st)); break;
+    case 6: HB_CUDA(launch_svt<6>(a, nblocks, st)); break;
+    case 7: HB_CUDA(launch_svt<7>(a, nblocks, st)); break;
+    default: HB_CUDA(launch_svt<8>(a, nblocks, st)); break;
   }
-  HB_CHECK_LAUNCH();
   return HB_OK;
 }
 

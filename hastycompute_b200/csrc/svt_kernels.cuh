@@ -8,12 +8,25 @@
 // row-major), column = d0 index), as extract_block(..., flatten_split 0, transpose) forms
 // it.  With M = U S V^H: soft f(s) = max(s - thresh, 0), hard keeps the `rank` largest s,
 // and the block is replaced by U f(S) V^H = M W,  W = V diag(f(s)/s) V^H  (0 where s = 0).
-// One CTA per block:
-//   1. G = M^H M in FP64 (rows staged through shared memory in chunks);
-//   2. one warp diagonalises G by cyclic complex Jacobi rotations (FP64, shared memory):
-//      G = V diag(lambda) V^H, s = sqrt(lambda);
+// One CTA of 128 threads per block, columns padded to a multiple of four:
+//   1. G = M^H M in FP64: rows are staged in shared memory as doubles (converted once), every
+//      thread accumulates one 4 x 4 tile of G over its share of the rows in registers;
+//   2. G is diagonalised by Jacobi rotations (FP64), G = V diag(lambda) V^H, s = sqrt(lambda): a round
+//      rotates the n / 2 disjoint pairs of a round-robin tournament at once, each 2 x 2 block of
+//      A' = J^H A J by one thread, so a round takes two barriers;
 //   3. W, then every row is replaced by (row) W in FP32, in place.
 // Blocks of one launch must not overlap (the host launches overlapping sets in waves).
+//
+// Bound: the three parts take about equal shares (of 2.65 ms, measured by leaving each out: Gram 0.97,
+// rotations 0.73, rows 0.92); the floors are FP64 issue 0.5 + 0.3 ms, FP32 issue 0.4 ms and two reads
+// and a write of the data 0.8 ms, with the shared-memory pipe (4 bytes per lane and cycle, broadcast
+// or not) next.  Measured, 3375 blocks of 2560 x 20: 2.65 ms against 10.03 ms when one warp made the
+// rotations one after the other and every thread computed single entries of G; 32 columns 5.64
+// against 19.5 ms, 8 columns 0.74 against 2.53 ms.  On the way: rotations of a round in parallel
+// 3.26 ms, staging ahead without divisions 2.93 ms, single-precision staging and unpaired W 2.65 ms,
+// rows last to first 2.51 ms, the real products of W summed apart (a sum of 40 terms in one chain
+// rounds worse than the 20 complex products it stands for) 2.65 ms.  G by FP64 mma.sync m8n8k4 straight from global memory: 3.26 ms; 96
+// registers for five CTAs per SM 3.65 ms, 168 for three 2.87 ms.
 #pragma once
 
 #include "common.cuh"
@@ -22,7 +35,7 @@ namespace hb {
 
 constexpr int kSvtMaxCols = 32;  // d0 <= 32
 constexpr int kSvtThreads = 128;
-constexpr int kSvtChunk = 32;    // rows staged per Gram step (the same space later holds W)
+constexpr int kSvtChunk = 64;    // rows staged per Gram step
 constexpr int kSvtMaxSweeps = 15;
 
 struct SvtArgs {
@@ -35,167 +48,357 @@ struct SvtArgs {
   int rank;
 };
 
-struct dcomplex {
-  double x, y;
+// Walks the rows of a block's matrix in steps of a fixed number of rows, keeping the row's element
+// offset in x: mixed-radix addition instead of divisions.
+struct SvtRow {
+  int i0, i1, i2;       // voxel in the block
+  int s0, s1, s2;       // the step's digits
+  long long off;
+  long long step, w2, w1, w0;  // offset of a step; corrections when i2, i1, i0 wrap
+  __device__ __forceinline__ SvtRow(const SvtArgs& a, int c0, int c1, int c2, int row, int stride) {
+    const long long p1 = a.S2, p0 = p1 * a.S1, pd = p0 * a.S0;
+    i2 = row % a.b2;
+    i1 = (row / a.b2) % a.b1;
+    i0 = (row / (a.b2 * a.b1)) % a.b0;
+    off = (long long)(row / (a.b2 * a.b1 * a.b0)) * pd + (c0 + i0) * p0 + (c1 + i1) * p1 + c2 + i2;
+    s2 = stride % a.b2;
+    s1 = (stride / a.b2) % a.b1;
+    s0 = (stride / (a.b2 * a.b1)) % a.b0;
+    step = (long long)(stride / (a.b2 * a.b1 * a.b0)) * pd + s0 * p0 + s1 * p1 + s2;
+    w2 = p1 - a.b2;
+    w1 = p0 - a.b1 * p1;
+    w0 = pd - a.b0 * p0;
+  }
+  __device__ __forceinline__ void next(const SvtArgs& a) {
+    off += step;
+    i2 += s2;
+    i1 += s1;
+    i0 += s0;
+    if (i2 >= a.b2) { i2 -= a.b2; ++i1; off += w2; }
+    if (i1 >= a.b1) { i1 -= a.b1; ++i0; off += w1; }
+    if (i0 >= a.b0) { i0 -= a.b0; off += w0; }
+  }
+  __device__ __forceinline__ void prev(const SvtArgs& a) {
+    off -= step;
+    i2 -= s2;
+    i1 -= s1;
+    i0 -= s0;
+    if (i2 < 0) { i2 += a.b2; --i1; off -= w2; }
+    if (i1 < 0) { i1 += a.b1; --i0; off -= w1; }
+    if (i0 < 0) { i0 += a.b0; off -= w0; }
+  }
 };
 
-__device__ __forceinline__ long long svt_row_offset(const SvtArgs& a, int c0, int c1, int c2, int r) {
-  const int nbv = a.b0 * a.b1 * a.b2;
-  const int d1i = r / nbv, v = r % nbv;
-  const int i0 = v / (a.b1 * a.b2), i1 = (v / a.b2) % a.b1, i2 = v % a.b2;
-  return (((long long)d1i * a.S0 + (c0 + i0)) * a.S1 + (c1 + i1)) * a.S2 + (c2 + i2);
+// NT: columns in tiles of four, NT = ceil(d0 / 4).  Dynamic shared memory: A and V [NC][NC + 1] doubles
+// (complex), then the staged rows [kSvtChunk][NC + 1], whose space later holds W.
+template <int NT>
+struct SvtCfg {
+  static constexpr int NC = 4 * NT;
+  static constexpr int LD = NC + 1;                      // odd pitch in 16-byte units: rows on distinct banks
+  static constexpr int TILES = NT * (NT + 1) / 2;        // upper-triangle tiles of G
+  static constexpr int GROUPS = kSvtThreads / TILES;     // row groups
+  static constexpr int RLD = NC + 2;                     // pitch of the staged rows
+  static constexpr size_t SMEM = (size_t)2 * NC * LD * sizeof(double2) + (size_t)kSvtChunk * RLD * sizeof(float2);
+  static_assert(kSvtChunk * RLD >= NC * NC, "W takes the place of the staged rows");
+};
+
+__device__ __forceinline__ double svt_block_sum(double v, double* red) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  __syncthreads();
+  if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = v;
+  __syncthreads();
+  double s = 0.0;
+  for (int w = 0; w < kSvtThreads / 32; ++w) s += red[w];
+  return s;
 }
 
-__global__ void __launch_bounds__(kSvtThreads) svt_blocks_kernel(SvtArgs a) {
-  static_assert(kSvtChunk == kSvtMaxCols, "the row chunk and W share their shared memory");
-  __shared__ float2 chunk[kSvtChunk][kSvtMaxCols + 1];  // Gram: staged rows; afterwards W
-  __shared__ dcomplex A[kSvtMaxCols][kSvtMaxCols + 1];
-  __shared__ dcomplex V[kSvtMaxCols][kSvtMaxCols + 1];
-  __shared__ double wdiag[kSvtMaxCols];
-  float2(*W)[kSvtMaxCols + 1] = chunk;
-  const int n = a.d0;
+template <int NT>
+__global__ void __launch_bounds__(kSvtThreads, 4) svt_blocks_kernel(SvtArgs a) {
+  using C = SvtCfg<NT>;
+  constexpr int NC = C::NC, LD = C::LD;
+  extern __shared__ __align__(16) double2 svt_smem[];
+  double2* A = svt_smem;           // [NC][LD]
+  double2* V = A + NC * LD;        // [NC][LD]
+  float2* rows = reinterpret_cast<float2*>(V + NC * LD);  // [kSvtChunk][RLD]
+  float2* W = rows;                                       // [NC][NC]
+  __shared__ double wdiag[kSvtMaxCols], red[kSvtThreads / 32];
+  // rotations of the current and the next round: columns p < q, c, s e
+  __shared__ int2 rot_pq[2][kSvtMaxCols / 2];
+  __shared__ double rot_c[2][kSvtMaxCols / 2];
+  __shared__ double2 rot_s[2][kSvtMaxCols / 2];
+  const int n = a.d0, tid = threadIdx.x;
   const int c0 = a.corners[3 * blockIdx.x], c1 = a.corners[3 * blockIdx.x + 1], c2 = a.corners[3 * blockIdx.x + 2];
   // a block that does not fit inside the image is left untouched (the host validates corners)
   if (c0 < 0 || c1 < 0 || c2 < 0 || c0 + a.b0 > a.S0 || c1 + a.b1 > a.S1 || c2 + a.b2 > a.S2) return;
   const int R = a.d1 * a.b0 * a.b1 * a.b2;
   const long long col_stride = (long long)a.d1 * a.S0 * a.S1 * a.S2;
 
-  // 1. Gram matrix, FP64: thread t accumulates the pairs (p, q), p <= q, numbered t, t + T, ...
-  const int npairs = n * (n + 1) / 2;
-  constexpr int kMaxPairsPerThread = (kSvtMaxCols * (kSvtMaxCols + 1) / 2 + kSvtThreads - 1) / kSvtThreads;
-  dcomplex acc[kMaxPairsPerThread];
-  int pp[kMaxPairsPerThread], pq[kMaxPairsPerThread];
-#pragma unroll
-  for (int k = 0; k < kMaxPairsPerThread; ++k) {
-    acc[k] = {0.0, 0.0};
-    int idx = threadIdx.x + k * kSvtThreads, p = 0;
-    while (idx >= n - p && p < n) {  // pair number -> (p, q)
-      idx -= n - p;
-      ++p;
-    }
-    pp[k] = p;
-    pq[k] = p + idx;
+  // 1. Gram matrix: thread (tile, group) accumulates G[4 ti + i][4 tj + j] over rows group, group + GROUPS, ...
+  const int tile = tid % C::TILES, group = tid / C::TILES;
+  int ti = 0, tj = tile;
+  while (tj >= NT - ti) {
+    tj -= NT - ti;
+    ++ti;
   }
+  tj += ti;
+  double2 g[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) g[i][j] = make_double2(0.0, 0.0);
+  // staging: consecutive threads take consecutive rows of one column, two column groups; the next
+  // chunk's values are loaded while the current one is used
+  constexpr int STEP = kSvtThreads / kSvtChunk, NV = NC / STEP;
+  const int srow = tid % kSvtChunk, scol = tid / kSvtChunk;
+  float2 v[NV];
+  SvtRow stage(a, c0, c1, c2, srow, kSvtChunk);
+  auto load = [&](int r0) {
+    const bool in = r0 + srow < R;
+    const float2* src = a.x + stage.off + scol * col_stride;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] = in && scol + STEP * k < n ? src[STEP * k * col_stride] : make_float2(0.f, 0.f);
+    stage.next(a);
+  };
+  load(0);
+#pragma unroll 1
   for (int r0 = 0; r0 < R; r0 += kSvtChunk) {
     const int nr = (R - r0) < kSvtChunk ? (R - r0) : kSvtChunk;
-    __syncthreads();
-    for (int i = threadIdx.x; i < nr * n; i += kSvtThreads) {
-      const int r = i % nr, c = i / nr;  // consecutive threads: consecutive rows of one column
-      chunk[r][c] = a.x[c * col_stride + svt_row_offset(a, c0, c1, c2, r0 + r)];
-    }
-    __syncthreads();
+    __syncthreads();  // the previous rows have been used
 #pragma unroll
-    for (int k = 0; k < kMaxPairsPerThread; ++k) {
-      if (threadIdx.x + k * kSvtThreads >= npairs) continue;
-      const int p = pp[k], q = pq[k];
-      double sx = 0.0, sy = 0.0;
-      for (int r = 0; r < nr; ++r) {
-        const float2 u = chunk[r][p], v = chunk[r][q];  // conj(u) * v
-        sx += (double)u.x * v.x + (double)u.y * v.y;
-        sy += (double)u.x * v.y - (double)u.y * v.x;
+    for (int k = 0; k < NV; ++k) rows[srow * C::RLD + scol + STEP * k] = v[k];
+    __syncthreads();
+    if (r0 + kSvtChunk < R) load(r0 + kSvtChunk);
+    if (group < C::GROUPS) {
+#pragma unroll 1
+      for (int r = group; r < nr; r += C::GROUPS) {
+        // shared memory delivers 4 bytes per lane and cycle, broadcast or not, so the rows stay in single
+        // precision there
+        const float4* u = reinterpret_cast<const float4*>(rows + r * C::RLD + 4 * ti);
+        const float4* w = reinterpret_cast<const float4*>(rows + r * C::RLD + 4 * tj);
+        double2 ui[4];
+        float2 wf[4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float4 p = u[i], q = w[i];
+          ui[2 * i] = make_double2((double)p.x, (double)p.y);
+          ui[2 * i + 1] = make_double2((double)p.z, (double)p.w);
+          wf[2 * i] = make_float2(q.x, q.y);
+          wf[2 * i + 1] = make_float2(q.z, q.w);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const double2 wj = make_double2((double)wf[j].x, (double)wf[j].y);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {  // conj(u_i) w_j
+            g[i][j].x = fma(ui[i].x, wj.x, fma(ui[i].y, wj.y, g[i][j].x));
+            g[i][j].y = fma(ui[i].x, wj.y, fma(-ui[i].y, wj.x, g[i][j].y));
+          }
+        }
       }
-      acc[k].x += sx;
-      acc[k].y += sy;
     }
   }
+  for (int i = tid; i < NC * LD; i += kSvtThreads) V[i] = make_double2(i / LD == i % LD ? 1.0 : 0.0, 0.0);
+#pragma unroll 1
+  for (int k = 0; k < C::GROUPS; ++k) {  // groups add up in a fixed order
+    if (group == k) {
 #pragma unroll
-  for (int k = 0; k < kMaxPairsPerThread; ++k) {
-    if (threadIdx.x + k * kSvtThreads >= npairs) continue;
-    const int p = pp[k], q = pq[k];
-    A[p][q] = acc[k];
-    A[q][p] = {acc[k].x, -acc[k].y};
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          double2* at = A + (4 * ti + i) * LD + 4 * tj + j;
+          *at = k == 0 ? g[i][j] : make_double2(at->x + g[i][j].x, at->y + g[i][j].y);
+        }
+    }
+    __syncthreads();
   }
-  for (int i = threadIdx.x; i < n * n; i += kSvtThreads) V[i / n][i % n] = {i / n == i % n ? 1.0 : 0.0, 0.0};
-  __syncthreads();
 
-  // 2. cyclic complex Jacobi by warp 0; lane k owns row / column k of the updates
-  if (threadIdx.x < 32) {
-    const int k = threadIdx.x;
-    double fro = 0.0;
-    for (int j = 0; j < n; ++j)
-      if (k < n) fro += A[k][j].x * A[k][j].x + A[k][j].y * A[k][j].y;
+  // 2. Jacobi rotations of the upper triangle of G (A).  m: n rounded up to even; a padding index
+  // has a zero row and column.  This thread's block of A (pairs bi < bj) and parts of V (pair, row):
+  const int m = (n + 1) & ~1, np = m / 2;
+  int bi = 0, bj = tid;  // tid counts the pairs of pairs (bi, bj), bi < bj
+  while (bi < np && bj >= np - 1 - bi) {
+    bj -= np - 1 - bi;
+    ++bi;
+  }
+  bj = bi < np ? bj + bi + 1 : bi;
+  constexpr int kVTasks = (NC / 2 * NC + kSvtThreads - 33) / (kSvtThreads - 32);
+  int vtask[kVTasks];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) fro += __shfl_xor_sync(0xffffffffu, fro, off);
-    for (int sweep = 0; sweep < kSvtMaxSweeps; ++sweep) {
-      double offd = 0.0;
-      for (int j = 0; j < n; ++j)
-        if (k < n && j != k) offd += A[k][j].x * A[k][j].x + A[k][j].y * A[k][j].y;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) offd += __shfl_xor_sync(0xffffffffu, offd, off);
-      if (!(offd > 1e-30 * fro)) break;  // uniform across the warp
-      for (int p = 0; p < n - 1; ++p) {
-        for (int q = p + 1; q < n; ++q) {
-          const dcomplex apq = A[p][q];
-          const double mag = sqrt(apq.x * apq.x + apq.y * apq.y);
-          if (!(mag > 1e-300)) continue;
-          const double tau = (A[q][q].x - A[p][p].x) / (2.0 * mag);
-          const double t = tau == 0.0 ? 1.0 : (tau > 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-          const double c = 1.0 / sqrt(1.0 + t * t), s = t * c;
-          const double ex = apq.x / mag, ey = apq.y / mag;  // e = apq / |apq|
-          __syncwarp();
-          if (k < n) {  // columns p, q of A and V: new_p = c col_p - s conj(e) col_q, new_q = s e col_p + c col_q
-            const dcomplex ap = A[k][p], aq = A[k][q];
-            A[k][p] = {c * ap.x - s * (ex * aq.x + ey * aq.y), c * ap.y - s * (ex * aq.y - ey * aq.x)};
-            A[k][q] = {s * (ex * ap.x - ey * ap.y) + c * aq.x, s * (ex * ap.y + ey * ap.x) + c * aq.y};
-            const dcomplex vp = V[k][p], vq = V[k][q];
-            V[k][p] = {c * vp.x - s * (ex * vq.x + ey * vq.y), c * vp.y - s * (ex * vq.y - ey * vq.x)};
-            V[k][q] = {s * (ex * vp.x - ey * vp.y) + c * vq.x, s * (ex * vp.y + ey * vp.x) + c * vq.y};
-          }
-          __syncwarp();
-          if (k < n) {  // rows p, q of A: new_p = c row_p - s e row_q, new_q = s conj(e) row_p + c row_q
-            const dcomplex rp = A[p][k], rq = A[q][k];
-            A[p][k] = {c * rp.x - s * (ex * rq.x - ey * rq.y), c * rp.y - s * (ex * rq.y + ey * rq.x)};
-            A[q][k] = {s * (ex * rp.x + ey * rp.y) + c * rq.x, s * (ex * rp.y - ey * rp.x) + c * rq.y};
-          }
-          __syncwarp();
-        }
+  for (int t = 0; t < kVTasks; ++t) {
+    const int i = tid - 32 + t * (kSvtThreads - 32);
+    vtask[t] = tid >= 32 && i < np * n ? (i / n) | (i % n) << 5 : -1;
+  }
+  // rotations of a round into buffer `to`, and what they make of the diagonal blocks (threads < np)
+  auto rotations = [&](int round, int to) {
+    if (tid >= np) return;
+    // round-robin tournament: m - 1 stays, the others turn
+    int p = tid == 0 ? m - 1 : round + tid, q = round - tid;
+    if (tid > 0 && p >= m - 1) p -= m - 1;
+    if (q < 0) q += m - 1;
+    if (p > q) {
+      const int h = p;
+      p = q;
+      q = h;
+    }
+    const double2 apq = A[p * LD + q];
+    const double app = A[p * LD + p].x, aqq = A[q * LD + q].x;
+    const double mag2 = apq.x * apq.x + apq.y * apq.y;
+    double c = 1.0, f = 0.0;  // s e = f apq
+    if (mag2 > 1e-300) {
+      // t = sign(d) |apq| / (|d| + sqrt(d^2 + |apq|^2)), d = (aqq - app) / 2; c = 1 / sqrt(1 + t^2)
+      const double d = 0.5 * (aqq - app), h = fabs(d) + sqrt(d * d + mag2);
+      const double te = (d < 0.0 ? -1.0 : 1.0) / h;  // t e = te apq
+      c = rsqrt(1.0 + te * te * mag2);
+      f = c * te;
+      A[p * LD + p].x = app - te * mag2;  // t |apq| = te |apq|^2
+      A[q * LD + q].x = aqq + te * mag2;
+      A[p * LD + q] = make_double2(0.0, 0.0);
+    }
+    rot_pq[to][tid] = make_int2(p, q);
+    rot_c[to][tid] = c;
+    rot_s[to][tid] = make_double2(f * apq.x, f * apq.y);
+  };
+  auto sum2 = [&](bool diagonal) {  // sum of |A|^2 over the full matrix, with or without its diagonal
+    double part = 0.0;
+    for (int i = tid; i < NC * NC; i += kSvtThreads) {
+      const int p = i / NC, q = i % NC;
+      if (p < q || (diagonal && p == q)) {
+        const double2 v = A[p * LD + q];
+        part += (p < q ? 2.0 : 1.0) * (v.x * v.x + v.y * v.y);
       }
     }
-    // 3a. thresholded weights f(s)/s per eigenvalue
-    if (k < n) {
-      const double lam = A[k][k].x > 0.0 ? A[k][k].x : 0.0;
-      const double sv = sqrt(lam);
-      double w = 0.0;
-      if (a.soft) {
-        w = sv > (double)a.thresh ? (sv - (double)a.thresh) / sv : 0.0;
+    return svt_block_sum(part, red);
+  };
+  const double fro = sum2(true);
+#pragma unroll 1
+  for (int sweep = 0; sweep < kSvtMaxSweeps; ++sweep) {
+    if (!(sum2(false) > 1e-30 * fro)) break;  // uniform across the block
+    rotations(0, 0);
+    __syncthreads();
+#pragma unroll 1
+    for (int round = 0; round < m - 1; ++round) {
+      const int cur = round & 1;
+      // new_p = c col_p - conj(se) col_q, new_q = se col_p + c col_q (columns; rows with se conjugated)
+      if (bi < bj) {
+        const int2 I = rot_pq[cur][bi], J = rot_pq[cur][bj];
+        const double ci = rot_c[cur][bi], cj = rot_c[cur][bj];
+        const double2 si = rot_s[cur][bi], sj = rot_s[cur][bj];
+        auto get = [&](int r, int c) {
+          const double2 v = A[r < c ? r * LD + c : c * LD + r];
+          return make_double2(v.x, r < c ? v.y : -v.y);
+        };
+        const double2 pp = get(I.x, J.x), pq = get(I.x, J.y), qp = get(I.y, J.x), qq = get(I.y, J.y);
+        auto left = [&](double2 u, double2 v) {
+          return make_double2(cj * u.x - (sj.x * v.x + sj.y * v.y), cj * u.y - (sj.x * v.y - sj.y * v.x));
+        };
+        auto right = [&](double2 u, double2 v) {
+          return make_double2(sj.x * u.x - sj.y * u.y + cj * v.x, sj.x * u.y + sj.y * u.x + cj * v.y);
+        };
+        const double2 tpp = left(pp, pq), tpq = right(pp, pq), tqp = left(qp, qq), tqq = right(qp, qq);
+        auto top = [&](double2 u, double2 v) {
+          return make_double2(ci * u.x - (si.x * v.x - si.y * v.y), ci * u.y - (si.x * v.y + si.y * v.x));
+        };
+        auto low = [&](double2 u, double2 v) {
+          return make_double2(si.x * u.x + si.y * u.y + ci * v.x, si.x * u.y - si.y * u.x + ci * v.y);
+        };
+        auto put = [&](int r, int c, double2 v) {  // only the upper triangle is kept
+          A[r < c ? r * LD + c : c * LD + r] = r < c ? v : make_double2(v.x, -v.y);
+        };
+        put(I.x, J.x, top(tpp, tqp));
+        put(I.y, J.x, low(tpp, tqp));
+        put(I.x, J.y, top(tpq, tqq));
+        put(I.y, J.y, low(tpq, tqq));
+      }
+      __syncthreads();
+      // the next round's rotations (warp 0) beside this round's update of V (the other warps)
+      if (tid < 32) {
+        if (round + 1 < m - 1) rotations(round + 1, cur ^ 1);
       } else {
-        int larger = 0;  // rank of this eigenvalue (ties broken by index)
-        for (int j = 0; j < n; ++j) {
-          const double lj = A[j][j].x;
-          larger += (lj > A[k][k].x || (lj == A[k][k].x && j < k)) ? 1 : 0;
-        }
-        w = larger < a.rank ? 1.0 : 0.0;
-      }
-      wdiag[k] = w;
-    }
-  }
-  __syncthreads();
-  // 3b. W = V diag(w) V^H
-  for (int i = threadIdx.x; i < n * n; i += kSvtThreads) {
-    const int r = i / n, c = i % n;
-    double sx = 0.0, sy = 0.0;
-    for (int j = 0; j < n; ++j) {
-      const dcomplex vr = V[r][j], vc = V[c][j];  // V[r][j] w_j conj(V[c][j])
-      sx += wdiag[j] * (vr.x * vc.x + vr.y * vc.y);
-      sy += wdiag[j] * (vr.y * vc.x - vr.x * vc.y);
-    }
-    W[r][c] = make_float2((float)sx, (float)sy);
-  }
-  __syncthreads();
-  // 3c. rows <- rows W, in place
-  for (int r = threadIdx.x; r < R; r += kSvtThreads) {
-    const long long off = svt_row_offset(a, c0, c1, c2, r);
-    float2 m[kSvtMaxCols];
 #pragma unroll
-    for (int c = 0; c < kSvtMaxCols; ++c)
-      if (c < n) m[c] = a.x[c * col_stride + off];
+        for (int t = 0; t < kVTasks; ++t) {
+          if (vtask[t] < 0) break;
+          const int b = vtask[t] & 31, k = vtask[t] >> 5;
+          const int2 J = rot_pq[cur][b];
+          const double c = rot_c[cur][b];
+          const double2 se = rot_s[cur][b], u = V[k * LD + J.x], v = V[k * LD + J.y];
+          V[k * LD + J.x] = make_double2(c * u.x - (se.x * v.x + se.y * v.y), c * u.y - (se.x * v.y - se.y * v.x));
+          V[k * LD + J.y] = make_double2(se.x * u.x - se.y * u.y + c * v.x, se.x * u.y + se.y * u.x + c * v.y);
+        }
+      }
+      __syncthreads();
+    }
+  }
+  // 3a. thresholded weights f(s)/s per eigenvalue
+  if (tid < n) {
+    const double ev = A[tid * LD + tid].x;
+    const double sv = sqrt(ev > 0.0 ? ev : 0.0);
+    double w = 0.0;
+    if (a.soft) {
+      w = sv > (double)a.thresh ? (sv - (double)a.thresh) / sv : 0.0;
+    } else {
+      int larger = 0;  // rank of this eigenvalue (ties broken by index)
+      for (int j = 0; j < n; ++j) {
+        const double lj = A[j * LD + j].x;
+        larger += (lj > ev || (lj == ev && j < tid)) ? 1 : 0;
+      }
+      w = larger < a.rank ? 1.0 : 0.0;
+    }
+    wdiag[tid] = w;
+  }
+  __syncthreads();
+  // 3b. W = V diag(w) V^H (zero in the padding)
+  for (int i = tid; i < NC * NC; i += kSvtThreads) {
+    const int r = i / NC, c = i % NC;
+    double sx = 0.0, sy = 0.0;
+    if (r < n && c < n) {
+      for (int j = 0; j < n; ++j) {
+        const double2 vr = V[r * LD + j], vc = V[c * LD + j];  // V[r][j] w_j conj(V[c][j])
+        sx += wdiag[j] * (vr.x * vc.x + vr.y * vc.y);
+        sy += wdiag[j] * (vr.y * vc.x - vr.x * vc.y);
+      }
+    }
+    W[i] = make_float2((float)sx, (float)sy);
+  }
+  __syncthreads();
+  // 3c. rows <- rows W, in place, last rows first (the end of the block is still in L2 from the
+  // Gram pass); a thread takes two rows, side by side in FP32x2 pairs
+  const int last = tid + (R - 1) / (2 * kSvtThreads) * (2 * kSvtThreads) + kSvtThreads;
+  SvtRow it(a, c0, c1, c2, last, kSvtThreads);
+#pragma unroll 1
+  for (int r = last - kSvtThreads; r >= 0; r -= 2 * kSvtThreads) {
+    const bool one = r < R, two = r + kSvtThreads < R;
+    const long long off1 = it.off;
+    it.prev(a);
+    const long long off0 = it.off;
+    it.prev(a);
+    if (!one) continue;
+    float2* row0 = a.x + off0;
+    float2* row1 = two ? a.x + off1 : row0;
+    float2 vx[NC], vy[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const float2 u = c < n ? row0[c * col_stride] : make_float2(0.f, 0.f);
+      const float2 v = c < n ? row1[c * col_stride] : make_float2(0.f, 0.f);
+      vx[c] = make_float2(u.x, v.x);
+      vy[c] = make_float2(u.y, v.y);
+    }
 #pragma unroll 1
     for (int c = 0; c < n; ++c) {
-      float2 o = make_float2(0.f, 0.f);
+      // the four real products in chains of their own: half the length, so the rounding of a plain sum
+      float2 xx = make_float2(0.f, 0.f), yy = xx, xy = xx, yx = xx;
 #pragma unroll
-      for (int j = 0; j < kSvtMaxCols; ++j)
-        if (j < n) o = cadd(o, cmul(m[j], W[j][c]));
-      a.x[c * col_stride + off] = o;
+      for (int j = 0; j < NC; ++j) {
+        const float2 w = W[j * NC + c];
+        const float2 wx = make_float2(w.x, w.x), wy = make_float2(w.y, w.y);
+        xx = __ffma2_rn(vx[j], wx, xx);
+        yy = __ffma2_rn(vy[j], wy, yy);
+        xy = __ffma2_rn(vx[j], wy, xy);
+        yx = __ffma2_rn(vy[j], wx, yx);
+      }
+      const float2 ox = csub(xx, yy), oy = cadd(xy, yx);
+      row0[c * col_stride] = make_float2(ox.x, oy.x);
+      if (two) row1[c * col_stride] = make_float2(ox.y, oy.y);
     }
   }
 }

@@ -92,3 +92,18 @@ def test_admm_llr_against_oracle(cuda):
                         admm_iters=3, cg_iters=4)
     assert O.rel_l2(_np(xg), xr) < 1e-4
     assert O.rel_l2(_np(zg), zr) < 1e-4
+
+
+@pytest.mark.parametrize("d0,d1,block,soft,thresh", [(1, 1, (3, 5, 7), True, 2.0), (3, 2, (1, 1, 1), True, 0.5),
+                                                     (5, 1, (4, 3, 5), False, 2), (13, 3, (5, 5, 5), True, 5.0),
+                                                     (16, 1, (8, 8, 4), True, 4.0), (24, 2, (6, 7, 3), False, 3),
+                                                     (27, 1, (3, 3, 3), True, 2.0), (31, 5, (8, 8, 8), True, 8.0)])
+def test_svt_odd_columns_and_rows(cuda, d0, d1, block, soft, thresh):
+    """Every column tile count, odd counts, row counts off the staging and pairing steps, fewer rows
+    than columns; block corners at both ends of the image.  Tolerance as test_svt_blocks_against_numpy_svd."""
+    S = (17, 19, 18)
+    x = _lowrank(d0, d1, S, min(3, d0), seed=60 + d0)
+    corners = [(0, 0, 0), tuple(s - b for s, b in zip(S, block))]
+    xt = _c64(x, cuda)
+    svt_blocks(xt, corners, block, thresh, soft)
+    assert O.rel_l2(_np(xt), O.svt_blocks(x, corners, block, thresh, soft)) < 1e-5
