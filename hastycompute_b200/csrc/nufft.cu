@@ -112,12 +112,22 @@ cudaError_t spread_reductions_w(const hb_nufft* p, Group q, cudaStream_t st) {
 }
 template <int W>
 cudaError_t interp_w(const hb_nufft* p, const InterpDest& dst, Group q, float csgn, cudaStream_t st) {
-  const unsigned grid = (unsigned)(((p->g.K << q.lgnb) + 255) / 256);
   LaunchScope ls(HB_KERNEL_NUFFT, st);
-  auto go = [&](auto kernel) { kernel<<<grid, 256, 0, st>>>(p->g, p->pts, p->grid, q.lgnb, q.nact, csgn, dst); };
-  if (p->g.dim == 3) go(nufft_interp_kernel<W, 3>);
-  else if (p->g.dim == 2) go(nufft_interp_kernel<W, 2>);
-  else go(nufft_interp_kernel<W, 1>);
+  if (p->g.dim < 3) {
+    const unsigned grid = (unsigned)(((p->g.K << q.lgnb) + 255) / 256);
+    auto go = [&](auto kernel) { kernel<<<grid, 256, 0, st>>>(p->g, p->pts, p->grid, q.lgnb, q.nact, csgn, dst); };
+    if (p->g.dim == 2) go(nufft_interp_points_kernel<W, 2>);
+    else go(nufft_interp_points_kernel<W, 1>);
+    return cudaGetLastError();
+  }
+  auto go = [&](auto kernel, int per_cta) {
+    const unsigned grid = (unsigned)((p->g.K + per_cta - 1) / per_cta);
+    kernel<<<grid, 32 * kInterpWarps, 0, st>>>(p->g, p->pts, p->grid, q.nact, csgn, dst);
+  };
+  if (q.lgnb == 3) go(nufft_interp_rows_kernel<W, 8>, InterpCfg<W, 8>::PER_CTA);
+  else if (q.lgnb == 2) go(nufft_interp_rows_kernel<W, 4>, InterpCfg<W, 4>::PER_CTA);
+  else if (q.lgnb == 1) go(nufft_interp_rows_kernel<W, 2>, InterpCfg<W, 2>::PER_CTA);
+  else go(nufft_interp_rows_kernel<W, 1>, InterpCfg<W, 1>::PER_CTA);
   return cudaGetLastError();
 }
 

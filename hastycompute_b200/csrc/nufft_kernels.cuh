@@ -241,58 +241,202 @@ struct InterpDest {
   float vsgn;  // -1 conjugates vals
 };
 
-// ---- type 2: interpolate (same thread mapping; csgn = -1 conjugates the result) ----
+// Stores transform b's value at sample j (sorted position i).
+__device__ __forceinline__ void interp_store(const InterpDest& dst, int b, int nact, int NB, long long i, int j,
+                                             float2 v, float csgn) {
+  if (b >= nact) {
+    if (!dst.c) dst.vals[i * NB + b] = make_float2(0.f, 0.f);
+    return;
+  }
+  v.y *= csgn;
+  if (dst.c) {
+    dst.c[b * dst.c_ld + j] = v;
+    return;
+  }
+  if (dst.y[b]) v = csub(v, dst.y[b][j]);
+  if (dst.w) v = cscale(v, dst.w[j]);
+  v.y *= dst.vsgn;
+  dst.vals[i * NB + b] = v;
+}
+
+// ---- type 2 of 1-D and 2-D plans: one thread per (sample, transform), transform fastest; csgn = -1
+// conjugates the result.  In 2-D a sample has W rows, too few to pay for a group of lanes per sample
+// (8 transforms, W = 6, 51 k samples: 16 us against 20-26 us). ----
 template <int W, int DIM>
-__global__ void __launch_bounds__(256) nufft_interp_kernel(NufftGeom g, const float4* pts, const float2* grid, int lgnb,
-                                                           int nact, float csgn,
-                                                           const __grid_constant__ InterpDest dst) {
-  constexpr int W0 = DIM >= 3 ? W : 1, W1 = DIM >= 2 ? W : 1;
+__global__ void __launch_bounds__(256) nufft_interp_points_kernel(NufftGeom g, const float4* pts, const float2* grid,
+                                                                  int lgnb, int nact, float csgn,
+                                                                  const __grid_constant__ InterpDest dst) {
+  constexpr int W1 = DIM == 2 ? W : 1;
   const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int bt = (int)(id & ((1 << lgnb) - 1));
   const long long i = id >> lgnb;
   if (i >= g.K) return;
-  if (bt >= nact) {
-    if (!dst.c) dst.vals[id] = make_float2(0.f, 0.f);
-    return;
-  }
   const float4 p = pts[i];
-  const int j = __float_as_int(p.w);
-  float w0[W0], w1[W1], w2[W];
-  const int i0 = nufft_axis<W, W0>(g, p.x, w0);
+  float w1[W1], w2[W];
   const int i1 = nufft_axis<W, W1>(g, p.y, w1);
   const int i2 = nufft_axis<W, W>(g, p.z, w2);
   int x2[W];
 #pragma unroll
-  for (int m = 0; m < W; ++m) x2[m] = wrap(i2 + m, g.n[2]) << lgnb;
+  for (int m = 0; m < W; ++m) x2[m] = (wrap(i2 + m, g.n[2]) << lgnb) + bt;
   float2 acc = make_float2(0.f, 0.f);
-#pragma unroll 1
-  for (int a = 0; a < W0; ++a) {
-    const float2* Ga = grid + ((long long)wrap(i0 + a, g.n[0]) * g.n[1] * g.n[2] << lgnb) + bt;
-    float2 sa = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int b = 0; b < W1; ++b) {
-      const float2* Gab = Ga + ((long long)wrap(i1 + b, g.n[1]) * g.n[2] << lgnb);
-      float2 sb = make_float2(0.f, 0.f);
+  for (int b = 0; b < W1; ++b) {
+    const float2* row = grid + ((long long)wrap(i1 + b, g.n[1]) * g.n[2] << lgnb);
+    float2 s = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int m = 0; m < W; ++m) {
-        const float2 v = Gab[x2[m]];
-        sb.x = fmaf(w2[m], v.x, sb.x);
-        sb.y = fmaf(w2[m], v.y, sb.y);
-      }
-      sa.x = fmaf(w1[b], sb.x, sa.x);
-      sa.y = fmaf(w1[b], sb.y, sa.y);
+    for (int m = 0; m < W; ++m) {
+      const float2 v = row[x2[m]];
+      s.x = fmaf(w2[m], v.x, s.x);
+      s.y = fmaf(w2[m], v.y, s.y);
     }
-    acc.x = fmaf(w0[a], sa.x, acc.x);
-    acc.y = fmaf(w0[a], sa.y, acc.y);
+    acc.x = fmaf(w1[b], s.x, acc.x);
+    acc.y = fmaf(w1[b], s.y, acc.y);
   }
-  acc.y *= csgn;
-  if (dst.c) {
-    dst.c[bt * dst.c_ld + j] = acc;
+  interp_store(dst, bt, nact, 1 << lgnb, i, __float_as_int(p.w), acc, csgn);
+}
+
+template <int V>
+__device__ __forceinline__ void load_cells(const float2* p, float2* v) {  // V float2 as one load
+  if constexpr (V == 4) {
+    asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[1].x), "=f"(v[1].y), "=f"(v[2].x), "=f"(v[2].y), "=f"(v[3].x), "=f"(v[3].y)
+        : "l"(p));
+  } else if constexpr (V == 2) {
+    const float4 q = *reinterpret_cast<const float4*>(p);
+    v[0] = make_float2(q.x, q.y);
+    v[1] = make_float2(q.z, q.w);
   } else {
-    if (dst.y[bt]) acc = csub(acc, dst.y[bt][j]);
-    if (dst.w) acc = cscale(acc, dst.w[j]);
-    acc.y *= dst.vsgn;
-    dst.vals[id] = acc;
+    v[0] = *p;
+  }
+}
+
+// ---- type 2 of a 3-D plan: a group of XL x PL lanes per sample (two to eight samples per warp).  A load
+// of the group reads one row of W cells x NB transforms, a contiguous run of the interleaved grid:
+// lane = (cell x, part of the cell), up to 32 bytes per lane.  Every lane sums its x over the
+// sample's rows (first y, then z), multiplies by its x weight once, and the group's lanes are added up
+// at the end.  Neighbours in the sorted order run at the same time, so most rows are in L1.
+//
+// Bound: the L1 data path (a request is served 128 bytes a cycle when its lines are aligned, and half
+// of that when every quarter of it straddles two lines).  Measured, 512 k radial samples on 256^3, one
+// thread per (sample, transform) -> this form: 8 transforms, W = 7 1175 -> 663 us, W = 6 665 -> 506 us,
+// W = 5 614 -> 360 us, W = 4 328 -> 139 us; 4 transforms, W = 7 609 -> 356 us; 1 transform 253 -> 129 us.
+// One warp per sample with 16-byte loads: 738 us (1081 us without the aligned window). ----
+constexpr int kInterpWarps = 8;
+template <int W, int NB>
+struct InterpCfg {
+  static constexpr int V = NB < 4 ? NB : 4;                // transforms per lane
+  static constexpr int PL = NB / V;                        // lanes per cell
+  static constexpr int XL = W <= 4 ? 4 : 8;                // cells per row and load
+  static constexpr int XS = (W + XL - 1) / XL;             // loads per row
+  static constexpr int LANES = XL * PL, SL = 32 / LANES;   // lanes per sample, samples per warp
+  // the load's window starts at a multiple of XA cells (a 128-byte line of 8 transforms is 2 cells, of 4
+  // transforms 4) where it is wide enough to reach over the row from there
+  static constexpr int LINE = NB == 8 ? 2 : NB == 4 ? 4 : 1, XA = XS * XL >= W + LINE - 1 ? LINE : 1;
+  static constexpr int ROUNDS = 4;                         // samples per group
+  static constexpr int PER_CTA = kInterpWarps * SL * ROUNDS;
+};
+template <int W, int NB>
+__global__ void __launch_bounds__(32 * kInterpWarps, W <= 5 && NB > 1 ? 4 : 3)
+nufft_interp_rows_kernel(NufftGeom g, const float4* pts, const float2* grid, int nact, float csgn,
+                         const __grid_constant__ InterpDest dst) {
+  using C = InterpCfg<W, NB>;
+  constexpr int V = C::V, PL = C::PL, XL = C::XL, XS = C::XS, SL = C::SL;
+  __shared__ float w_s[kInterpWarps][SL][3 * W];  // z, y, x weights of the warp's samples
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int p = lane % PL, xl = (lane / PL) % XL, sl = lane / C::LANES;
+  const float hw = 0.5f * (float)W, inv_hw = 1.f / hw;
+  const unsigned rowlen = (unsigned)g.n[2] * NB, planelen = (unsigned)g.n[1] * rowlen;
+  const long long base = (long long)blockIdx.x * C::PER_CTA + warp * SL;
+#pragma unroll 1
+  for (int k = 0; k < C::ROUNDS; ++k) {
+    const long long w0 = base + k * (kInterpWarps * SL);  // the warp's first sample
+    if (w0 >= g.K) break;
+    const long long i = w0 + sl < g.K ? w0 + sl : g.K - 1;
+    const float4 pt = pts[i];
+    const int c0 = (int)ceilf(pt.x - hw), c1 = (int)ceilf(pt.y - hw), c2 = (int)ceilf(pt.z - hw);
+    __syncwarp();  // the previous weights have been read
+#pragma unroll
+    for (int m = lane % C::LANES; m < 3 * W; m += C::LANES) {
+      const int ax = m / W, t = m - ax * W;
+      const float u = ax == 0 ? pt.x : ax == 1 ? pt.y : pt.z;
+      const int c = ax == 0 ? c0 : ax == 1 ? c1 : c2;
+      w_s[warp][sl][m] = es_kernel((float)(c + t) - u, g.beta, inv_hw);
+    }
+    __syncwarp();
+    const float* wt = w_s[warp][sl];
+    unsigned yo[W], xo[XS];
+    float2 wy[W];
+    bool xok[XS];
+#pragma unroll
+    for (int b = 0; b < W; ++b) {
+      wy[b] = make_float2(wt[W + b], wt[W + b]);
+      yo[b] = (unsigned)wrap(c1 + b, g.n[1]) * rowlen;
+    }
+    const int x0 = (c2 & ~(C::XA - 1)) - c2 + xl;
+#pragma unroll
+    for (int c = 0; c < XS; ++c) {
+      const int x = x0 + c * XL;
+      xok[c] = x >= 0 && x < W;
+      xo[c] = (unsigned)wrap(c2 + (xok[c] ? x : 0), g.n[2]) * NB + V * p;
+    }
+    float2 acc[XS][V];
+#pragma unroll
+    for (int c = 0; c < XS; ++c)
+#pragma unroll
+      for (int v = 0; v < V; ++v) acc[c][v] = make_float2(0.f, 0.f);
+#pragma unroll 1
+    for (int a = 0; a < W; ++a) {
+      const unsigned zo = (unsigned)wrap(c0 + a, g.n[0]) * planelen;
+      float2 s[XS][V];
+#pragma unroll
+      for (int c = 0; c < XS; ++c)
+#pragma unroll
+        for (int v = 0; v < V; ++v) s[c][v] = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int c = 0; c < XS; ++c)
+        if (xok[c]) {
+#pragma unroll
+          for (int b = 0; b < W; ++b) {
+            float2 q[V];
+            load_cells<V>(grid + (zo + yo[b] + xo[c]), q);  // fewer than 2^32 values in a grid
+#pragma unroll
+            for (int v = 0; v < V; ++v) s[c][v] = __ffma2_rn(wy[b], q[v], s[c][v]);
+          }
+        }
+      const float2 wz = make_float2(wt[a], wt[a]);
+#pragma unroll
+      for (int c = 0; c < XS; ++c)
+#pragma unroll
+        for (int v = 0; v < V; ++v) acc[c][v] = __ffma2_rn(wz, s[c][v], acc[c][v]);
+    }
+    float2 r[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      r[v] = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int c = 0; c < XS; ++c)
+        if (xok[c]) {
+          const float w = wt[2 * W + x0 + c * XL];
+          r[v] = __ffma2_rn(make_float2(w, w), acc[c][v], r[v]);
+        }
+    }
+    // add up the group's lanes; while a lane has several transforms, each half keeps half of them
+    int b = V * p, d = C::LANES / 2;
+#pragma unroll
+    for (int h = V / 2; h >= 1; h /= 2, d /= 2) {
+      const bool hi = lane & d;
+#pragma unroll
+      for (int v = 0; v < h; ++v) {
+        const float2 give = hi ? r[v] : r[v + h], keep = hi ? r[v + h] : r[v];
+        r[v] = cadd(keep, make_float2(__shfl_xor_sync(0xffffffffu, give.x, d), __shfl_xor_sync(0xffffffffu, give.y, d)));
+      }
+      b += hi ? h : 0;
+    }
+    const int same = 2 * d;  // lanes that agree above these bits hold the same transform
+#pragma unroll
+    for (; d >= PL; d /= 2)
+      r[0] = cadd(r[0], make_float2(__shfl_xor_sync(0xffffffffu, r[0].x, d), __shfl_xor_sync(0xffffffffu, r[0].y, d)));
+    if (lane % same < PL && w0 + sl < g.K) interp_store(dst, b, nact, NB, i, __float_as_int(pt.w), r[0], csgn);
   }
 }
 
