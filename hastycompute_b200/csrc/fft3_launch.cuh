@@ -139,5 +139,29 @@ inline std::vector<float2> team_tables(const int* n) {
   return tw;
 }
 
+// The same tables computed on the device (FP64), tw [n0 + n1 + n2].
+struct TeamShapes {
+  int n[3], S[3];
+};
+__global__ static void __launch_bounds__(256) team_tables_kernel(TeamShapes s, float2* tw) {
+  const int id = blockIdx.x * blockDim.x + threadIdx.x;
+  const int a = id < s.n[0] ? 0 : id < s.n[0] + s.n[1] ? 1 : 2;
+  const int i = id - (a > 0 ? s.n[0] : 0) - (a > 1 ? s.n[1] : 0);
+  if (i >= s.n[a]) return;
+  const double ang = -2.0 * 3.14159265358979323846 * (double)((i % s.S[a]) * (i / s.S[a])) / (double)s.n[a];
+  tw[id] = make_float2((float)cos(ang), (float)sin(ang));
+}
+inline cudaError_t team_tables_device(const int* n, float2* tw, cudaStream_t st, int kind) {
+  TeamShapes s{};
+  for (int a = 0; a < 3; ++a) {
+    int E = 0;
+    s.n[a] = n[a];
+    if (!team_length(n[a], &E, &s.S[a])) s.S[a] = 1;  // a length-1 axis: the single entry 1
+  }
+  LaunchScope ls(kind, st);
+  team_tables_kernel<<<(n[0] + n[1] + n[2] + 255) / 256, 256, 0, st>>>(s, tw);
+  return cudaGetLastError();
+}
+
 }  // namespace fftl
 }  // namespace hb

@@ -19,7 +19,7 @@
 using namespace hb;
 using hb::fftl::fft3_grid;
 using hb::fftl::team_length;
-using hb::fftl::team_tables;
+using hb::fftl::team_tables_device;
 
 struct hb_nufft {
   int device;
@@ -49,10 +49,9 @@ int width_for_tol(double tol) {
 
 // Gauss-Legendre nodes and weights on [-1, 1] (Newton iteration on the Legendre
 // polynomial, the textbook method), computed once.
-constexpr int kGaussNodes = 64;
-struct GaussLegendre {
-  double x[kGaussNodes], w[kGaussNodes];
-  GaussLegendre() {
+const GaussLegendre& gauss_legendre() {
+  static const GaussLegendre gl = [] {
+    GaussLegendre r;
     const int n = kGaussNodes;
     for (int i = 0; i < n; ++i) {
       double z = std::cos(M_PI * (i + 0.75) / (n + 0.5)), dp = 1.0;
@@ -68,26 +67,12 @@ struct GaussLegendre {
         z -= dz;
         if (std::fabs(dz) < 1e-16) break;
       }
-      x[i] = z;
-      w[i] = 2.0 / ((1.0 - z * z) * dp * dp);
+      r.x[i] = z;
+      r.w[i] = 2.0 / ((1.0 - z * z) * dp * dp);
     }
-  }
-};
-
-// phi_hat(k) = integral over |z| < w/2 of phi(z) cos(2 pi k z / n), by 64-point
-// Gauss-Legendre quadrature on [0, w/2] (the integrand is even); relative error below
-// 1e-11 for the widths of tolerances <= 1e-4.
-double phi_hat(int k, int n, int w, double beta) {
-  static const GaussLegendre gl;
-  const double hw = 0.5 * w;
-  double acc = 0.0;
-  for (int i = 0; i < kGaussNodes; ++i) {
-    const double z = 0.5 * hw * (gl.x[i] + 1.0);
-    const double t = z / hw, s = 1.0 - t * t;
-    const double phi = s > 0.0 ? std::exp(beta * (std::sqrt(s) - 1.0)) : 0.0;
-    acc += gl.w[i] * phi * std::cos(2.0 * M_PI * k * z / n);
-  }
-  return 2.0 * 0.5 * hw * acc;
+    return r;
+  }();
+  return gl;
 }
 
 // Transforms of one group: nact <= NB = 1 << lgnb interleaved grids.  Sizes that are not a
@@ -104,10 +89,13 @@ Group next_group(const hb_nufft* p, int64_t left) {
 
 template <int W>
 cudaError_t spread_reductions_w(const hb_nufft* p, Group q, cudaStream_t st) {
-  const unsigned grid = (unsigned)(((p->g.K << q.lgnb) + 255) / 256);
   LaunchScope ls(HB_KERNEL_NUFFT, st);
-  if (p->g.dim == 3) nufft_spread_reductions_kernel<W, 3><<<grid, 256, 0, st>>>(p->g, p->pts, p->vals, q.lgnb, p->grid);
-  else nufft_spread_reductions_kernel<W, 1><<<grid, 256, 0, st>>>(p->g, p->pts, p->vals, q.lgnb, p->grid);
+  if (p->g.dim == 3) {  // one transform
+    nufft_spread_reductions_kernel<W><<<(unsigned)((p->g.K + 255) / 256), 256, 0, st>>>(p->g, p->pts, p->vals, p->grid);
+  } else {
+    const unsigned grid = (unsigned)(((p->g.K << q.lgnb) + 255) / 256);
+    nufft_spread_line_kernel<W><<<grid, 256, 0, st>>>(p->g, p->pts, p->vals, q.lgnb, p->grid);
+  }
   return cudaGetLastError();
 }
 template <int W>
@@ -329,7 +317,7 @@ int create_plan(hb_nufft** out, int64_t nz, int64_t ny, int64_t nx, const float*
                                           "and >= 2w)");
     g.N[a] = (int)Nv[a];
     g.n[a] = (int)n;
-    g.bin[a] = g.dim == 3 && a < 2 ? 4 : 8;  // every fine-grid length is a multiple of 8
+    g.bin[a] = g.dim == 3 && a < 2 && tiles ? 4 : 8;  // every fine-grid length is a multiple of 8
     g.nb[a] = g.n[a] / g.bin[a];
   }
   DeviceGuard dg(device);
@@ -381,7 +369,7 @@ int create_plan(hb_nufft** out, int64_t nz, int64_t ny, int64_t nx, const float*
   carve(ar);
   carve_tmp(ar_tmp);
 
-  // counting sort of the samples by bin, while the host fills its tables
+  // counting sort of the samples by bin
   const unsigned blocks = (unsigned)((nsamples + 255) / 256);
   if ((e = cudaMemsetAsync(counts, 0, nbins * sizeof(int), st)) != cudaSuccess) return bail(e, "memset");
   {
@@ -424,16 +412,12 @@ int create_plan(hb_nufft** out, int64_t nz, int64_t ny, int64_t nx, const float*
   }
   if ((e = cudaGetLastError()) != cudaSuccess) return bail(e, "binning");
 
-  // host tables: 1/phi_hat per axis and the team twiddles of each fine-grid length
-  std::vector<float> corr;
-  for (int a = 0; a < 3; ++a)
-    for (int i = 0; i < g.N[a]; ++i)
-      corr.push_back(a < 3 - g.dim ? 1.f : (float)(1.0 / phi_hat(i - g.N[a] / 2, g.n[a], g.w, 2.30 * g.w)));
-  const std::vector<float2> tw = team_tables(g.n);
-  if ((e = cudaMemcpyAsync(p->corr, corr.data(), corr.size() * sizeof(float), cudaMemcpyHostToDevice, st)) != cudaSuccess)
-    return bail(e, "upload");
-  if ((e = cudaMemcpyAsync(p->tw, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice, st)) != cudaSuccess)
-    return bail(e, "upload");
+  // tables: 1/phi_hat per axis and the team twiddles of each fine-grid length
+  {
+    LaunchScope ls(HB_KERNEL_NUFFT, st);
+    nufft_corr_kernel<<<(g.N[0] + g.N[1] + g.N[2] + 255) / 256, 256, 0, st>>>(g, 2.30 * g.w, gauss_legendre(), p->corr);
+  }
+  if ((e = team_tables_device(g.n, p->tw, st, HB_KERNEL_NUFFT)) != cudaSuccess) return bail(e, "tables");
   if (ntiles > 0) {
     if ((e = cudaMemcpyAsync(&p->nitems, &nwork->items, sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
         (e = cudaStreamSynchronize(st)) != cudaSuccess)
@@ -471,25 +455,11 @@ int nufft_psf_circulant(const int* M, const float* coords, int64_t nsamples, dou
   hb_nufft* np = nullptr;
   // type 1 over the grid's modes: sum_j exp(+i c_j . d), d in [-M/2, M/2)
   if (int r = create_plan(&np, M[0], M[1], M[2], coords, nsamples, tol, 1, device, st, false)) return r;
-  float2* modes = nullptr;
-  int rc = HB_OK;
-  cudaError_t e = cudaMalloc(&modes, vol * sizeof(float2));
-  if (e == cudaSuccess) {
-    rc = type1_group(np, {nullptr, 0, weights}, plain_modes(modes, vol), {1, 0}, +1, st);
-    if (rc == HB_OK) {
-      LaunchScope ls(HB_KERNEL_DIAG, st);
-      ifftshift3_scale_kernel<<<(unsigned)((vol + 255) / 256), 256, 0, st>>>(modes, M[0], M[1], M[2],
-                                                                             (float)(1.0 / (double)vol), out);
-    }
-    if (rc == HB_OK && (e = cudaGetLastError()) != cudaSuccess)
-      rc = fail(HB_ERR_CUDA, std::string("psf: ") + cudaGetErrorString(e));
-    if (rc == HB_OK && (e = cudaStreamSynchronize(st)) != cudaSuccess)
-      rc = fail(HB_ERR_CUDA, std::string("psf: ") + cudaGetErrorString(e));
-  } else {
-    rc = fail(HB_ERR_CUDA, std::string("psf: ") + cudaGetErrorString(e));
-  }
-  if (rc != HB_OK) cudaStreamSynchronize(st);
-  cudaFree(modes);
+  NufftModeOp op = plain_modes(out, vol);
+  op.circulant = (float)(1.0 / (double)vol);
+  int rc = type1_group(np, {nullptr, 0, weights}, op, {1, 0}, +1, st);
+  const cudaError_t e = cudaStreamSynchronize(st);
+  if (rc == HB_OK && e != cudaSuccess) rc = fail(HB_ERR_CUDA, std::string("psf: ") + cudaGetErrorString(e));
   hb_nufft_destroy(np);
   return rc;
 }
@@ -622,36 +592,34 @@ int hb_diag_build_nufft(const hb_plan* plan, const float* coords, int64_t nsampl
   cudaStream_t st = (cudaStream_t)stream;
   const int M[3] = {2 * N[0], 2 * N[1], 2 * N[2]};
   const long long vol = (long long)M[0] * M[1] * M[2];
-  float2* T = nullptr;
-  float2* tw = nullptr;
+  // T goes straight to the caller's array when that is wanted
+  float2* T = (float2*)T_complex;
+  void* mem = nullptr;
   int rc = HB_OK;
   auto cuda_fail = [&](cudaError_t e, const char* what) {
     rc = fail(HB_ERR_CUDA, std::string("hb_diag_build_nufft: ") + what + ": " + cudaGetErrorString(e));
   };
   do {
     cudaError_t e;
-    if ((e = cudaMalloc(&T, vol * sizeof(float2))) != cudaSuccess) { cuda_fail(e, "alloc"); break; }
-    const std::vector<float2> tables = team_tables(M);
-    if ((e = cudaMalloc(&tw, tables.size() * sizeof(float2))) != cudaSuccess) { cuda_fail(e, "alloc"); break; }
-    if ((e = cudaMemcpyAsync(tw, tables.data(), tables.size() * sizeof(float2), cudaMemcpyHostToDevice, st)) !=
-        cudaSuccess) {
-      cuda_fail(e, "upload");
-      break;
-    }
+    float2* tw = nullptr;
+    auto carve = [&](Arena& ar) {
+      tw = ar.take<float2>(M[0] + M[1] + M[2]);
+      if (!T_complex) T = ar.take<float2>(vol);
+    };
+    Arena size(nullptr);
+    carve(size);
+    if ((e = cudaMalloc(&mem, size.off)) != cudaSuccess) { cuda_fail(e, "alloc"); break; }
+    Arena ar(mem);
+    carve(ar);
+    if ((e = team_tables_device(M, tw, st, HB_KERNEL_DIAG)) != cudaSuccess) { cuda_fail(e, "tables"); break; }
     // PSF in circulant layout on the 2x grid, then T = FFT(PSF)
     if ((rc = nufft_psf_circulant(M, coords, nsamples, tol, weights, dev, T, st)) != HB_OK) break;
     if ((e = fft3_grid<-1>(M[0], M[1], M[2], tw, T, 1, st)) != cudaSuccess) { cuda_fail(e, "fft"); break; }
     if (packed && (rc = hb_diag_pack(plan, T, packed, stream)) != HB_OK) break;
-    if (T_complex &&
-        (e = cudaMemcpyAsync(T_complex, T, vol * sizeof(float2), cudaMemcpyDeviceToDevice, st)) != cudaSuccess) {
-      cuda_fail(e, "copy");
-      break;
-    }
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) cuda_fail(e, "sync");
   } while (false);
   if (rc != HB_OK) cudaStreamSynchronize(st);
-  cudaFree(T);
-  cudaFree(tw);
+  cudaFree(mem);
   return rc;
 }
 

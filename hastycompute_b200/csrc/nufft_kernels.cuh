@@ -36,7 +36,7 @@ constexpr float kNufftInvTwoPi = 0.159154943091895336f;
 struct NufftGeom {
   int N[3];          // modes per axis
   int n[3];          // fine grid per axis (2 N; 1 on a degenerate axis)
-  int bin[3];        // cells per bin: (4, 4, 8), (1, 8, 8) in 2-D, (1, 1, 8) in 1-D
+  int bin[3];        // cells per bin: (4, 4, 8) for spreading by tiles, (8, 8, 8) without; (1, 8, 8) in 2-D, (1, 1, 8) in 1-D
   int nb[3];         // bins per axis
   int w;             // kernel width (cells)
   float beta;        // kernel shape
@@ -192,37 +192,49 @@ __device__ __forceinline__ int nufft_axis(const NufftGeom& g, float u, float* wt
   }
 }
 
-// ---- type 1 by vector reductions into a zeroed grid [n0][n1][n2][NB], NB = 1 << lgnb: one thread
-// per (sample, transform), transform fastest.  Used where the tile form (nufft_spread_kernels.cuh)
-// is not: 1-D plans (a sample has only W cells, fewer than a tile's tests would cost) and the
-// point-spread function, whose thousands of equal terms at the centre of a trajectory round
-// differently when they are summed tile by tile (2e-3 of the diagonal's rms at single
-// entries). ----
-template <int W, int DIM>
-__global__ void __launch_bounds__(256) nufft_spread_reductions_kernel(NufftGeom g, const float4* pts, const float2* vals,
-                                                                      int lgnb, float2* grid) {
-  constexpr int W0 = DIM >= 3 ? W : 1, W1 = DIM >= 2 ? W : 1;
+// ---- type 1 by vector reductions into a zeroed grid.  Used where the tile form
+// (nufft_spread_kernels.cuh) is not: 1-D plans (a sample has only W cells, fewer than a tile's tests
+// would cost) and the point-spread function, whose thousands of equal terms at the centre of a
+// trajectory round differently when they are summed tile by tile (2e-3 of the diagonal's rms at
+// single entries). ----
+// 1-D, grid [n2][NB], NB = 1 << lgnb: one thread per (sample, transform), transform fastest
+template <int W>
+__global__ void __launch_bounds__(256) nufft_spread_line_kernel(NufftGeom g, const float4* pts, const float2* vals,
+                                                                int lgnb, float2* grid) {
   const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int bt = (int)(id & ((1 << lgnb) - 1));
   const long long i = id >> lgnb;
   if (i >= g.K) return;
-  const float2 cj = vals[id];
+  const float2 v = vals[id];
+  float w[W];
+  const int i2 = nufft_axis_weights<W>(pts[i].z, g.beta, w);
+#pragma unroll
+  for (int m = 0; m < W; ++m) red_add(grid + (wrap(i2 + m, g.n[2]) << lgnb) + (id & ((1 << lgnb) - 1)), cscale(v, w[m]));
+}
+// 3-D, one transform: one thread per sample.  (Eight lanes per sample, each the cells of one x, take 409
+// against 1300 us for 512 k samples on 512^3; but the order of the sums decides how the equal terms at
+// the centre round, and that order moves single entries of the diagonal by 1e-3 of its rms.)
+template <int W>
+__global__ void __launch_bounds__(256) nufft_spread_reductions_kernel(NufftGeom g, const float4* pts, const float2* vals,
+                                                                      float2* grid) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= g.K) return;
+  const float2 cj = vals[i];
   const float4 p = pts[i];
-  float w0[W0], w1[W1], w2[W];
-  const int i0 = nufft_axis<W, W0>(g, p.x, w0);
-  const int i1 = nufft_axis<W, W1>(g, p.y, w1);
-  const int i2 = nufft_axis<W, W>(g, p.z, w2);
+  float w0[W], w1[W], w2[W];
+  const int i0 = nufft_axis_weights<W>(p.x, g.beta, w0);
+  const int i1 = nufft_axis_weights<W>(p.y, g.beta, w1);
+  const int i2 = nufft_axis_weights<W>(p.z, g.beta, w2);
   int x2[W];
 #pragma unroll
-  for (int m = 0; m < W; ++m) x2[m] = wrap(i2 + m, g.n[2]) << lgnb;
+  for (int m = 0; m < W; ++m) x2[m] = wrap(i2 + m, g.n[2]);
 #pragma unroll 1
-  for (int a = 0; a < W0; ++a) {
+  for (int a = 0; a < W; ++a) {
     const float2 ca = cscale(cj, w0[a]);
-    float2* Ga = grid + ((long long)wrap(i0 + a, g.n[0]) * g.n[1] * g.n[2] << lgnb) + bt;
+    float2* Ga = grid + (long long)wrap(i0 + a, g.n[0]) * g.n[1] * g.n[2];
 #pragma unroll
-    for (int b = 0; b < W1; ++b) {
+    for (int b = 0; b < W; ++b) {
       const float2 cab = cscale(ca, w1[b]);
-      float2* Gab = Ga + ((long long)wrap(i1 + b, g.n[1]) * g.n[2] << lgnb);
+      float2* Gab = Ga + (long long)wrap(i1 + b, g.n[1]) * g.n[2];
 #pragma unroll
       for (int m = 0; m < W; ++m) red_add(Gab + x2[m], cscale(cab, w2[m]));
     }
@@ -440,16 +452,34 @@ nufft_interp_rows_kernel(NufftGeom g, const float4* pts, const float2* grid, int
   }
 }
 
-// ---- Toeplitz diagonal through the NUFFT ----
-// Circulant (ifftshift) layout of a centred [M0][M1][M2] array, scaled:
-// out[n] = s * in[(n + M/2) mod M] per axis (offset d = n for n < M/2, n - M otherwise).
-__global__ void ifftshift3_scale_kernel(const float2* in, int M0, int M1, int M2, float s, float2* out) {
-  const long long nv = (long long)M0 * M1 * M2;
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nv) return;
-  const int n2 = (int)(i % M2), n1 = (int)((i / M2) % M1), n0 = (int)(i / ((long long)M1 * M2));
-  const int c0 = (n0 + M0 / 2) % M0, c1 = (n1 + M1 / 2) % M1, c2 = (n2 + M2 / 2) % M2;
-  out[i] = cscale(in[((long long)c0 * M1 + c1) * M2 + c2], s);
+// ---- tables (once per plan): corr = 1/phi_hat per axis [N0 | N1 | N2], team twiddles of n0, n1, n2 ----
+// phi_hat(k) = integral over |z| < w/2 of phi(z) cos(2 pi k z / n), by 64-point Gauss-Legendre quadrature on
+// [0, w/2] (the integrand is even); relative error below 1e-11 for the widths of tolerances <= 1e-4.
+// In FP64 on the device: on the host the 64 x (N0 + N1 + N2) exponentials and cosines took 3 ms for a 256^3 plan.
+constexpr int kGaussNodes = 64;
+struct GaussLegendre {
+  double x[kGaussNodes], w[kGaussNodes];
+};
+__global__ void __launch_bounds__(256) nufft_corr_kernel(NufftGeom g, double beta, const __grid_constant__ GaussLegendre gl,
+                                                         float* corr) {
+  const int id = blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= g.N[0] + g.N[1] + g.N[2]) return;
+  const int a = id < g.N[0] ? 0 : id < g.N[0] + g.N[1] ? 1 : 2;
+  if (a < 3 - g.dim) {
+    corr[id] = 1.f;
+    return;
+  }
+  const int i = id - (a > 0 ? g.N[0] : 0) - (a > 1 ? g.N[1] : 0);
+  const int k = i - g.N[a] / 2, n = g.n[a];
+  const double hw = 0.5 * g.w;
+  double acc = 0.0;
+  for (int j = 0; j < kGaussNodes; ++j) {
+    const double z = 0.5 * hw * (gl.x[j] + 1.0);
+    const double t = z / hw, s = 1.0 - t * t;
+    const double phi = s > 0.0 ? exp(beta * (sqrt(s) - 1.0)) : 0.0;
+    acc += gl.w[j] * phi * cos(2.0 * 3.14159265358979323846 * k * z / n);
+  }
+  corr[id] = (float)(1.0 / (hw * acc));  // 2 x (hw / 2) x the sum
 }
 
 }  // namespace hb

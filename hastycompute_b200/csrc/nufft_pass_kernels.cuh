@@ -138,6 +138,7 @@ nufft_axis_pass_kernel(float2* grid, long long row_stride, int ncols, int outer_
 struct NufftModeOp {
   float2* f;         // plain modes (read by type 2, written by type 1); null selects the coil form
   long long f_ld;
+  float circulant;   // nonzero: type 1 writes circulant order (offset d at d mod N) times this factor
   const float2* x;   // coil form, type 2: the image
   float2* out;       // coil form, type 1: the combined image
   int accumulate;    // coil form, type 1: add to out
@@ -254,7 +255,12 @@ nufft_grid_to_modes_kernel(NufftGeom g, const __grid_constant__ NufftModeOp op, 
       if (b >= nact) continue;
       float2 v = cscale(tile[tile_at(r, c)], s);
       v.y *= sgn;
-      op.f[b * op.f_ld + m] = v;
+      if (op.circulant != 0.f) {
+        const int j0 = (i0 + g.N[0] / 2) % g.N[0], j1 = (i1 + g.N[1] / 2) % g.N[1], j2 = (i2 + N2 / 2) % N2;
+        op.f[((long long)j0 * g.N[1] + j1) * N2 + j2] = cscale(v, op.circulant);
+      } else {
+        op.f[b * op.f_ld + m] = v;
+      }
     } else {
       float2 acc = op.accumulate ? op.out[m] : make_float2(0.f, 0.f);
       for (int b = 0; b < nact; ++b) {
