@@ -98,6 +98,9 @@ SIGNATURES = {
     "hb_sense_normal_nufft": (c_int, [c_void_p, c_void_p, c_void_p, P_i64, c_i64, c_void_p, c_void_p, c_void_p,
                                       c_int, c_void_p]),
     "hb_diag_build_nufft": (c_int, [c_void_p, c_void_p, c_i64, c_double, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "hb_diag_build_nufft_workspace_bytes": (c_size, [c_void_p, c_i64, c_double]),
+    "hb_diag_build_nufft_ws": (c_int, [c_void_p, c_void_p, c_i64, c_double, c_void_p, c_void_p, c_void_p, c_void_p,
+                                       c_size, c_void_p]),
     "hb_sense_forward_nufft": (c_int, [c_void_p, c_void_p, c_void_p, P_i64, c_i64, c_void_p, c_void_p]),
     "hb_precond_build": (c_int, [c_void_p, c_void_p, c_i64, c_double, c_void_p, P_i64, c_i64, c_float, c_void_p,
                                  c_void_p]),

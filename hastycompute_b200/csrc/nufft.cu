@@ -25,7 +25,7 @@ struct hb_nufft {
   int device;
   NufftGeom g;
   int group;                // transforms interleaved in the grid at once: 1, 2, 4 or 8
-  void* mem = nullptr;        // one allocation: the arrays below up to vals
+  void* mem = nullptr;        // one allocation (null: in the creator's workspace): the arrays below up to vals
   float4* pts = nullptr;      // [K] grid positions and sample numbers in bin order
   int* start = nullptr;       // [bins + 1] first position of every bin
   float* corr = nullptr;      // [N0 | N1 | N2] 1 / phi_hat
@@ -287,12 +287,16 @@ void free_plan(hb_nufft* p) {
   delete p;
 }
 
-// hb_nufft_create; tiles = false leaves out the tile work lists (spread by reductions only)
+// hb_nufft_create; tiles = false leaves out the tile work lists (spread by reductions only).  With
+// `external` the plan's arrays and the temporaries of the sort are taken from that arena, which
+// outlives the plan, and nothing waits for the stream; a dry arena (base null) measures them and
+// creates nothing.
 int create_plan(hb_nufft** out, int64_t nz, int64_t ny, int64_t nx, const float* coords, int64_t nsamples, double tol,
-                int maxbatch, int device, void* stream, bool tiles) {
+                int maxbatch, int device, void* stream, bool tiles, Arena* external = nullptr) {
   if (!out) return fail(HB_ERR_INVALID, "hb_nufft_create: null output");
   *out = nullptr;
-  if (!coords || nsamples < 1 || nsamples > (int64_t)0x7fffffff)
+  const bool dry = external && !external->base;
+  if ((!coords && !dry) || nsamples < 1 || nsamples > (int64_t)0x7fffffff)
     return fail(HB_ERR_INVALID, "hb_nufft_create: need coords and 1 <= nsamples < 2^31");
   if (!(tol > 0.0 && tol < 1.0)) return fail(HB_ERR_INVALID, "hb_nufft_create: tol must be in (0, 1)");
   if (maxbatch < 1 || maxbatch > kNufftMaxBatch)
@@ -359,15 +363,24 @@ int create_plan(hb_nufft** out, int64_t nz, int64_t ny, int64_t nx, const float*
     candidates = ar.take<int>(ntiles);
     nwork = ar.take<SpreadCounts>(1);
   };
-  Arena size(nullptr), size_tmp(nullptr);
-  carve(size);
-  carve_tmp(size_tmp);
   cudaError_t e;
-  if ((e = cudaMalloc(&p->mem, size.off)) != cudaSuccess) return bail(e, "plan arrays and fine grid");
-  if ((e = cudaMalloc(&tmp, size_tmp.off)) != cudaSuccess) return bail(e, "sort temporaries");
-  Arena ar(p->mem), ar_tmp(tmp);
-  carve(ar);
-  carve_tmp(ar_tmp);
+  if (external) {
+    carve(*external);
+    carve_tmp(*external);
+    if (dry) {
+      delete p;
+      return HB_OK;
+    }
+  } else {
+    Arena size(nullptr), size_tmp(nullptr);
+    carve(size);
+    carve_tmp(size_tmp);
+    if ((e = cudaMalloc(&p->mem, size.off)) != cudaSuccess) return bail(e, "plan arrays and fine grid");
+    if ((e = cudaMalloc(&tmp, size_tmp.off)) != cudaSuccess) return bail(e, "sort temporaries");
+    Arena ar(p->mem), ar_tmp(tmp);
+    carve(ar);
+    carve_tmp(ar_tmp);
+  }
 
   // counting sort of the samples by bin
   const unsigned blocks = (unsigned)((nsamples + 255) / 256);
@@ -439,7 +452,7 @@ int create_plan(hb_nufft** out, int64_t nz, int64_t ny, int64_t nx, const float*
     if ((e = cudaMemcpyAsync(&p->nsplit, &nwork->split_tiles, sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
       return bail(e, "spread items");
   }
-  if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return bail(e, "binning");
+  if (!external && (e = cudaStreamSynchronize(st)) != cudaSuccess) return bail(e, "binning");
   cudaFree(tmp);
   *out = p;
   return HB_OK;
@@ -449,18 +462,37 @@ int create_plan(hb_nufft** out, int64_t nz, int64_t ny, int64_t nx, const float*
 
 namespace hb {
 
-int nufft_psf_circulant(const int* M, const float* coords, int64_t nsamples, double tol, const float* weights,
-                        int device, float2* out, cudaStream_t st) {
+// The NUFFT plan of the point-spread function on an M grid, in `ar` (measured only when ar is dry)
+static int psf_plan(hb_nufft** np, const int* M, const float* coords, int64_t nsamples, double tol, int device,
+                    cudaStream_t st, Arena& ar) {
+  // type 1 over the grid's modes: sum_j exp(+i c_j . d), d in [-M/2, M/2)
+  return create_plan(np, M[0], M[1], M[2], coords, nsamples, tol, 1, device, st, false, &ar);
+}
+
+static int psf_in(const int* M, const float* coords, int64_t nsamples, double tol, const float* weights, int device,
+                  float2* out, cudaStream_t st, Arena& ar) {
   const long long vol = (long long)M[0] * M[1] * M[2];
   hb_nufft* np = nullptr;
-  // type 1 over the grid's modes: sum_j exp(+i c_j . d), d in [-M/2, M/2)
-  if (int r = create_plan(&np, M[0], M[1], M[2], coords, nsamples, tol, 1, device, st, false)) return r;
+  if (int r = psf_plan(&np, M, coords, nsamples, tol, device, st, ar)) return r;
   NufftModeOp op = plain_modes(out, vol);
   op.circulant = (float)(1.0 / (double)vol);
-  int rc = type1_group(np, {nullptr, 0, weights}, op, {1, 0}, +1, st);
+  const int rc = type1_group(np, {nullptr, 0, weights}, op, {1, 0}, +1, st);
+  free_plan(np);  // host state only: its arrays are the arena's
+  return rc;
+}
+
+int nufft_psf_circulant(const int* M, const float* coords, int64_t nsamples, double tol, const float* weights,
+                        int device, float2* out, cudaStream_t st) {
+  Arena size(nullptr);
+  hb_nufft* none = nullptr;
+  if (int r = psf_plan(&none, M, nullptr, nsamples, tol, device, st, size)) return r;
+  void* mem = nullptr;
+  HB_CUDA(cudaMalloc(&mem, size.off));
+  Arena ar(mem);
+  int rc = psf_in(M, coords, nsamples, tol, weights, device, out, st, ar);
   const cudaError_t e = cudaStreamSynchronize(st);
   if (rc == HB_OK && e != cudaSuccess) rc = fail(HB_ERR_CUDA, std::string("psf: ") + cudaGetErrorString(e));
-  hb_nufft_destroy(np);
+  cudaFree(mem);
   return rc;
 }
 
@@ -582,6 +614,51 @@ int hb_sense_normal_nufft(const hb_nufft* plan, const void* x, const void* smaps
   return HB_OK;
 }
 
+// Scratch of a diagonal build: twiddles, T (unless the caller's array takes it) and the NUFFT plan.
+// Returns an error code; with a dry arena it only measures.
+static int diag_scratch(const hb_plan* plan, int64_t nsamples, double tol, bool own_T, cudaStream_t st, Arena& ar,
+                        float2** tw, float2** T) {
+  int N[3], dev = 0;
+  plan_geometry(plan, N, &dev);
+  const int M[3] = {2 * N[0], 2 * N[1], 2 * N[2]};
+  *tw = ar.take<float2>(M[0] + M[1] + M[2]);
+  if (own_T) *T = ar.take<float2>((size_t)M[0] * M[1] * M[2]);
+  if (ar.base) return HB_OK;
+  hb_nufft* none = nullptr;
+  return psf_plan(&none, M, nullptr, nsamples, tol, dev, st, ar);
+}
+
+size_t hb_diag_build_nufft_workspace_bytes(const hb_plan* plan, int64_t nsamples, double tol) {
+  if (!plan || nsamples < 1) return 0;
+  Arena size(nullptr);
+  float2 *tw = nullptr, *T = nullptr;
+  return diag_scratch(plan, nsamples, tol, true, nullptr, size, &tw, &T) == HB_OK ? size.off + 256 : 0;
+}
+
+int hb_diag_build_nufft_ws(const hb_plan* plan, const float* coords, int64_t nsamples, double tol, const float* weights,
+                           float* packed, void* T_complex, void* ws, size_t ws_bytes, void* stream) {
+  if (!plan || !coords || nsamples < 1) return fail(HB_ERR_INVALID, "hb_diag_build_nufft: null plan or no samples");
+  if (!packed && !T_complex) return fail(HB_ERR_INVALID, "hb_diag_build_nufft: no output requested");
+  int N[3], dev = 0;
+  plan_geometry(plan, N, &dev);
+  DeviceGuard dg(dev);
+  cudaStream_t st = (cudaStream_t)stream;
+  const int M[3] = {2 * N[0], 2 * N[1], 2 * N[2]};
+  float2 *tw = nullptr, *T = (float2*)T_complex;  // T goes straight to the caller's array when that is wanted
+  Arena size(nullptr);
+  if (int r = diag_scratch(plan, nsamples, tol, !T_complex, st, size, &tw, &T)) return r;
+  if (!ws || ws_bytes < size.off) return fail(HB_ERR_WORKSPACE, "hb_diag_build_nufft: workspace too small");
+  if (((uintptr_t)ws & 255u) != 0) return fail(HB_ERR_INVALID, "hb_diag_build_nufft: workspace not 256-byte aligned");
+  Arena ar(ws);
+  T = (float2*)T_complex;
+  if (int r = diag_scratch(plan, nsamples, tol, !T_complex, st, ar, &tw, &T)) return r;
+  HB_CUDA(team_tables_device(M, tw, st, HB_KERNEL_DIAG));
+  // PSF in circulant layout on the 2x grid, then T = FFT(PSF)
+  if (int r = psf_in(M, coords, nsamples, tol, weights, dev, T, st, ar)) return r;
+  HB_CUDA(fft3_grid<-1>(M[0], M[1], M[2], tw, T, 1, st));
+  return packed ? hb_diag_pack(plan, T, packed, stream) : HB_OK;
+}
+
 int hb_diag_build_nufft(const hb_plan* plan, const float* coords, int64_t nsamples, double tol, const float* weights,
                         float* packed, void* T_complex, void* stream) {
   if (!plan || !coords || nsamples < 1) return fail(HB_ERR_INVALID, "hb_diag_build_nufft: null plan or no samples");
@@ -590,35 +667,15 @@ int hb_diag_build_nufft(const hb_plan* plan, const float* coords, int64_t nsampl
   plan_geometry(plan, N, &dev);
   DeviceGuard dg(dev);
   cudaStream_t st = (cudaStream_t)stream;
-  const int M[3] = {2 * N[0], 2 * N[1], 2 * N[2]};
-  const long long vol = (long long)M[0] * M[1] * M[2];
-  // T goes straight to the caller's array when that is wanted
-  float2* T = (float2*)T_complex;
+  float2 *tw = nullptr, *T = nullptr;
+  Arena size(nullptr);
+  if (int r = diag_scratch(plan, nsamples, tol, !T_complex, st, size, &tw, &T)) return r;
   void* mem = nullptr;
-  int rc = HB_OK;
-  auto cuda_fail = [&](cudaError_t e, const char* what) {
-    rc = fail(HB_ERR_CUDA, std::string("hb_diag_build_nufft: ") + what + ": " + cudaGetErrorString(e));
-  };
-  do {
-    cudaError_t e;
-    float2* tw = nullptr;
-    auto carve = [&](Arena& ar) {
-      tw = ar.take<float2>(M[0] + M[1] + M[2]);
-      if (!T_complex) T = ar.take<float2>(vol);
-    };
-    Arena size(nullptr);
-    carve(size);
-    if ((e = cudaMalloc(&mem, size.off)) != cudaSuccess) { cuda_fail(e, "alloc"); break; }
-    Arena ar(mem);
-    carve(ar);
-    if ((e = team_tables_device(M, tw, st, HB_KERNEL_DIAG)) != cudaSuccess) { cuda_fail(e, "tables"); break; }
-    // PSF in circulant layout on the 2x grid, then T = FFT(PSF)
-    if ((rc = nufft_psf_circulant(M, coords, nsamples, tol, weights, dev, T, st)) != HB_OK) break;
-    if ((e = fft3_grid<-1>(M[0], M[1], M[2], tw, T, 1, st)) != cudaSuccess) { cuda_fail(e, "fft"); break; }
-    if (packed && (rc = hb_diag_pack(plan, T, packed, stream)) != HB_OK) break;
-    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) cuda_fail(e, "sync");
-  } while (false);
-  if (rc != HB_OK) cudaStreamSynchronize(st);
+  HB_CUDA(cudaMalloc(&mem, size.off));
+  int rc = hb_diag_build_nufft_ws(plan, coords, nsamples, tol, weights, packed, T_complex, mem, size.off, stream);
+  const cudaError_t e = cudaStreamSynchronize(st);
+  if (rc == HB_OK && e != cudaSuccess)
+    rc = fail(HB_ERR_CUDA, std::string("hb_diag_build_nufft: ") + cudaGetErrorString(e));
   cudaFree(mem);
   return rc;
 }

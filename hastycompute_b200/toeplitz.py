@@ -163,8 +163,13 @@ class ToeplitzPlan:
             if weights.numel() != K:
                 raise RuntimeError("weights must hold one value per sample")
         if method == "nufft":
-            capi.check(self.lib.hb_diag_build_nufft(self._h, _ptr(coords), K, float(tol), _ptr(weights), _ptr(packed),
-                                                    _ptr(T), _stream_ptr(self.device)))
+            # scratch (a NUFFT plan, 1.2 GB at 128^3) from torch's caching allocator: a cudaMalloc and its
+            # cudaFree took 3 to 30 ms of a call whose kernels take 2.4 ms
+            nb = int(self.lib.hb_diag_build_nufft_workspace_bytes(self._h, K, float(tol)))
+            ws = torch.empty(max(nb, 256), dtype=torch.uint8, device=self.device)
+            capi.check(self.lib.hb_diag_build_nufft_ws(self._h, _ptr(coords), K, float(tol), _ptr(weights), _ptr(packed),
+                                                       _ptr(T), _ptr(ws), ws.numel(), _stream_ptr(self.device)))
+            torch.cuda.current_stream(self.device).synchronize()  # the outputs are ready for any stream
         elif method == "exact":
             nb = self.lib.hb_diag_build_workspace_bytes(self._h, K)
             ws = torch.empty(int(nb), dtype=torch.uint8, device=self.device)

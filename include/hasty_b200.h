@@ -348,6 +348,12 @@ int hb_sense_normal_nufft(const hb_nufft* plan, const void* x, const void* smaps
  * complex64 fine grid) for the duration of the call and synchronises `stream`. */
 int hb_diag_build_nufft(const hb_plan* plan, const float* coords, int64_t nsamples, double tol, const float* weights,
                         float* packed, void* T_complex, void* stream);
+/* The same with the caller's workspace (256-byte aligned, hb_diag_build_nufft_workspace_bytes; 0 for
+ * sizes or tolerances the NUFFT does not take): allocates nothing and does not wait for `stream`, so the
+ * workspace must stay until the stream has passed the build. */
+size_t hb_diag_build_nufft_workspace_bytes(const hb_plan* plan, int64_t nsamples, double tol);
+int hb_diag_build_nufft_ws(const hb_plan* plan, const float* coords, int64_t nsamples, double tol, const float* weights,
+                           float* packed, void* T_complex, void* workspace, size_t workspace_bytes, void* stream);
 
 /* SENSE forward: kdata[b] = type2(S[coils[b]] * x) (isign -1). */
 int hb_sense_forward_nufft(const hb_nufft* plan, const void* x, const void* smaps, const int64_t* coils,

@@ -240,3 +240,30 @@ def test_spreading_crowded_and_empty_tiles(cuda, shape, tol, nt):
     f, ref = _np(plan.type1(_c64(c, cuda))), O.nudft_type1(coords, c, shape, +1)
     for t in range(nt):
         assert O.rel_l2(f[t], ref[t]) < max(10 * tol, 1e-5 + 1.41e-7 * 2 * max(shape))
+
+
+def test_diagonal_in_a_caller_workspace(cuda):
+    """hb_diag_build_nufft_ws against hb_diag_build_nufft (to reduction order), its workspace size, and
+    what it refuses."""
+    import ctypes
+
+    shape = (16, 8, 32)
+    plan = ToeplitzPlan(shape, cuda)
+    lib, st = plan.lib, torch.cuda.current_stream(cuda).cuda_stream
+    coords = torch.from_numpy(_coords(3000, 71)).to(cuda)
+    w = torch.rand(3000, device=cuda)
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    a = torch.empty(plan.packed_numel(), device=cuda)
+    b = torch.empty_like(a)
+    T = torch.empty(plan.grid, dtype=torch.complex64, device=cuda)
+    capi.check(lib.hb_diag_build_nufft(plan._h, ptr(coords), 3000, 1e-6, ptr(w), ptr(a), None, st))
+    nb = lib.hb_diag_build_nufft_workspace_bytes(plan._h, 3000, 1e-6)
+    ws = torch.empty(nb, dtype=torch.uint8, device=cuda)
+    capi.check(lib.hb_diag_build_nufft_ws(plan._h, ptr(coords), 3000, 1e-6, ptr(w), ptr(b), ptr(T), ptr(ws), nb, st))
+    assert float((a - b).norm() / a.norm()) < 1e-6
+    assert float((plan.pack_diagonal(T) - b).norm() / a.norm()) < 1e-6
+    assert lib.hb_diag_build_nufft_ws(plan._h, ptr(coords), 3000, 1e-6, None, ptr(b), None, ptr(ws), 1000, st) == \
+        capi.HB_ERR_WORKSPACE
+    assert lib.hb_diag_build_nufft_ws(plan._h, ptr(coords), 3000, 1e-6, None, None, None, ptr(ws), nb, st) == \
+        capi.HB_ERR_INVALID
+    assert lib.hb_diag_build_nufft_workspace_bytes(plan._h, 3000, 2.0) == 0
