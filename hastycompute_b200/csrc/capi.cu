@@ -14,6 +14,7 @@
 #include "cg_kernels.cuh"
 #include "diag_kernels.cuh"
 #include "fft3_launch.cuh"
+#include "plane_full_kernels.cuh"
 #include "plane_odd_kernels.cuh"
 #include "runtime.cuh"
 #include "tc_kernels.cuh"
@@ -248,6 +249,16 @@ cudaError_t launch_bodd(const PassArgs& a, int nslots, cudaStream_t st) {
   return launch_plane_clusters<plane_odd_kernel<K, THREADS>>(a, nslots, K, THREADS, smem, st);
 }
 
+template <int N0, int N1, int THREADS>
+cudaError_t launch_bfull(const PassArgs& a, int nslots, cudaStream_t st) {
+  constexpr size_t smem = PlaneFullCfg<N0, N1, THREADS>::SMEM_F2 * sizeof(float2);
+  cudaError_t e = ensure_smem<plane_full_kernel<N0, N1, THREADS>>(smem);
+  if (e != cudaSuccess) return e;
+  LaunchScope ls(HB_KERNEL_PLANE_YZ, st);
+  plane_full_kernel<N0, N1, THREADS><<<dim3(nslots, 2 * a.N2), THREADS, smem, st>>>(a);
+  return cudaGetLastError();
+}
+
 // Plane-pass schedules (cluster split Q x CTA size) per plane size; hb_plan_autotune
 // times them, HB_PLANE_VARIANT overrides, index 0 is the default.
 struct PlaneVariant {
@@ -262,10 +273,8 @@ const PlaneVariant kPlane128[] = {
     {"mod8t256", &launch_bmod<128, 128, 8, 256>}, {"mod8t128", &launch_bmod<128, 128, 8, 128>},
 };
 const PlaneVariant kPlane64[] = {
-    {"q1t256", &launch_b<64, 64, 1, 256>}, {"q2t128", &launch_b<64, 64, 2, 128>},
-    {"q1t128", &launch_b<64, 64, 1, 128>}, {"q2t256", &launch_b<64, 64, 2, 256>},
-    {"mod4t256", &launch_bmod<64, 64, 4, 256>}, {"mod4t128", &launch_bmod<64, 64, 4, 128>},
-    {"mod8t128", &launch_bmod<64, 64, 8, 128>},
+    {"full256", &launch_bfull<64, 64, 256>}, {"full512", &launch_bfull<64, 64, 512>},
+    {"full128", &launch_bfull<64, 64, 128>},
 };
 const PlaneVariant kPlane96[] = {{"odd3t128", &launch_bodd<3, 128>}};
 const PlaneVariant kPlane160[] = {{"odd5t256", &launch_bodd<5, 256>}};
@@ -273,7 +282,7 @@ const PlaneVariant kPlane160[] = {{"odd5t256", &launch_bodd<5, 256>}};
 const PlaneVariant* plane_variants(int N0, int N1, int* n) {
   *n = 0;
   if (N0 == 128 && N1 == 128) { *n = 10; return kPlane128; }
-  if (N0 == 64 && N1 == 64) { *n = 7; return kPlane64; }
+  if (N0 == 64 && N1 == 64) { *n = 3; return kPlane64; }
   if (N0 == 96 && N1 == 96) { *n = 1; return kPlane96; }
   if (N0 == 160 && N1 == 160) { *n = 1; return kPlane160; }
   return nullptr;
@@ -296,10 +305,19 @@ const PassLauncher kLaunchA[7][2] = {HB_XROW(8, launch_a),   HB_XROW(16, launch_
 const PassLauncher kLaunchC[7][2] = {HB_XROW(8, launch_c),   HB_XROW(16, launch_c), HB_XROW(32, launch_c),
                                      HB_XROW(64, launch_c),  HB_XROW(128, launch_c), HB_XROW(96, launch_c),
                                      HB_XROW(160, launch_c)};
-#define HB_BROW(N0)                                                                                    \
-  {&launch_b<N0, 8, 1, 128>, &launch_b<N0, 16, 1, 128>, &launch_b<N0, 32, 1, 128>, &launch_b<N0, 64, 1, 256>, \
-   &launch_b<N0, 128, 1, 512>}
-const PassLauncher kLaunchB[5][5] = {HB_BROW(8), HB_BROW(16), HB_BROW(32), HB_BROW(64), HB_BROW(128)};
+// Planes of powers of two other than 128 x 128 fit one CTA.  128 threads where 256 would leave teams without
+// a row (measured, 128 kx planes of 1 / 16 slots, us, 256 against 128 threads: 16 x 64 4.6 / 33.5
+// against 4.6 / 25.1, 32 x 16 3.3 / 19.1 against 3.3 / 14.6; 32 x 32 3.9 / 24.4 against 4.6 / 23.8,
+// 64 x 64 9.8 / 99.6 against 12.4 / 110).
+constexpr int full_threads(int N0, int N1) { return N0 * N1 <= (N0 < 32 ? 1024 : 512) ? 128 : 256; }
+#define HB_BROW(N0)                                                                                          \
+  &launch_bfull<N0, 8, full_threads(N0, 8)>, &launch_bfull<N0, 16, full_threads(N0, 16)>,                    \
+      &launch_bfull<N0, 32, full_threads(N0, 32)>, &launch_bfull<N0, 64, full_threads(N0, 64)>
+const PassLauncher kLaunchB[5][5] = {{HB_BROW(8), &launch_bfull<8, 128, full_threads(8, 128)>},
+                                     {HB_BROW(16), &launch_bfull<16, 128, full_threads(16, 128)>},
+                                     {HB_BROW(32), &launch_bfull<32, 128, full_threads(32, 128)>},
+                                     {HB_BROW(64), &launch_bfull<64, 128, full_threads(64, 128)>},
+                                     {HB_BROW(128), nullptr}};  // 128 x 128 has its own schedules
 
 PassLauncher plane_launcher(const hb_plan* p) {
   int n = 0;
@@ -1445,7 +1463,7 @@ const char* hb_plan_plane_schedule(const hb_plan* p) {
   if (!p) return "";
   int n = 0;
   const PlaneVariant* v = plane_variants(p->N0, p->N1, &n);
-  if (!v) return "plane_yz:q1";
+  if (!v) return "full";
   return v[plane_variant_index(n, p->plane_variant)].name;
 }
 

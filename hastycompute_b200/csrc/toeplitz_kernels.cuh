@@ -86,6 +86,12 @@ struct SpillPlane {
     lo = swap ? make_float2(w.z, w.w) : make_float2(w.x, w.y);
     hi = swap ? make_float2(w.x, w.y) : make_float2(w.z, w.w);
   }
+  // the same as one 16-byte store
+  __device__ __forceinline__ void put_pair(int z, int y, float2 lo, float2 hi) const {
+    const bool swap = sw & 1;
+    *reinterpret_cast<float4*>(base + (z * (int)rs + (y / YT) * (int)cs + ((2 * (y % (YT / 2))) ^ (sw & ~1)))) =
+        swap ? make_float4(hi.x, hi.y, lo.x, lo.y) : make_float4(lo.x, lo.y, hi.x, hi.y);
+  }
 };
 
 // ---------------------------------------------------------------- launch geometry ----

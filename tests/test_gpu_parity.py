@@ -306,6 +306,25 @@ def test_sense_normal_non_power_of_two(cuda, shape, ncoil):
     assert O.rel_l2(_np(out), ref) < TOL
 
 
+@pytest.mark.parametrize("n0,n1", [(8, 8), (8, 128), (128, 8), (16, 64), (32, 16), (32, 32), (64, 16), (64, 64),
+                                   (64, 128), (128, 64)])
+def test_one_cta_planes(cuda, n0, n1):
+    """Every (team length, CTA size, pair or single loads) combination of the planes that one CTA
+    holds, with a diagonal per system."""
+    shape = (n0, n1, 8)
+    plan = ToeplitzPlan(shape, cuda)
+    rng = np.random.default_rng(56)
+    T = rng.standard_normal((2, 2 * n0, 2 * n1, 16)) + 1.0
+    packed = torch.stack([plan.pack_diagonal(_c64(t, cuda)) for t in T])
+    sm = synth.coil_maps(3, shape, seed=57)
+    x = np.stack([synth.gaussian_image(shape, seed=s) for s in (58, 59)])
+    out = torch.empty(x.shape, dtype=torch.complex64, device=cuda)
+    plan.sense_normal(_c64(x, cuda), out, _c64(sm, cuda), packed, diag_index=[1, 0])
+    for i in range(2):
+        ref = O.sense_normal_toeplitz_t(_c64(x[i], cuda), _c64(sm, cuda), torch.from_numpy(T[1 - i]).to(cuda))
+        assert O.rel_l2(out[i], ref) < TOL, i
+
+
 @pytest.mark.parametrize("shape", [(96, 96, 8), (160, 160, 16)])
 def test_odd_planes_with_a_diagonal_per_system(cuda, shape):
     """The 96- and 160-point planes (frequency residues mod 3 and mod 5) with several systems, each its
