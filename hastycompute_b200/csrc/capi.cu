@@ -1,6 +1,7 @@
 // C ABI of the B200 Toeplitz SENSE normal operator and batched CG (include/hasty_b200.h).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 #include <cmath>
@@ -153,15 +154,24 @@ std::vector<uint16_t> tc_dft_table(int N2) {
   return t;
 }
 
+// A pass-A CTA owns a tile of lines and loops over the system's coils; a small call leaves most SMs without
+// one, so its coils are shared by up to this many CTAs in all (four per SM; the tiles of a coil do not
+// depend on who makes them).  Measured: 64^3 x 8 coils 15.7 -> 12.5 us, x 16 coils 28.8 -> 22.3 us, 32^3 x 8
+// 9.5 -> 4.3 us; eight or sixteen per SM 13.0 and 13.5 us at 64^3 x 8.
+constexpr long long kXPassCtas = 148 * 4;
 template <int N2, int YT>
 cudaError_t launch_a(const PassArgs& a, int nsys, cudaStream_t st) {
   using C = XPassCfg<N2, YT>;
   const size_t smem = C::SMEM_F2 * sizeof(float2);
   cudaError_t e = ensure_smem<expand_fwd_x_kernel<N2, YT>>(smem);
   if (e != cudaSuccess) return e;
-  dim3 grid(a.N1 / YT, a.N0, nsys);
+  const long long ctas = (long long)(a.N1 / YT) * a.N0 * nsys, want = kXPassCtas;
+  const int coils = a.nslots / nsys;  // on average
+  PassArgs b = a;
+  b.x_parts = ctas >= want ? 1 : (int)std::max<long long>(1, std::min<long long>(coils, want / ctas));
+  dim3 grid(a.N1 / YT, a.N0, nsys * b.x_parts);
   LaunchScope ls(HB_KERNEL_EXPAND_FWD_X, st);
-  expand_fwd_x_kernel<N2, YT><<<grid, C::THREADS, smem, st>>>(a);
+  expand_fwd_x_kernel<N2, YT><<<grid, C::THREADS, smem, st>>>(b);
   return cudaGetLastError();
 }
 

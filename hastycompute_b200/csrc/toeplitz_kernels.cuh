@@ -216,6 +216,7 @@ struct PassArgs {
   int accumulate;                  // 1: out += result, 0: out = result
   double* dot_partials;            // [nsys][nblocks_c] Re<x, out> partials (nullable)
   int prefetch_ahead;              // mod-4 plane pass: L2-prefetch distance in clusters (0 = off)
+  int x_parts;                     // pass A: CTAs that share a tile's coils
   int inject_stall;                // tests only: pass C omits the tile copy of coil index
                                    // inject_stall - 1 of every system (0 = off)
 };
@@ -234,8 +235,12 @@ expand_fwd_x_kernel(PassArgs a) {
   float2* smt = tile + C::TILE;       // 2 x [YT][N2] coil-map stages
   float2* tw = smt + 2 * C::SMT;      // [M2]
 
-  const int sys = blockIdx.z;
+  // part `part` of the system's coils (x_parts: 1 unless the call is small)
+  const int sys = blockIdx.z / a.x_parts, part = blockIdx.z % a.x_parts;
   if (a.active && !a.active[sys]) return;
+  const int coils = a.sys_nslot[sys], coil0 = coils * part / a.x_parts;
+  const int ncoil = coils * (part + 1) / a.x_parts - coil0;
+  if (ncoil == 0) return;
   const int z = blockIdx.y;
   const int y0 = blockIdx.x * YT;
   const int N0 = a.N0, N1 = a.N1;
@@ -246,7 +251,7 @@ expand_fwd_x_kernel(PassArgs a) {
   float2* buf = tile + team * C::TBUF;
   const long long plane = (long long)N1 * N2;
   const float2* sm = a.sys_smaps[sys];
-  const int slot0 = a.sys_slot0[sys], ncoil = a.sys_nslot[sys];
+  const int slot0 = a.sys_slot0[sys] + coil0;
   // Coil ci's map rows [y0, y0 + YT) of plane z are one contiguous block: one bulk copy
   // into smt[ci & 1], landing on bar[ci & 1] (phase ci >> 1), when the maps are 16-byte
   // aligned; per-thread 8-byte asynchronous copies otherwise.

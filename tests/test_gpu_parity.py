@@ -306,6 +306,30 @@ def test_sense_normal_non_power_of_two(cuda, shape, ncoil):
     assert O.rel_l2(_np(out), ref) < TOL
 
 
+@pytest.mark.parametrize("counts", [(1,), (5,), (1, 7, 2), (3, 3, 16, 1)])
+def test_coils_shared_by_pass_a_ctas(cuda, counts):
+    """Small calls, whose x pass splits a system's coils between CTAs: uneven coil counts in one
+    launch, fewer coils than parts; each system against the oracle."""
+    from hastycompute_b200.toeplitz import System
+
+    shape = (8, 16, 32)
+    plan = ToeplitzPlan(shape, cuda)
+    rng = np.random.default_rng(61)
+    T = rng.standard_normal(tuple(2 * n for n in shape)) + 1.0
+    packed = plan.pack_diagonal(_c64(T, cuda))
+    sm = synth.coil_maps(16, shape, seed=62)
+    smt, systems, want = _c64(sm, cuda), [], []
+    for i, n in enumerate(counts):
+        coils = rng.permutation(16)[:n].tolist()
+        x = synth.gaussian_image(shape, seed=63 + i)
+        systems.append(System(_c64(x, cuda), smt, packed, out=torch.empty(shape, dtype=torch.complex64, device=cuda),
+                              coils=coils))
+        want.append(O.sense_normal_toeplitz(x, sm, T, coils))
+    plan.sense_normal_systems(systems)
+    for q, ref in zip(systems, want):
+        assert O.rel_l2(_np(q.out), ref) < TOL
+
+
 @pytest.mark.parametrize("n0,n1", [(8, 8), (8, 128), (128, 8), (16, 64), (32, 16), (32, 32), (64, 16), (64, 64),
                                    (64, 128), (128, 64)])
 def test_one_cta_planes(cuda, n0, n1):
