@@ -23,9 +23,9 @@
 // of L rows x 16 columns (128-byte rows), staged by 16-byte asynchronous copies; the FFT's
 // exchange reuses the tile, so a CTA needs 128 L bytes + twiddles (34 KB at L = 256) and
 // several CTAs per SM overlap their copies with each other's arithmetic.  Measured at 128^3
-// modes x 16 transforms: 1040 us for the three passes with the coil combination (type 1, 5.9 TB/s
+// modes x 16 transforms: 1000 us for the three passes with the coil combination (type 1, 5.9 TB/s
 // in the two axis passes) against 3210 us of memset, in-place passes, mode pass and combination
-// on separate grids; type 2 1160 us against 3200 us.
+// on separate grids; type 2 1060 us against 3200 us.
 #pragma once
 
 #include "bulk.cuh"
@@ -149,6 +149,20 @@ struct NufftModeOp {
 // nact <= NB transforms exist; the others are zero and are not stored.  sgn = -1 conjugates
 // the modes.
 
+// Grid offset (cells) and y, z correction of the CTA's lines, once per CTA: 64-bit products and a division
+// per element cost more than the transform.
+__device__ __forceinline__ void mode_lines(const NufftGeom& g, int line0, int nl, const float* corr, long long* cell,
+                                           float* scale) {
+  if ((int)threadIdx.x < nl) {
+    const int line = min(line0 + (int)threadIdx.x, g.N[0] * g.N[1] - 1);
+    const int i0 = line / g.N[1], i1 = line - i0 * g.N[1];
+    const int k0 = i0 - g.N[0] / 2, k1 = i1 - g.N[1] / 2;
+    const int c0 = k0 < 0 ? k0 + g.n[0] : k0, c1 = k1 < 0 ? k1 + g.n[1] : k1;
+    cell[threadIdx.x] = ((long long)c0 * g.n[1] + c1) * g.n[2];
+    scale[threadIdx.x] = corr[i0] * corr[g.N[0] + i1];
+  }
+}
+
 // type 2: grid lines = FFT along x of the corrected modes, at the kept (z, y) rows
 template <int L>
 __global__ void __launch_bounds__(TilePassCfg<L>::THREADS)
@@ -162,41 +176,50 @@ nufft_modes_to_grid_kernel(NufftGeom g, const __grid_constant__ NufftModeOp op, 
   const int nb = 1 << lgnb, nl = C::XT >> lgnb;
   const int nlines = g.N[0] * g.N[1], line0 = blockIdx.x * nl;
   const float* corr2 = corr + g.N[0] + g.N[1];
+  __shared__ long long cell_s[C::XT];
+  __shared__ float scale_s[C::XT];
+  mode_lines(g, line0, nl, corr, cell_s, scale_s);
   for (int i = threadIdx.x; i < L; i += C::THREADS) tws[i] = tw[i];
-  for (int i = threadIdx.x; i < C::XT * N2; i += C::THREADS) {
-    const int i2 = i % N2, col = i / N2;
+  // all loads of a thread first (E / 2 columns' modes), then the tile
+  constexpr int LD = C::XT * N2 / C::THREADS;
+  static_assert(LD * C::THREADS == C::XT * N2, "whole rounds");
+  float2 v[LD], w[LD];
+#pragma unroll
+  for (int k = 0; k < LD; ++k) {
+    const int i = threadIdx.x + k * C::THREADS, i2 = i % N2, col = i / N2;
     const int line = line0 + (col >> lgnb), b = col & (nb - 1);
-    float2 v = make_float2(0.f, 0.f);
+    v[k] = w[k] = make_float2(0.f, 0.f);
     if (line < nlines && b < nact) {
-      const int i0 = line / g.N[1], i1 = line % g.N[1];
-      const float s = corr[i0] * corr[g.N[0] + i1] * corr2[i2];
       const long long m = (long long)line * N2 + i2;
-      v = cscale(op.f ? op.f[b * op.f_ld + m] : cmul(op.x[m], op.maps.s[b][m]), s);
-      v.y *= sgn;
+      v[k] = op.f ? op.f[b * op.f_ld + m] : op.x[m];
+      if (!op.f) w[k] = op.maps.s[b][m];
     }
-    tile[tile_at(i2 < N2 / 2 ? i2 + L - N2 / 2 : i2 - N2 / 2, col)] = v;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < LD; ++k) {
+    const int i = threadIdx.x + k * C::THREADS, i2 = i % N2, col = i / N2;
+    float2 u = cscale(op.f ? v[k] : cmul(v[k], w[k]), scale_s[col >> lgnb] * corr2[i2]);
+    u.y *= sgn;
+    tile[tile_at(i2 < N2 / 2 ? i2 + L - N2 / 2 : i2 - N2 / 2, col)] = u;
   }
   __syncthreads();
   int col, t;
   tile_team<C::S>(&col, &t);
   tile_fft<L, true>(tile, col, t, tws);
   __syncthreads();
-  auto row_base = [&](int line) {  // grid line of a mode line
-    const int k0 = line / g.N[1] - g.N[0] / 2, k1 = line % g.N[1] - g.N[1] / 2;
-    const int c0 = k0 < 0 ? k0 + g.n[0] : k0, c1 = k1 < 0 ? k1 + g.n[1] : k1;
-    return grid + (((long long)c0 * g.n[1] + c1) * L << lgnb);
-  };
+  auto row_base = [&](int lc) { return grid + (cell_s[lc] << lgnb); };  // grid line of the CTA's mode line
   if (lgnb == 0) {
     for (int i = threadIdx.x; i < C::XT * L; i += C::THREADS) {
       const int r = i % L, c = i / L;
-      if (line0 + c < nlines) row_base(line0 + c)[r] = tile[tile_at(r, c)];
+      if (line0 + c < nlines) row_base(c)[r] = tile[tile_at(r, c)];
     }
   } else {
     const int lgp = lgnb - 1;  // 16-byte pairs per cell
     for (int i = threadIdx.x; i < 8 * L; i += C::THREADS) {
       const int r = (i >> lgp) % L, lc = (i >> lgp) / L, p = i & ((1 << lgp) - 1);
       if (line0 + lc < nlines)
-        *reinterpret_cast<float4*>(row_base(line0 + lc) + (r << lgnb) + 2 * p) =
+        *reinterpret_cast<float4*>(row_base(lc) + (r << lgnb) + 2 * p) =
             *reinterpret_cast<const float4*>(&tile[tile_at(r, (lc << lgnb) + 2 * p)]);
     }
   }
@@ -215,22 +238,22 @@ nufft_grid_to_modes_kernel(NufftGeom g, const __grid_constant__ NufftModeOp op, 
   const int nb = 1 << lgnb, nl = C::XT >> lgnb;
   const int nlines = g.N[0] * g.N[1], line0 = blockIdx.x * nl;
   const float* corr2 = corr + g.N[0] + g.N[1];
-  auto row_base = [&](int line) {
-    const int k0 = line / g.N[1] - g.N[0] / 2, k1 = line % g.N[1] - g.N[1] / 2;
-    const int c0 = k0 < 0 ? k0 + g.n[0] : k0, c1 = k1 < 0 ? k1 + g.n[1] : k1;
-    return grid + (((long long)c0 * g.n[1] + c1) * L << lgnb);
-  };
+  __shared__ long long cell_s[C::XT];
+  __shared__ float scale_s[C::XT];
+  mode_lines(g, line0, nl, corr, cell_s, scale_s);
+  __syncthreads();
+  auto row_base = [&](int lc) { return grid + (cell_s[lc] << lgnb); };
   if (lgnb == 0) {
     for (int i = threadIdx.x; i < C::XT * L; i += C::THREADS) {
       const int r = i % L, c = i / L;
-      if (line0 + c < nlines) cp_async8(&tile[tile_at(r, c)], row_base(line0 + c) + r);
+      if (line0 + c < nlines) cp_async8(&tile[tile_at(r, c)], row_base(c) + r);
     }
   } else {
     const int lgp = lgnb - 1;
     for (int i = threadIdx.x; i < 8 * L; i += C::THREADS) {
       const int r = (i >> lgp) % L, lc = (i >> lgp) / L, p = i & ((1 << lgp) - 1);
       if (line0 + lc < nlines)
-        cp_async16(&tile[tile_at(r, (lc << lgnb) + 2 * p)], row_base(line0 + lc) + (r << lgnb) + 2 * p);
+        cp_async16(&tile[tile_at(r, (lc << lgnb) + 2 * p)], row_base(lc) + (r << lgnb) + 2 * p);
     }
   }
   cp_async_commit();
@@ -247,8 +270,7 @@ nufft_grid_to_modes_kernel(NufftGeom g, const __grid_constant__ NufftModeOp op, 
     const int lc = op.f ? c >> lgnb : c, line = line0 + lc;
     if (line >= nlines) continue;
     const int r = i2 < N2 / 2 ? i2 + L - N2 / 2 : i2 - N2 / 2;
-    const int i0 = line / g.N[1], i1 = line % g.N[1];
-    const float s = corr[i0] * corr[g.N[0] + i1] * corr2[i2];
+    const float s = scale_s[lc] * corr2[i2];
     const long long m = (long long)line * N2 + i2;
     if (op.f) {
       const int b = c & (nb - 1);
@@ -256,6 +278,7 @@ nufft_grid_to_modes_kernel(NufftGeom g, const __grid_constant__ NufftModeOp op, 
       float2 v = cscale(tile[tile_at(r, c)], s);
       v.y *= sgn;
       if (op.circulant != 0.f) {
+        const int i0 = line / g.N[1], i1 = line % g.N[1];
         const int j0 = (i0 + g.N[0] / 2) % g.N[0], j1 = (i1 + g.N[1] / 2) % g.N[1], j2 = (i2 + N2 / 2) % N2;
         op.f[((long long)j0 * g.N[1] + j1) * N2 + j2] = cscale(v, op.circulant);
       } else {
@@ -263,11 +286,17 @@ nufft_grid_to_modes_kernel(NufftGeom g, const __grid_constant__ NufftModeOp op, 
       }
     } else {
       float2 acc = op.accumulate ? op.out[m] : make_float2(0.f, 0.f);
-      for (int b = 0; b < nact; ++b) {
-        float2 v = cscale(tile[tile_at(r, (lc << lgnb) + b)], s);
-        v.y *= sgn;
-        acc = cadd(acc, cmulc(v, op.maps.s[b][m]));
-      }
+      float2 w[kNufftGroup];
+#pragma unroll
+      for (int b = 0; b < kNufftGroup; ++b)
+        if (b < nact) w[b] = op.maps.s[b][m];
+#pragma unroll
+      for (int b = 0; b < kNufftGroup; ++b)
+        if (b < nact) {
+          float2 v = cscale(tile[tile_at(r, (lc << lgnb) + b)], s);
+          v.y *= sgn;
+          acc = cadd(acc, cmulc(v, w[b]));
+        }
       op.out[m] = acc;
     }
   }
