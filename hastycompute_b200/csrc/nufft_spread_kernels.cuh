@@ -14,11 +14,11 @@
 // Bound: issue (56 % of the slots in ncu, 5.6 M visits of 32 FP32x2 FMAs + about 50 other
 // instructions) with 20 warps per SM.  The reduction form it replaces issued W^3 vector
 // reductions per sample and transform.  Measured at W = 7, 512 k radial samples on a 256^3 grid:
-// 8 transforms 782 us + 24 us (gathering the values) + 9 us (zeroing) against 2145 + 172 us,
+// 8 transforms 751 us + 24 us (gathering the values) + 9 us (zeroing) against 2145 + 172 us,
 // 4: 484 us, 1: 307 us against 916 us.  Choices, 8 transforms: one warp per CTA (two: 1192 us, a
 // CTA waits for its slower warp; four: 1140 us), 96 registers (128: 825 us), long pieces first
 // (in tile order: 821 us), values gathered into sorted order first (read from the caller's rows:
-// 1018 us).  Tile: 4 x 4 x 8 gives each lane four cells x 8 transforms (64 accumulators); a
+// 1018 us).  Tile: 4 x 4 x 8 gives each lane 64 accumulators for 8 transforms; a
 // sample visits 10.9 tiles at W = 7, where a quarter of the weights are inside its support.
 #pragma once
 
@@ -27,9 +27,20 @@
 
 namespace hb {
 
-// Cells of a tile: lane l holds (y = l / 8, x = l % 8) and kTileR rows of the slowest axis; in
-// 2-D the slowest axis is y, and lane row l / 8 holds y = 4 (l / 8) + r.
-constexpr int kTileR = 4;
+// Cells and transforms of a lane: x = l % 8, then the y group and the half of the transforms.
+// A visit reads the lane's weights and transform values from shared memory, which delivers 4 bytes
+// per lane and cycle whether or not the lanes share an address.  In 3-D with eight transforms
+// each half of the warp therefore takes four of them on two y (cells z = 0..3 x 2 y): 15 cycles of
+// reads a visit instead of 22 for all of them on one y (751 us against 775 us for 512 k samples on a
+// 256^3 grid, 525 against 546 for 128^3).  Elsewhere a lane holds one y (in 2-D four) and all
+// transforms: the added products undo it with four transforms (485 us against 537) and in 2-D
+// (28.2 us against 30.4 for 128 x 128 modes x 8).
+template <int DIM, int NB>
+struct SpreadLane {
+  static constexpr int HALVES = DIM == 3 && NB == 8 ? 2 : 1, TL = NB / HALVES;  // transforms of a lane
+  static constexpr int YC = HALVES, R = 4 * YC;                                // y in 3-D, cells
+  static constexpr int YG = 4 / HALVES;                                        // y groups
+};
 template <int DIM>
 struct SpreadTile {
   static constexpr int T0 = DIM == 3 ? 4 : 1, T1 = DIM == 3 ? 4 : 16, T2 = 8;
@@ -189,11 +200,14 @@ nufft_spread_tiles_kernel(NufftGeom g, const float4* pts, const int* start, cons
   const SpreadItem it = items[blockIdx.x];
   const TileRuns<DIM> tr(g, it.origin);
 
-  float2 acc[kTileR][NB];
+  using Q = SpreadLane<DIM, NB>;
+  constexpr int R = Q::R, TL = Q::TL, YC = Q::YC;
+  const int yg = (lane / 8) % Q::YG, tb = TL * (lane / (8 * Q::YG));  // y group, first transform
+  float2 acc[R][TL];
 #pragma unroll
-  for (int r = 0; r < kTileR; ++r)
+  for (int r = 0; r < R; ++r)
 #pragma unroll
-    for (int b = 0; b < NB; ++b) acc[r][b] = make_float2(0.f, 0.f);
+    for (int b = 0; b < TL; ++b) acc[r][b] = make_float2(0.f, 0.f);
   const float hw = 0.5f * (float)g.w, inv_hw = 1.f / hw;
 
   // kernel values: lane l evaluates cell coordinate l % 16 of every other sample: in 3-D z 0-3, y 0-3,
@@ -296,48 +310,69 @@ nufft_spread_tiles_kernel(NufftGeom g, const float4* pts, const int* start, cons
 #pragma unroll 2
     for (int e = 0; e < n; ++e) {
       const float* w = w_s[e];
-      const float4 wr = *reinterpret_cast<const float4*>(DIM == 3 ? w : w + kTileR * (lane / 8));
-      float wyx = w[WX + lane % 8];
-      if (DIM == 3) wyx *= w[T::T0 + lane / 8];
-      float2 cv2[NB];
-      if constexpr (NB >= 2) {
+      const float wx = w[WX + lane % 8];
+      float wr[R];  // weights of the lane's cells: z major in 3-D
+      if constexpr (DIM == 3) {
+        const float4 wz = *reinterpret_cast<const float4*>(w);
+        float wyx[YC];
+        if constexpr (YC == 2) {
+          const float2 wy = *reinterpret_cast<const float2*>(w + T::T0 + 2 * yg);
+          wyx[0] = wy.x * wx;
+          wyx[1] = wy.y * wx;
+        } else {
+          wyx[0] = w[T::T0 + yg] * wx;
+        }
 #pragma unroll
-        for (int b = 0; b < NB; b += 2) {
-          const float4 q = *reinterpret_cast<const float4*>(&c_s[e][b]);
+        for (int y = 0; y < YC; ++y) {
+          wr[y] = wz.x * wyx[y];
+          wr[YC + y] = wz.y * wyx[y];
+          wr[2 * YC + y] = wz.z * wyx[y];
+          wr[3 * YC + y] = wz.w * wyx[y];
+        }
+      } else {
+        const float4 wy = *reinterpret_cast<const float4*>(w + R * yg);
+        wr[0] = wy.x * wx;
+        wr[1] = wy.y * wx;
+        wr[2] = wy.z * wx;
+        wr[3] = wy.w * wx;
+      }
+      float2 cv2[TL];
+      if constexpr (TL >= 2) {
+#pragma unroll
+        for (int b = 0; b < TL; b += 2) {
+          const float4 q = *reinterpret_cast<const float4*>(&c_s[e][tb + b]);
           cv2[b] = make_float2(q.x, q.y);
           cv2[b + 1] = make_float2(q.z, q.w);
         }
       } else {
         cv2[0] = c_s[e][0];
       }
-      const float wz[kTileR] = {wr.x * wyx, wr.y * wyx, wr.z * wyx, wr.w * wyx};
 #pragma unroll
-      for (int r = 0; r < kTileR; ++r) {
-        const float2 wv = make_float2(wz[r], wz[r]);
+      for (int r = 0; r < R; ++r) {
+        const float2 wv = make_float2(wr[r], wr[r]);
 #pragma unroll
-        for (int b = 0; b < NB; ++b) acc[r][b] = __ffma2_rn(wv, cv2[b], acc[r][b]);
+        for (int b = 0; b < TL; ++b) acc[r][b] = __ffma2_rn(wv, cv2[b], acc[r][b]);
       }
     }
     __syncwarp();
   }
 
-  // cells (z = r, y = lane / 8, x = lane % 8) in 3-D, (y = 4 (lane / 8) + r, x) in 2-D
 #pragma unroll
-  for (int r = 0; r < kTileR; ++r) {
-    const int z = tr.o[0] + (DIM == 3 ? r : 0), y = tr.o[1] + (DIM == 3 ? lane / 8 : kTileR * (lane / 8) + r);
+  for (int r = 0; r < R; ++r) {
+    const int z = tr.o[0] + (DIM == 3 ? r / YC : 0), y = tr.o[1] + (DIM == 3 ? YC * yg + r % YC : R * yg + r);
     if (DIM == 2 && y >= g.n[1]) continue;
-    float2* p = grid + (((long long)z * g.n[1] + y) * g.n[2] + tr.o[2] + lane % 8) * NB;
+    float2* p = grid + (((long long)z * g.n[1] + y) * g.n[2] + tr.o[2] + lane % 8) * NB + tb;
     if (it.split) {
-      if constexpr (NB == 1) red_add(p, acc[r][0]);
+      if constexpr (TL == 1) red_add(p, acc[r][0]);
       else
 #pragma unroll
-        for (int b = 0; b < NB; b += 2) red_add4(p + b, acc[r][b], acc[r][b + 1]);
+        for (int b = 0; b < TL; b += 2) red_add4(p + b, acc[r][b], acc[r][b + 1]);
     } else {
-      if constexpr (NB == 1) p[0] = acc[r][0];
-      else if constexpr (NB == 2) *reinterpret_cast<float4*>(p) = make_float4(acc[r][0].x, acc[r][0].y, acc[r][1].x, acc[r][1].y);
+      if constexpr (TL == 1) p[0] = acc[r][0];
+      else if constexpr (TL == 2) *reinterpret_cast<float4*>(p) = make_float4(acc[r][0].x, acc[r][0].y, acc[r][1].x, acc[r][1].y);
       else
 #pragma unroll
-        for (int b = 0; b < NB; b += 4) store_cell8(p + b, &acc[r][b]);
+        for (int b = 0; b < TL; b += 4) store_cell8(p + b, &acc[r][b]);
     }
   }
 }
