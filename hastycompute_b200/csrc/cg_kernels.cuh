@@ -76,6 +76,7 @@ __device__ void block_write_partial(double s, double* out, double* red) {
 
 // r = b - Ap; p = r; partial Re<r, r>
 __global__ void __launch_bounds__(256) cg_init_kernel(CgState s) {
+  chained_kernel_begin();
   __shared__ double red[32];
   const int sys = blockIdx.y;
   const long long base = (long long)sys * s.nv;
@@ -92,6 +93,7 @@ __global__ void __launch_bounds__(256) cg_init_kernel(CgState s) {
 
 // rz[0] = sum of partials; status/active from tol.   grid: nsys blocks
 __global__ void __launch_bounds__(256) cg_init_finish_kernel(CgState s, int nrr) {
+  chained_kernel_begin();
   __shared__ double red[32];
   const int sys = blockIdx.x;
   const double rz = block_sum_fixed(s.rr_part + (long long)sys * nrr, nrr, red);
@@ -106,6 +108,7 @@ __global__ void __launch_bounds__(256) cg_init_finish_kernel(CgState s, int nrr)
 }
 
 __global__ void __launch_bounds__(256) cg_step_xr_kernel(CgState s) {
+  chained_kernel_begin();
   __shared__ double red[32];
   const int sys = blockIdx.y;
   if (!s.active[sys]) return;
@@ -140,6 +143,7 @@ __global__ void __launch_bounds__(256) cg_step_xr_kernel(CgState s) {
 }
 
 __global__ void __launch_bounds__(256) cg_step_p_kernel(CgState s) {
+  chained_kernel_begin();
   __shared__ double red[32];
   const int sys = blockIdx.y;
   if (!s.active[sys]) return;
@@ -185,6 +189,7 @@ __global__ void __launch_bounds__(256) cg_rz_kernel(CgState s, int init) {
 // Frequency-domain step of z = P r: z[sys] *= pdiag[sys] / nv (identity for a system
 // without a preconditioner; 1/nv is the inverse FFT's normalisation).
 __global__ void __launch_bounds__(256) cg_precond_scale_kernel(CgState s) {
+  chained_kernel_begin();
   const int sys = blockIdx.y;
   const float* d = s.sys_pdiag[sys];
   const float inv = 1.f / (float)s.nv;
@@ -194,7 +199,10 @@ __global__ void __launch_bounds__(256) cg_precond_scale_kernel(CgState s) {
 }
 
 // Ends an iteration: every kernel of the next one reads the advanced counter.
-__global__ void cg_advance_kernel(int* iter) { *iter += 1; }
+__global__ void cg_advance_kernel(int* iter) {
+  chained_kernel_begin();
+  *iter += 1;
+}
 
 // ------------------------------------------------------------ running batch (engine) ----
 // A running batch holds systems at different points of their solves: a member that joined

@@ -8,6 +8,12 @@
 
 namespace hb {
 
+// First statement of the kernels that launch_chained launches: waits until the kernels before it on
+// the stream are complete and their writes visible.  Without effect in other launches.
+__device__ __forceinline__ void chained_kernel_begin() {
+  cudaGridDependencySynchronize();
+}
+
 // Complex add/subtract as one packed FP32x2 instruction on sm_100 (same IEEE results
 // as two scalar adds).  Packed multiplies are not used: they need the operands
 // broadcast or swapped within the pair, which costs more than the scalar FMAs.

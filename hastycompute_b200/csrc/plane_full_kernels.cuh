@@ -34,6 +34,7 @@ struct PlaneFullCfg {
 
 template <int N0, int N1, int THREADS_>
 __global__ void __launch_bounds__(THREADS_) plane_full_kernel(PassArgs a) {
+  chained_kernel_begin();
   using C = PlaneFullCfg<N0, N1, THREADS_>;
   constexpr int M0 = C::M0, M1 = C::M1, LDP = C::LDP;
   constexpr int SR = C::SR, ER = C::ER, SZ = C::SZ, EZ = C::EZ, NTR = C::NTR, NTZ = C::NTZ;

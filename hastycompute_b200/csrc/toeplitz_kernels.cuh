@@ -4,8 +4,12 @@
 //
 // Pass A  expand_fwd_x : per (slot, z, y-tile): S_c * x, zero-pad along x, M2-point FFT,
 //                        written transposed to the spill  spill[slot][z][kx][y].
-// Pass B  plane_yz     : per (slot, kx) a 2-CTA cluster owns one N0 x N1 (z, y) plane of
-//                        the spill.  CTA h takes the ky-parity-h half of the 2x y-grid
+// Pass B  per (slot, kx), one N0 x N1 (z, y) plane of the spill, in place: forward along y and z
+//                        on the doubled grid, x T, inverse, crop.  plane_mod below for 128 x 128,
+//                        plane_full_kernels.cuh (one CTA per plane) for the other powers of two,
+//                        plane_odd_kernels.cuh for 96 x 96 and 160 x 160.
+//         plane_yz     : alternative for 128 x 128 that the autotuner may choose.  CTA h of a
+//                        2-CTA cluster takes the ky-parity-h half of the 2x y-grid
 //                        (ky = 2*ky' + h): pre-twiddle, N1-point FFT along y, then per ky'
 //                        column an M0-point FFT along z (upper half zero), x T, inverse
 //                        M0-point FFT keeping z < N0, inverse N1-point FFT along y and
@@ -228,6 +232,7 @@ struct PassArgs {
 template <int N2, int YT>
 __global__ void __launch_bounds__(XPassCfg<N2, YT>::THREADS)
 expand_fwd_x_kernel(PassArgs a) {
+  chained_kernel_begin();
   using C = XPassCfg<N2, YT>;
   constexpr int M2 = C::M2, E = C::E, S = C::S, LPT = C::LPT;
   extern __shared__ __align__(128) float2 smem[];
@@ -846,6 +851,7 @@ plane_mod_kernel(PassArgs a) {
 template <int N2, int YT>
 __global__ void __launch_bounds__(XPassCfg<N2, YT>::THREADS, XPassCfg<N2, YT>::C_IN_TILE ? 3 : 1)
 inv_x_combine_kernel(PassArgs a) {
+  chained_kernel_begin();
   using C = XPassCfg<N2, YT>;
   constexpr int M2 = C::M2, E = C::E, S = C::S, LPT = C::LPT;
   extern __shared__ __align__(128) float2 smem[];

@@ -10,7 +10,10 @@
  * asynchronous on `stream` unless documented otherwise.
  *
  * Calls that take systems (hb_toeplitz_apply, hb_sense_normal_apply*, hb_cg_run*)
- * synchronise `stream` once per group of systems to upload its descriptor tables.
+ * write their descriptor tables (76 bytes per system and 8 per coil) on `stream` once per
+ * group of systems: up to 3840 bytes travel with a launch, larger ones are copied and
+ * `stream` is synchronised.  So are all of them while `stream` is being captured, which
+ * refuses the synchronisation: those calls fail under capture.
  *
  * Every function returns HB_OK (0) or an error code; hb_last_error() gives the
  * message of the last failure on the calling thread.  No function aborts the process
@@ -249,7 +252,9 @@ int hb_cg_run(const hb_plan* plan, int64_t nsys, void* x, const void* b, const v
 size_t hb_autotune_workspace_bytes(const hb_plan* plan, int64_t nslots);
 /* Name of the plane-pass schedule the plan's next call launches ("mod4t256": the ky-mod-4
  * split plane_mod_kernel, 4-CTA clusters of 256 threads; "q2t128": the parity split
- * plane_yz_kernel, 2x2-CTA clusters of 128 threads; ...), after HB_PLANE_VARIANT and
+ * plane_yz_kernel, 2x2-CTA clusters of 128 threads; "odd3t128" / "odd5t256": the split by 3 / 5
+ * residues of 96^2 / 160^2 planes; "full256": one CTA per plane, also "full" where there is
+ * one such schedule; ...), after HB_PLANE_VARIANT and
  * hb_plan_autotune.  A static string owned by the library.  No counterpart in the
  * reference (cuFFT chooses its own plans, nufft.cpp:1184-1186). */
 const char* hb_plan_plane_schedule(const hb_plan* plan);
@@ -279,7 +284,7 @@ int hb_plan_autotune(hb_plan* plan, int64_t nslots, void* workspace, size_t work
  *    cudaMemcpyAsync on `stream` and then waits for `stream` with
  *    cudaStreamSynchronize, so the call returns only after the work queued on `stream`
  *    before it has finished; the three passes themselves are then queued on `stream`
- *    without waiting.  hb_toeplitz_apply does the same through its table upload.
+ *    without waiting.
  *  - All calls share the arrays, which keep the last call's contents (nothing in them
  *    needs to start at zero).  Calls that overlap on the GPU (several streams or
  *    threads) race on the shared scratch: serialise them.
@@ -302,14 +307,16 @@ int hb_toeplitz_apply_noalloc(int64_t nz, int64_t ny, int64_t nx, const void* in
  * Method: exponential-of-semicircle gridding kernel with upsampling 2 (the published
  * method of finufft); kernel width w = ceil(log10(1/tol)) + 1 fine-grid cells.
  * 2*N_a must be one of 8, 16, 32, 64, 128, 256, 512, 96, 160, 192, 320 and >= 2w.
- * Type 1 accumulates with atomics, so its last bits vary from run to run.
+ * The order of a bin's samples and the sums of crowded tiles come from atomics, so the last bits
+ * of type 1 vary from plan to plan and from run to run.
  * Lower dimensions (the reference's 1-D and 2-D plans, nufft.ixx:72-160): nz = 1 makes a
  * 2-D plan over (ny, nx) and nz = ny = 1 a 1-D plan over nx; coords is then [2][nsamples]
  * or [1][nsamples] (rows pairing with the transformed axes in order).
  *
- * hb_nufft_create copies coords, sorts the samples by fine-grid bin and allocates the
- * fine grids of `maxbatch` (1..32) transforms plus as many mode and k-space arrays; it synchronises
- * `stream`.  Transforms run in batches of maxbatch.  c is [ntransf][nsamples], f is
+ * hb_nufft_create sorts the samples by fine-grid bin (16 bytes per sample; coords is not kept) and
+ * allocates one fine grid of g interleaved transforms, the sorted values of g transforms and the list
+ * of spreading work, g = `maxbatch` (1..32) rounded up to 1, 2, 4 or 8 at most; it synchronises
+ * `stream`.  Transforms run g at a time.  c is [ntransf][nsamples], f is
  * [ntransf][nz][ny][nx]. */
 typedef struct hb_nufft hb_nufft;
 int hb_nufft_create(hb_nufft** plan, int64_t nz, int64_t ny, int64_t nx, const float* coords, int64_t nsamples,
@@ -331,8 +338,7 @@ int hb_sense_adjoint_nufft(const hb_nufft* plan, const void* kdata, const void* 
  * manipulators, lib/mri/batch_sense.cpp:452-486; the coil loop of sense.ixx:426-497):
  *   out (+)= sum_b conj(S[c_b]) * type1( w * (type2(S[c_b] * x) - kdata[c_b]) ),  c_b = coils[b]
  * kdata [C][nsamples] indexed by coil number (nullable), weights [nsamples] float32
- * (nullable); with both NULL it is the explicit normal operator A^H A.  The plan's mode
- * and k-space arrays are its temporaries. */
+ * (nullable); with both NULL it is the explicit normal operator A^H A. */
 int hb_sense_normal_nufft(const hb_nufft* plan, const void* x, const void* smaps, const int64_t* coils, int64_t ncoil,
                           const void* kdata, const float* weights, void* out, int accumulate, void* stream);
 
@@ -344,8 +350,8 @@ int hb_sense_normal_nufft(const hb_nufft* plan, const void* x, const void* smaps
  * scaled by 1/prod(2N), then FFT'd.  Same outputs as hb_diag_build (packed and/or the
  * complex T [2nz][2ny][2nx]) to the NUFFT tolerance instead of FP64-exact, in
  * milliseconds instead of seconds.  Needs 4*N per axis among the NUFFT's fine-grid lengths
- * (image axes of 8..128; HB_ERR_UNSUPPORTED for 96 and 160, use hb_diag_build there).  Allocates its NUFFT plan (a (4nz)(4ny)(4nx)
- * complex64 fine grid) for the duration of the call and synchronises `stream`. */
+ * (image axes of 8..128; HB_ERR_UNSUPPORTED for 96 and 160, use hb_diag_build there).  Allocates hb_diag_build_nufft_workspace_bytes (a (4nz)(4ny)(4nx)
+ * complex64 fine grid and the sorted samples) for the duration of the call and synchronises `stream`. */
 int hb_diag_build_nufft(const hb_plan* plan, const float* coords, int64_t nsamples, double tol, const float* weights,
                         float* packed, void* T_complex, void* stream);
 /* The same with the caller's workspace (256-byte aligned, hb_diag_build_nufft_workspace_bytes; 0 for

@@ -330,6 +330,30 @@ def test_coils_shared_by_pass_a_ctas(cuda, counts):
         assert O.rel_l2(_np(q.out), ref) < TOL
 
 
+@pytest.mark.parametrize("shape", [(8, 8, 8), (64, 32, 16), (96, 96, 16), (128, 128, 8)])
+def test_calls_queued_without_waiting(cuda, shape):
+    """Calls queued one behind the other, each reading the last one's output and reusing its
+    workspace: bitwise the results of the same calls with a wait after each."""
+    plan = ToeplitzPlan(shape, cuda)
+    rng = np.random.default_rng(71)
+    packed = plan.pack_diagonal(_c64(rng.standard_normal(tuple(2 * n for n in shape)) + 1.0, cuda))
+    sm = _c64(synth.coil_maps(3, shape, seed=72), cuda)
+    x = _c64(synth.gaussian_image(shape, seed=73), cuda)[None]
+
+    def run(wait):
+        outs = [x]
+        for _ in range(12):
+            outs.append(torch.empty_like(x))
+            plan.sense_normal(outs[-2], outs[-1], sm, packed)
+            if wait:
+                torch.cuda.synchronize()
+        return torch.stack(outs)
+
+    queued, waited = run(False), run(True)
+    assert torch.isfinite(torch.view_as_real(waited)).all()
+    assert torch.equal(torch.view_as_real(queued), torch.view_as_real(waited))
+
+
 @pytest.mark.parametrize("n0,n1", [(8, 8), (8, 128), (128, 8), (16, 64), (32, 16), (32, 32), (64, 16), (64, 64),
                                    (64, 128), (128, 64)])
 def test_one_cta_planes(cuda, n0, n1):
