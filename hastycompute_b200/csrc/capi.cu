@@ -159,27 +159,6 @@ std::vector<uint16_t> tc_dft_table(int N2) {
 // depend on who makes them).  Measured: 64^3 x 8 coils 15.7 -> 12.5 us, x 16 coils 28.8 -> 22.3 us, 32^3 x 8
 // 9.5 -> 4.3 us; eight or sixteen per SM 13.0 and 13.5 us at 64^3 x 8.
 constexpr long long kXPassCtas = 148 * 4;
-// Launches a kernel that begins with chained_kernel_begin as a programmatic dependent of the kernel
-// before it: it is set up while that one runs and starts as its last CTA leaves.  For the passes of small
-// calls and the CG's vector kernels, where the gaps between launches are a tenth of the time.  Measured
-// against plain launches: 64^3 apply 28.5 -> 26.1 us, 64^3 x 8 coils 86.9 -> 82.0 us, five CG iterations
-// of it 692 -> 620 us; 128^3 x 16 coils x 10 systems the same.  With the next kernel released at the start
-// (an explicit trigger) its CTAs take room from the last ones of the running kernel: 87.4 and 669 us.
-template <class... P, class... A>
-cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, const A&... args) {
-  cudaLaunchAttribute attr = {};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
-}
-
 template <int N2, int YT>
 cudaError_t launch_a(const PassArgs& a, int nsys, cudaStream_t st) {
   using C = XPassCfg<N2, YT>;

@@ -76,14 +76,15 @@ const GaussLegendre& gauss_legendre() {
 }
 
 // Transforms of one group: nact <= NB = 1 << lgnb interleaved grids.  Sizes that are not a
-// power of two are padded, except 5, which runs as 4 + 1 (padding it to 8 moves 1.6 times the
-// bytes); at 3, 6 and 7 the padding costs at most a third and saves a second set of launches.
+// power of two are padded, except 5 in 3-D, which runs as 4 + 1 (padding it to 8 moves 1.6 times the
+// bytes); at 3, 6 and 7, and in the small grids of 2-D and 1-D, a second set of launches costs
+// more than the padding.
 struct Group {
   int nact, lgnb;
 };
 Group next_group(const hb_nufft* p, int64_t left) {
   int n = (int)(left < p->group ? left : p->group);
-  if (n == 5) n = 4;
+  if (n == 5 && p->g.dim == 3) n = 4;
   return {n, n > 4 ? 3 : n > 2 ? 2 : n - 1};
 }
 
@@ -103,45 +104,42 @@ cudaError_t interp_w(const hb_nufft* p, const InterpDest& dst, Group q, float cs
   LaunchScope ls(HB_KERNEL_NUFFT, st);
   if (p->g.dim < 3) {
     const unsigned grid = (unsigned)(((p->g.K << q.lgnb) + 255) / 256);
-    auto go = [&](auto kernel) { kernel<<<grid, 256, 0, st>>>(p->g, p->pts, p->grid, q.lgnb, q.nact, csgn, dst); };
-    if (p->g.dim == 2) go(nufft_interp_points_kernel<W, 2>);
-    else go(nufft_interp_points_kernel<W, 1>);
-    return cudaGetLastError();
+    return launch_chained(p->g.dim == 2 ? nufft_interp_points_kernel<W, 2> : nufft_interp_points_kernel<W, 1>, grid, 256, 0, st,
+                          p->g, p->pts, p->grid, q.lgnb, q.nact, csgn, dst);
   }
   auto go = [&](auto kernel, int per_cta) {
     const unsigned grid = (unsigned)((p->g.K + per_cta - 1) / per_cta);
-    kernel<<<grid, 32 * kInterpWarps, 0, st>>>(p->g, p->pts, p->grid, q.nact, csgn, dst);
+    return launch_chained(kernel, grid, 32 * kInterpWarps, 0, st, p->g, p->pts, p->grid, q.nact, csgn, dst);
   };
-  if (q.lgnb == 3) go(nufft_interp_rows_kernel<W, 8>, InterpCfg<W, 8>::PER_CTA);
-  else if (q.lgnb == 2) go(nufft_interp_rows_kernel<W, 4>, InterpCfg<W, 4>::PER_CTA);
-  else if (q.lgnb == 1) go(nufft_interp_rows_kernel<W, 2>, InterpCfg<W, 2>::PER_CTA);
-  else go(nufft_interp_rows_kernel<W, 1>, InterpCfg<W, 1>::PER_CTA);
-  return cudaGetLastError();
+  if (q.lgnb == 3) return go(nufft_interp_rows_kernel<W, 8>, InterpCfg<W, 8>::PER_CTA);
+  if (q.lgnb == 2) return go(nufft_interp_rows_kernel<W, 4>, InterpCfg<W, 4>::PER_CTA);
+  if (q.lgnb == 1) return go(nufft_interp_rows_kernel<W, 2>, InterpCfg<W, 2>::PER_CTA);
+  return go(nufft_interp_rows_kernel<W, 1>, InterpCfg<W, 1>::PER_CTA);
 }
 
 // p->vals = the values to spread
 cudaError_t gather_values(const hb_nufft* p, const SpreadSource& src, Group q, float csgn, cudaStream_t st) {
   const unsigned grid = (unsigned)(((p->g.K << q.lgnb) + 255) / 256);
   LaunchScope ls(HB_KERNEL_NUFFT, st);
-  nufft_gather_values_kernel<<<grid, 256, 0, st>>>(p->g.K, p->pts, src, q.lgnb, q.nact, csgn, p->vals);
-  return cudaGetLastError();
+  return launch_chained(nufft_gather_values_kernel, grid, 256, 0, st, p->g.K, p->pts, src, q.lgnb, q.nact, csgn, p->vals);
 }
 
 template <int DIM>
 cudaError_t spread_tiles(const hb_nufft* p, Group q, cudaStream_t st) {
   if (p->nsplit > 0) {
     LaunchScope ls(HB_KERNEL_NUFFT, st);
-    nufft_zero_tiles_kernel<DIM><<<p->nsplit, 128, 0, st>>>(p->g, p->split_tiles, q.lgnb, p->grid);
+    const cudaError_t e =
+        launch_chained(nufft_zero_tiles_kernel<DIM>, (unsigned)p->nsplit, 128, 0, st, p->g, p->split_tiles, q.lgnb, p->grid);
+    if (e != cudaSuccess) return e;
   }
   LaunchScope ls(HB_KERNEL_NUFFT, st);
   auto go = [&](auto kernel) {
-    kernel<<<p->nitems, 32, 0, st>>>(p->g, p->pts, p->start, p->items, p->vals, p->grid);
+    return launch_chained(kernel, (unsigned)p->nitems, 32, 0, st, p->g, p->pts, p->start, p->items, p->vals, p->grid);
   };
-  if (q.lgnb == 3) go(nufft_spread_tiles_kernel<DIM, 8>);
-  else if (q.lgnb == 2) go(nufft_spread_tiles_kernel<DIM, 4>);
-  else if (q.lgnb == 1) go(nufft_spread_tiles_kernel<DIM, 2>);
-  else go(nufft_spread_tiles_kernel<DIM, 1>);
-  return cudaGetLastError();
+  if (q.lgnb == 3) return go(nufft_spread_tiles_kernel<DIM, 8>);
+  if (q.lgnb == 2) return go(nufft_spread_tiles_kernel<DIM, 4>);
+  if (q.lgnb == 1) return go(nufft_spread_tiles_kernel<DIM, 2>);
+  return go(nufft_spread_tiles_kernel<DIM, 1>);
 }
 
 #define HB_W_DISPATCH(FN, ...)                                                                      \
@@ -178,14 +176,13 @@ cudaError_t axis_pass_l(const hb_nufft* p, int axis, int lgnb, cudaStream_t st) 
   LaunchScope ls(HB_KERNEL_NUFFT, st);
   if (axis == 0) {  // z: every (y, x) column
     const long long ncols = (long long)g.n[1] * g.n[2] << lgnb;
-    nufft_axis_pass_kernel<L, PAD><<<dim3((unsigned)((ncols + 15) / 16), 1), C::THREADS, smem, st>>>(
-        p->grid, ncols, (int)ncols, 1, 1, 0, p->tw);
+    return launch_chained(nufft_axis_pass_kernel<L, PAD>, dim3((unsigned)((ncols + 15) / 16), 1), C::THREADS, smem, st, p->grid,
+                          ncols, (int)ncols, 1, 1, 0, p->tw);
   } else {  // y: the kept z planes
     const int ncols = g.n[2] << lgnb;
-    nufft_axis_pass_kernel<L, PAD><<<dim3((ncols + 15) / 16, g.N[0]), C::THREADS, smem, st>>>(
-        p->grid, ncols, ncols, g.N[0], g.n[0], (long long)ncols * L, p->tw + g.n[0]);
+    return launch_chained(nufft_axis_pass_kernel<L, PAD>, dim3((ncols + 15) / 16, g.N[0]), C::THREADS, smem, st, p->grid, ncols,
+                          ncols, g.N[0], g.n[0], (long long)ncols * L, p->tw + g.n[0]);
   }
-  return cudaGetLastError();
 }
 // to_grid: modes -> grid (type 2), else grid -> modes (type 1)
 template <int L>
@@ -200,13 +197,14 @@ cudaError_t mode_pass_l(const hb_nufft* p, const NufftModeOp& op, Group q, float
   if (to_grid) {
     if ((e = hb::fftl::allow_smem<nufft_modes_to_grid_kernel<L>>(smem)) != cudaSuccess) return e;
     LaunchScope ls(HB_KERNEL_NUFFT, st);
-    nufft_modes_to_grid_kernel<L><<<grid, C::THREADS, smem, st>>>(g, op, q.lgnb, q.nact, sgn, p->corr, tw, p->grid);
+    return launch_chained(nufft_modes_to_grid_kernel<L>, grid, C::THREADS, smem, st, g, op, q.lgnb, q.nact, sgn, p->corr, tw,
+                          p->grid);
   } else {
     if ((e = hb::fftl::allow_smem<nufft_grid_to_modes_kernel<L>>(smem)) != cudaSuccess) return e;
     LaunchScope ls(HB_KERNEL_NUFFT, st);
-    nufft_grid_to_modes_kernel<L><<<grid, C::THREADS, smem, st>>>(g, op, q.lgnb, q.nact, sgn, p->corr, tw, p->grid);
+    return launch_chained(nufft_grid_to_modes_kernel<L>, grid, C::THREADS, smem, st, g, op, q.lgnb, q.nact, sgn, p->corr, tw,
+                          p->grid);
   }
-  return cudaGetLastError();
 }
 
 #define HB_L_DISPATCH(n, CALL)                                                        \

@@ -278,6 +278,7 @@ template <int W, int DIM>
 __global__ void __launch_bounds__(256) nufft_interp_points_kernel(NufftGeom g, const float4* pts, const float2* grid,
                                                                   int lgnb, int nact, float csgn,
                                                                   const __grid_constant__ InterpDest dst) {
+  chained_kernel_begin();
   constexpr int W1 = DIM == 2 ? W : 1;
   const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int bt = (int)(id & ((1 << lgnb) - 1));
@@ -351,6 +352,7 @@ template <int W, int NB>
 __global__ void __launch_bounds__(32 * kInterpWarps, W <= 5 && NB > 1 ? 4 : 3)
 nufft_interp_rows_kernel(NufftGeom g, const float4* pts, const float2* grid, int nact, float csgn,
                          const __grid_constant__ InterpDest dst) {
+  chained_kernel_begin();
   using C = InterpCfg<W, NB>;
   constexpr int V = C::V, PL = C::PL, XL = C::XL, XS = C::XS, SL = C::SL;
   __shared__ float w_s[kInterpWarps][SL][3 * W];  // z, y, x weights of the warp's samples

@@ -103,6 +103,7 @@ template <int L, bool PAD>
 __global__ void __launch_bounds__(TilePassCfg<L>::THREADS)
 nufft_axis_pass_kernel(float2* grid, long long row_stride, int ncols, int outer_N, int outer_n, long long outer_stride,
                        const float2* tw) {
+  chained_kernel_begin();
   using C = TilePassCfg<L>;
   extern __shared__ __align__(128) float2 smem[];
   float2* tile = smem;
@@ -168,6 +169,7 @@ template <int L>
 __global__ void __launch_bounds__(TilePassCfg<L>::THREADS)
 nufft_modes_to_grid_kernel(NufftGeom g, const __grid_constant__ NufftModeOp op, int lgnb, int nact, float sgn, const float* corr,
                            const float2* tw, float2* grid) {
+  chained_kernel_begin();
   using C = TilePassCfg<L>;
   constexpr int N2 = L / 2;
   extern __shared__ __align__(128) float2 smem[];
@@ -230,6 +232,7 @@ template <int L>
 __global__ void __launch_bounds__(TilePassCfg<L>::THREADS)
 nufft_grid_to_modes_kernel(NufftGeom g, const __grid_constant__ NufftModeOp op, int lgnb, int nact, float sgn, const float* corr,
                            const float2* tw, const float2* grid) {
+  chained_kernel_begin();
   using C = TilePassCfg<L>;
   constexpr int N2 = L / 2;
   extern __shared__ __align__(128) float2 smem[];

@@ -160,6 +160,7 @@ nufft_tile_items_kernel(NufftGeom g, int ntiles, int cap, const int* candidates,
 __global__ void __launch_bounds__(256) nufft_gather_values_kernel(long long K, const float4* pts,
                                                                   const __grid_constant__ SpreadSource src, int lgnb,
                                                                   int nact, float csgn, float2* vals) {
+  chained_kernel_begin();
   const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int b = (int)(id & ((1 << lgnb) - 1));
   const long long i = id >> lgnb;
@@ -178,6 +179,7 @@ __device__ __forceinline__ void red_add4(float2* p, float2 a, float2 b) {
 
 template <int DIM>
 __global__ void __launch_bounds__(128) nufft_zero_tiles_kernel(NufftGeom g, const int* split_tiles, int lgnb, float2* grid) {
+  chained_kernel_begin();
   using T = SpreadTile<DIM>;
   const TileRuns<DIM> tr(g, split_tiles[blockIdx.x]);
   for (int i = threadIdx.x; i < T::T0 * T::T1 * (T::T2 << lgnb); i += 128) {
@@ -191,6 +193,7 @@ template <int DIM, int NB>
 __global__ void __launch_bounds__(32, NB < 4 ? 28 : NB == 4 ? 24 : DIM == 3 ? 20 : 16)
 nufft_spread_tiles_kernel(NufftGeom g, const float4* pts, const int* start, const SpreadItem* items,
                           const float2* vals, float2* grid) {
+  chained_kernel_begin();
   using T = SpreadTile<DIM>;
   constexpr int NW = T::NW, WX = NW - T::T2;  // x values last
   __shared__ float4 list[kSpreadList];  // position relative to the tile's first cell, sorted index

@@ -87,6 +87,28 @@ inline cudaEvent_t take_event() {
   return e;
 }
 
+// Launches a kernel that begins with chained_kernel_begin as a programmatic dependent of the kernel
+// before it: it is set up while that one runs and starts as its last CTA leaves.  For the passes of small
+// calls, the CG's vector kernels and the NUFFT, where the gaps between launches are a tenth of the time.  Measured
+// against plain launches: 64^3 apply 28.5 -> 26.1 us, 64^3 x 8 coils 86.9 -> 82.0 us, five CG iterations
+// of it 692 -> 620 us; 128^3 x 16 coils x 10 systems the same; 2-D NUFFT there and back, 128^2 x 8,
+// 77 -> 63 us.  With the next kernel released at the start
+// (an explicit trigger) its CTAs take room from the last ones of the running kernel: 87.4 and 669 us.
+template <class... P, class... A>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, const A&... args) {
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // Counts one kernel launch; while profiling, brackets it with an event pair on `st`.
 struct LaunchScope {
   int kind;
