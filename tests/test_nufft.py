@@ -221,6 +221,22 @@ def test_every_pass_length_and_group_of_transforms(cuda, shape, nt):
             assert O.rel_l2(f[t], ref[t]) < bound and O.rel_l2(y[t], ref2[t]) < bound
 
 
+@pytest.mark.parametrize("shape", [(48, 16), (32,)])
+def test_five_transforms_of_a_lower_dimensional_plan(cuda, shape):
+    """One group of eight with three unused transforms, then a group of its own after it.  Bound as in
+    test_every_pass_length_and_group_of_transforms."""
+    d, K = len(shape), 300
+    bound = 1e-5 + 1.41e-7 * 2 * max(shape)
+    coords = np.random.default_rng(33).uniform(-np.pi, np.pi, (d, K)).astype(np.float32)
+    plan = NufftPlan(torch.from_numpy(coords).to(cuda), shape, tol=1e-6, maxbatch=8)
+    for nt in (5, 13):
+        c, fm = _rand((nt, K), 34), _rand((nt,) + shape, 35)
+        f, ref = _np(plan.type1(_c64(c, cuda), isign=1)), O.nudft_type1(coords, c, shape, 1)
+        y, ref2 = _np(plan.type2(_c64(fm, cuda), isign=-1)), O.nudft_type2(coords, fm, -1)
+        for t in range(nt):
+            assert O.rel_l2(f[t], ref[t]) < bound and O.rel_l2(y[t], ref2[t]) < bound
+
+
 @pytest.mark.parametrize("shape,tol,nt", [((16, 16, 16), 1e-6, 8), ((32, 8, 48), 1e-4, 3), ((4, 4, 4), 1e-3, 2),
                                           ((16, 32, 16), 1e-9, 1), ((64, 32), 1e-6, 8), ((4, 64), 1e-3, 4),
                                           ((80, 16), 1e-5, 1)])
