@@ -446,7 +446,10 @@ nufft_interp_rows_kernel(NufftGeom g, const float4* pts, const float2* grid, int
       }
       b += hi ? h : 0;
     }
-    const int same = 2 * d;  // lanes that agree above these bits hold the same transform
+    // The halving above has left every transform to LANES / V neighbouring lanes (one lane each for four
+    // transforms and four cells a load); the first of them (PL = 2: of both parts) stores.
+    constexpr int same = C::LANES / V;
+    static_assert(same >= 1 && same * V == C::LANES, "a group holds every transform");
 #pragma unroll
     for (; d >= PL; d /= 2)
       r[0] = cadd(r[0], make_float2(__shfl_xor_sync(0xffffffffu, r[0].x, d), __shfl_xor_sync(0xffffffffu, r[0].y, d)));

@@ -237,6 +237,46 @@ def test_five_transforms_of_a_lower_dimensional_plan(cuda, shape):
             assert O.rel_l2(f[t], ref[t]) < bound and O.rel_l2(y[t], ref2[t]) < bound
 
 
+@pytest.mark.parametrize("W", [2, 3, 4, 5, 6, 7, 8, 10, 16])
+def test_type2_every_width_and_group_writes_every_sample(cuda, W):
+    """Type 2 of a 3-D plan at each layout of its lanes (kernel widths with 4 and 8 cells a load, one and two
+    loads a row; groups of 1, 2, 4 and 8 transforms and their remainders), samples at both ends of the
+    periodic grid included, into an output that starts as NaN.  Bound: 5 x tol (10 x below 1e-3) plus the
+    float32 floor of test_every_pass_length_and_group_of_transforms and three axes of kernel values whose
+    exponent, up to 2.30 W, is rounded twice."""
+    shape, tol = (16, 32, 16), 1.01 * 10.0 ** (1 - W)
+    bound = (5 if W <= 4 else 10) * tol + 1e-5 + 1.41e-7 * 2 * max(shape) + 3 * 2.30 * W * 2.0 ** -23
+    ends = np.float32([-np.pi, -np.pi + 1e-4, -1e-4, 0.0, 1e-4, np.pi - 1e-4, np.pi])
+    ends = np.stack([g.ravel() for g in np.meshgrid(ends, ends, ends, indexing="ij")])
+    coords = np.concatenate([ends, _coords(150, 81)], 1).astype(np.float32)
+    K = coords.shape[1]
+    plan = NufftPlan(torch.from_numpy(coords).to(cuda), shape, tol=tol, maxbatch=8)
+    assert plan.width == W
+    fm = _rand((12,) + shape, 82)
+    ref, f = O.nudft_type2(coords, fm, -1), _c64(fm, cuda)
+    for nt in (1, 2, 3, 4, 5, 8, 12):
+        y = _np(plan.type2(f[:nt], torch.full((nt, K), complex("nan+nanj"), dtype=torch.complex64, device=cuda)))
+        for t in range(nt):
+            assert O.rel_l2(y[t], ref[t]) < bound, (nt, t)
+
+
+@pytest.mark.parametrize("ncoil", [3, 4, 5, 12])
+@pytest.mark.parametrize("tol", [1e-2, 1e-3])
+def test_sense_normal_at_coarse_tolerances(cuda, ncoil, tol):
+    """Groups of three and four coils (the remainders of 5 = 4 + 1 and 12 = 8 + 4 among them) at kernel widths 3 and
+    4, twice with other inputs between, so that a sample left out would meet stale values.  Bound: 5 x tol
+    for each of the two transforms."""
+    shape, K = (16, 16, 16), 1500
+    coords, sm = _coords(K, 83), synth.coil_maps(ncoil, shape, seed=84)
+    plan = NufftPlan(torch.from_numpy(coords).to(cuda), shape, tol=tol, maxbatch=8)
+    smt = _c64(sm, cuda)
+    for seed in (85, 86):
+        x, y = _rand(shape, seed), _rand((ncoil, K), seed + 10)
+        out = plan.sense_normal(_c64(x, cuda), smt, kdata=_c64(y, cuda))
+        ref = O.sense_normal_nufft(coords, x, sm, kdata=y)
+        assert O.rel_l2(_np(out), ref) < 10 * tol
+
+
 @pytest.mark.parametrize("shape,tol,nt", [((16, 16, 16), 1e-6, 8), ((32, 8, 48), 1e-4, 3), ((4, 4, 4), 1e-3, 2),
                                           ((16, 32, 16), 1e-9, 1), ((64, 32), 1e-6, 8), ((4, 64), 1e-3, 4),
                                           ((80, 16), 1e-5, 1)])
