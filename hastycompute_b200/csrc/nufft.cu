@@ -25,13 +25,14 @@ struct hb_nufft {
   int device;
   NufftGeom g;
   int group;                // transforms interleaved in the grid at once: 1, 2, 4 or 8
-  void* mem = nullptr;        // one allocation (null: in the creator's workspace): the arrays below up to vals
+  void* mem = nullptr;        // one allocation (null: in the creator's workspace): the arrays below up to image
   float4* pts = nullptr;      // [K] grid positions and sample numbers in bin order
   int* start = nullptr;       // [bins + 1] first position of every bin
   float* corr = nullptr;      // [N0 | N1 | N2] 1 / phi_hat
   float2* tw = nullptr;       // team twiddle tables of n0, n1, n2 (offsets 0, n0, n0 + n1)
   float2* grid = nullptr;     // [n0][n1][n2][group]
   float2* vals = nullptr;     // [K][group] values to spread, in sorted order
+  float2* image = nullptr;    // [modes] sum of the coils so far of a call with several groups
   // spreading (2-D and 3-D): pieces of tile work and the tiles cut into several
   void* items_mem = nullptr;
   SpreadItem* items = nullptr;
@@ -277,6 +278,13 @@ NufftModeOp coil_modes(const void* smaps, const int64_t* coils, int64_t b0, int 
   for (int b = 0; b < n; ++b) op.maps.s[b] = (const float2*)smaps + coils[b0 + b] * nm;
   return op;
 }
+// Where the coil sum of coils [b0, b0 + n) of ncoil starts and goes.  `out` is written by the last group
+// only, so that it may be one of the call's inputs (the normal operator in place): every group has read
+// them by then.  The groups before it keep their sum in the plan.
+void coil_sum(const hb_nufft* p, NufftModeOp* op, int64_t b0, int n, int64_t ncoil, void* out, int accumulate) {
+  op->add = b0 > 0 ? p->image : accumulate ? (const float2*)out : nullptr;
+  op->out = b0 + n < ncoil ? p->image : (float2*)out;
+}
 
 void free_plan(hb_nufft* p) {
   if (!p) return;
@@ -350,6 +358,7 @@ int create_plan(hb_nufft** out, int64_t nz, int64_t ny, int64_t nx, const float*
     p->tw = ar.take<float2>(g.n[0] + g.n[1] + g.n[2]);
     p->grid = ar.take<float2>((size_t)p->group * vol);
     p->vals = ar.take<float2>((size_t)p->group * nsamples);
+    if (!external) p->image = ar.take<float2>((size_t)g.N[0] * g.N[1] * g.N[2]);
   };
   int2* bin_rank;
   int *counts, *sums, *candidates;
@@ -555,8 +564,7 @@ int hb_sense_adjoint_nufft(const hb_nufft* plan, const void* kdata, const void* 
     const Group q = next_group(plan, ncoil - b0);
     const int nb = q.nact;
     NufftModeOp op = coil_modes(smaps, coils, b0, nb, nm);
-    op.out = (float2*)out;
-    op.accumulate = (b0 > 0 || accumulate) ? 1 : 0;
+    coil_sum(plan, &op, b0, nb, ncoil, out, accumulate);
     if (int r = type1_group(plan, {(const float2*)kdata + b0 * K, K, weights}, op, q, +1, st)) return r;
     b0 += nb;
   }
@@ -603,8 +611,7 @@ int hb_sense_normal_nufft(const hb_nufft* plan, const void* x, const void* smaps
     mid.vsgn = conj_sign(+1);
     NufftModeOp op = coil_modes(smaps, coils, b0, nb, nm);
     op.x = (const float2*)x;
-    op.out = (float2*)out;
-    op.accumulate = (b0 > 0 || accumulate) ? 1 : 0;
+    coil_sum(plan, &op, b0, nb, ncoil, out, accumulate);
     if (int r = type2_group(plan, op, mid, q, -1, st)) return r;
     if (int r = type1_from_vals(plan, op, q, +1, st)) return r;
     b0 += nb;

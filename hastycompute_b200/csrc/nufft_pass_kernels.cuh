@@ -135,14 +135,14 @@ nufft_axis_pass_kernel(float2* grid, long long row_stride, int ncols, int outer_
 
 // Mode side of a group of transforms: either plain mode arrays (transform b at f + b * f_ld),
 // or the SENSE operators' coil-weighted images: coil b's modes are maps.s[b] * x (type 2), and
-// out (+)= sum_b conj(maps.s[b]) * modes_b (type 1).
+// out = add + sum_b conj(maps.s[b]) * modes_b (type 1).
 struct NufftModeOp {
   float2* f;         // plain modes (read by type 2, written by type 1); null selects the coil form
   long long f_ld;
   float circulant;   // nonzero: type 1 writes circulant order (offset d at d mod N) times this factor
   const float2* x;   // coil form, type 2: the image
   float2* out;       // coil form, type 1: the combined image
-  int accumulate;    // coil form, type 1: add to out
+  const float2* add;  // coil form, type 1: what the sum starts from (null: zero; may be out)
   CoilMaps maps;
 };
 
@@ -288,7 +288,7 @@ nufft_grid_to_modes_kernel(NufftGeom g, const __grid_constant__ NufftModeOp op, 
         op.f[b * op.f_ld + m] = v;
       }
     } else {
-      float2 acc = op.accumulate ? op.out[m] : make_float2(0.f, 0.f);
+      float2 acc = op.add ? op.add[m] : make_float2(0.f, 0.f);
       float2 w[kNufftGroup];
 #pragma unroll
       for (int b = 0; b < kNufftGroup; ++b)

@@ -314,8 +314,8 @@ int hb_toeplitz_apply_noalloc(int64_t nz, int64_t ny, int64_t nx, const void* in
  * or [1][nsamples] (rows pairing with the transformed axes in order).
  *
  * hb_nufft_create sorts the samples by fine-grid bin (16 bytes per sample; coords is not kept) and
- * allocates one fine grid of g interleaved transforms, the sorted values of g transforms and the list
- * of spreading work, g = `maxbatch` (1..32) rounded up to 1, 2, 4 or 8 at most; it synchronises
+ * allocates one fine grid of g interleaved transforms, the sorted values of g transforms, an image and the
+ * list of spreading work, g = `maxbatch` (1..32) rounded up to 1, 2, 4 or 8 at most; it synchronises
  * `stream`.  Transforms run g at a time.  c is [ntransf][nsamples], f is
  * [ntransf][nz][ny][nx]. */
 typedef struct hb_nufft hb_nufft;
@@ -338,7 +338,8 @@ int hb_sense_adjoint_nufft(const hb_nufft* plan, const void* kdata, const void* 
  * manipulators, lib/mri/batch_sense.cpp:452-486; the coil loop of sense.ixx:426-497):
  *   out (+)= sum_b conj(S[c_b]) * type1( w * (type2(S[c_b] * x) - kdata[c_b]) ),  c_b = coils[b]
  * kdata [C][nsamples] indexed by coil number (nullable), weights [nsamples] float32
- * (nullable); with both NULL it is the explicit normal operator A^H A. */
+ * (nullable); with both NULL it is the explicit normal operator A^H A.  out may be x: it is
+ * written once every coil has been read. */
 int hb_sense_normal_nufft(const hb_nufft* plan, const void* x, const void* smaps, const int64_t* coils, int64_t ncoil,
                           const void* kdata, const float* weights, void* out, int accumulate, void* stream);
 

@@ -132,6 +132,50 @@ def test_sense_adjoint_and_forward(cuda):
     assert O.rel_l2(_np(y), O.sense_forward(coords, x, sm, coils)) < 1e-5
 
 
+@pytest.mark.parametrize("shape,ncoil,maxbatch", [((16, 16, 16), 4, 8), ((16, 16, 16), 5, 8), ((16, 16, 16), 12, 16),
+                                                  ((32, 16), 20, 32), ((16, 16, 16), 11, 4)])
+def test_sense_normal_in_place(cuda, shape, ncoil, maxbatch):
+    """The image of sense_normal as its own output, in one group of coils and in several: every group reads
+    the image as it was.  Against the oracle (1e-5 per transform) and the call with an output of its own
+    (order of the sums of crowded tiles: 1e-6)."""
+    d, K = len(shape), 1200
+    coords = np.random.default_rng(87).uniform(-np.pi, np.pi, (d, K)).astype(np.float32)
+    sm = synth.coil_maps(ncoil, (1,) * (3 - d) + shape, seed=88).reshape((ncoil,) + shape)
+    x, y = _rand(shape, 89), _rand((ncoil, K), 90)
+    w = np.random.default_rng(91).uniform(0.5, 1.0, K).astype(np.float32)
+    plan = NufftPlan(torch.from_numpy(coords).to(cuda), shape, tol=1e-6, maxbatch=maxbatch)
+    smt, kd, wt = _c64(sm, cuda), _c64(y, cuda), torch.from_numpy(w).to(cuda)
+    ref = O.sense_normal_nufft(coords, x, sm, kdata=y, weights=w)
+    apart = _np(plan.sense_normal(_c64(x, cuda), smt, kdata=kd, weights=wt))
+    xt = _c64(x, cuda)
+    assert plan.sense_normal(xt, smt, kdata=kd, weights=wt, out=xt) is xt
+    assert O.rel_l2(_np(xt), ref) < 2e-5 and O.rel_l2(_np(xt), apart) < 1e-6
+    xt = _c64(x, cuda)
+    plan.sense_normal(xt, smt, kdata=kd, weights=wt, out=xt, accumulate=True)
+    assert O.rel_l2(_np(xt), x + ref) < 2e-5
+    # the result over a coil's map: maps are read by every group, too
+    over = smt.clone()
+    plan.sense_normal(_c64(x, cuda), over, kdata=kd, weights=wt, out=over[0])
+    assert O.rel_l2(_np(over[0]), ref) < 2e-5
+    over = smt.clone()
+    plan.sense_adjoint(kd, over, out=over[0])
+    assert O.rel_l2(_np(over[0]), O.sense_adjoint(coords, y, sm)) < 1e-5
+
+
+def test_batched_sense_normal_in_place(cuda):
+    """BatchedSenseNormal.apply(x, out=x) on more coils than one group transforms (10 x tol per transform)."""
+    from hastycompute_b200.batched_sense import BatchedSenseNormal
+
+    shape, ncoil, K = (16, 16, 16), 10, 900
+    coords = [_coords(K, 92), _coords(K, 93)]
+    sm, x = synth.coil_maps(ncoil, shape, seed=94), _rand((2, 1) + shape, 95)
+    op = BatchedSenseNormal([torch.from_numpy(c) for c in coords], _c64(sm, cuda), maxbatch=16)
+    xt = _c64(x, cuda)
+    op.apply(xt, out=xt)
+    for o in range(2):
+        assert O.rel_l2(_np(xt[o, 0]), O.sense_normal_nufft(coords[o], x[o, 0], sm)) < 2e-4
+
+
 def test_nufft_normal_equals_eight_times_toeplitz(cuda):
     """type1(type2(x)) / prod(N) (the reference's explicit normal operator) equals 8x the
     Toeplitz operator built from the same samples (the scaling of compare_normal_methods,
