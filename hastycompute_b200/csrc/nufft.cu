@@ -24,14 +24,15 @@ using hb::fftl::team_tables_device;
 struct hb_nufft {
   int device;
   NufftGeom g;
-  int group;                // transforms interleaved in the grid at once: 1, 2, 4 or 8
+  int group;                // transforms interleaved in one grid: 1, 2, 4 or 8
+  int sides;                // grids side by side (1, or up to 4 of 8 transforms in small plans)
   void* mem = nullptr;        // one allocation (null: in the creator's workspace): the arrays below up to image
   float4* pts = nullptr;      // [K] grid positions and sample numbers in bin order
   int* start = nullptr;       // [bins + 1] first position of every bin
   float* corr = nullptr;      // [N0 | N1 | N2] 1 / phi_hat
   float2* tw = nullptr;       // team twiddle tables of n0, n1, n2 (offsets 0, n0, n0 + n1)
-  float2* grid = nullptr;     // [n0][n1][n2][group]
-  float2* vals = nullptr;     // [K][group] values to spread, in sorted order
+  float2* grid = nullptr;     // [sides][n0][n1][n2][group]
+  float2* vals = nullptr;     // [sides][K][group] values to spread, in sorted order
   float2* image = nullptr;    // [modes] sum of the coils so far of a call with several groups
   // spreading (2-D and 3-D): pieces of tile work and the tiles cut into several
   void* items_mem = nullptr;
@@ -76,17 +77,35 @@ const GaussLegendre& gauss_legendre() {
   return gl;
 }
 
-// Transforms of one group: nact <= NB = 1 << lgnb interleaved grids.  Sizes that are not a
-// power of two are padded, except 5 in 3-D, which runs as 4 + 1 (padding it to 8 moves 1.6 times the
-// bytes); at 3, 6 and 7, and in the small grids of 2-D and 1-D, a second set of launches costs
-// more than the padding.
+// Plans whose calls are bound by their launches: 1-D, 2-D, and 3-D of up to 16^3 modes.  (A larger 3-D grid
+// keeps the GPU busy with 8 transforms.)
+bool small_plan(const NufftGeom& g) { return g.dim < 3 || (long long)g.n[0] * g.n[1] * g.n[2] <= 32768; }
+
+// Transforms of one set of launches: nact <= nz * NB, NB = 1 << lgnb interleaved in each of nz grids.
+// Sizes that are not a power of two are padded, except 5 in 3-D, which runs as 4 + 1 (padding it to 8 moves
+// 1.6 times the bytes); at 3, 6 and 7, and in small plans, a second set of launches costs more than the
+// padding (type 1 of 5 transforms, 8^3 modes and 1 k samples: 22 us padded, 36 us as 4 + 1).
+// Beyond 8 transforms small plans run several grids in one set of launches: type 1 of 16 transforms, 64 x 64
+// modes and 3 k samples, tol 1e-3, 21 us against 40 us one grid after the other; 32 of 64 modes and 300 samples
+// 14 against 44 us.  The last grid may be padded, too: always from 5 transforms on, which would be padded on
+// their own as well, and below that where the padding is less work than another set of launches.  9
+// transforms, 160 x 160 modes, type 1: 52 us padded and 64 us on its own at 30 k samples, 147 and 131 us at
+// 150 k; 12: 147 and 147 us at 150 k.
 struct Group {
-  int nact, lgnb;
+  int nact, lgnb, nz;
 };
 Group next_group(const hb_nufft* p, int64_t left) {
+  if (left > p->group && p->sides > 1) {
+    const int64_t full = left / p->group < p->sides ? left / p->group : p->sides, rem = left - full * p->group;
+    const int64_t cells = (int64_t)p->g.n[0] * p->g.n[1] * p->g.n[2];
+    const bool pad = full < p->sides && rem > 0 &&
+                     (rem > 4 || (p->g.K + cells / 8) * (p->group - rem) <= (int64_t)1 << 19);
+    const int64_t nz = full + (pad ? 1 : 0), n = nz * p->group;
+    return {(int)(left < n ? left : n), 3, (int)nz};
+  }
   int n = (int)(left < p->group ? left : p->group);
-  if (n == 5 && p->g.dim == 3) n = 4;
-  return {n, n > 4 ? 3 : n > 2 ? 2 : n - 1};
+  if (n == 5 && !small_plan(p->g)) n = 4;
+  return {n, n > 4 ? 3 : n > 2 ? 2 : n - 1, 1};
 }
 
 template <int W>
@@ -95,7 +114,7 @@ cudaError_t spread_reductions_w(const hb_nufft* p, Group q, cudaStream_t st) {
   if (p->g.dim == 3) {  // one transform
     nufft_spread_reductions_kernel<W><<<(unsigned)((p->g.K + 255) / 256), 256, 0, st>>>(p->g, p->pts, p->vals, p->grid);
   } else {
-    const unsigned grid = (unsigned)(((p->g.K << q.lgnb) + 255) / 256);
+    const dim3 grid((unsigned)(((p->g.K << q.lgnb) + 255) / 256), q.nz);
     nufft_spread_line_kernel<W><<<grid, 256, 0, st>>>(p->g, p->pts, p->vals, q.lgnb, p->grid);
   }
   return cudaGetLastError();
@@ -104,25 +123,26 @@ template <int W>
 cudaError_t interp_w(const hb_nufft* p, const InterpDest& dst, Group q, float csgn, cudaStream_t st) {
   LaunchScope ls(HB_KERNEL_NUFFT, st);
   if (p->g.dim < 3) {
-    const unsigned grid = (unsigned)(((p->g.K << q.lgnb) + 255) / 256);
+    const dim3 grid((unsigned)(((p->g.K << q.lgnb) + 255) / 256), q.nz);
     return launch_chained(p->g.dim == 2 ? nufft_interp_points_kernel<W, 2> : nufft_interp_points_kernel<W, 1>, grid, 256, 0, st,
                           p->g, p->pts, p->grid, q.lgnb, q.nact, csgn, dst);
   }
   auto go = [&](auto kernel, int per_cta) {
-    const unsigned grid = (unsigned)((p->g.K + per_cta - 1) / per_cta);
+    const dim3 grid((unsigned)((p->g.K + per_cta - 1) / per_cta), q.nz);
     return launch_chained(kernel, grid, 32 * kInterpWarps, 0, st, p->g, p->pts, p->grid, q.nact, csgn, dst);
   };
-  if (q.lgnb == 3) return go(nufft_interp_rows_kernel<W, 8>, InterpCfg<W, 8>::PER_CTA);
-  if (q.lgnb == 2) return go(nufft_interp_rows_kernel<W, 4>, InterpCfg<W, 4>::PER_CTA);
-  if (q.lgnb == 1) return go(nufft_interp_rows_kernel<W, 2>, InterpCfg<W, 2>::PER_CTA);
-  return go(nufft_interp_rows_kernel<W, 1>, InterpCfg<W, 1>::PER_CTA);
+  if (q.nz > 1) return go(nufft_interp_rows_kernel<W, 8, true>, InterpCfg<W, 8>::PER_CTA);
+  if (q.lgnb == 3) return go(nufft_interp_rows_kernel<W, 8, false>, InterpCfg<W, 8>::PER_CTA);
+  if (q.lgnb == 2) return go(nufft_interp_rows_kernel<W, 4, false>, InterpCfg<W, 4>::PER_CTA);
+  if (q.lgnb == 1) return go(nufft_interp_rows_kernel<W, 2, false>, InterpCfg<W, 2>::PER_CTA);
+  return go(nufft_interp_rows_kernel<W, 1, false>, InterpCfg<W, 1>::PER_CTA);
 }
 
 // p->vals = the values to spread
 cudaError_t gather_values(const hb_nufft* p, const SpreadSource& src, Group q, float csgn, cudaStream_t st) {
-  const unsigned grid = (unsigned)(((p->g.K << q.lgnb) + 255) / 256);
+  const dim3 grid((unsigned)(((p->g.K << q.lgnb) + 255) / 256), q.nz);
   LaunchScope ls(HB_KERNEL_NUFFT, st);
-  return launch_chained(nufft_gather_values_kernel, grid, 256, 0, st, p->g.K, p->pts, src, q.lgnb, q.nact, csgn, p->vals);
+  return launch_chained(q.nz > 1 ? nufft_gather_values_kernel<true> : nufft_gather_values_kernel<false>, grid, 256, 0, st, p->g.K, p->pts, src, q.lgnb, q.nact, csgn, p->vals);
 }
 
 template <int DIM>
@@ -130,17 +150,18 @@ cudaError_t spread_tiles(const hb_nufft* p, Group q, cudaStream_t st) {
   if (p->nsplit > 0) {
     LaunchScope ls(HB_KERNEL_NUFFT, st);
     const cudaError_t e =
-        launch_chained(nufft_zero_tiles_kernel<DIM>, (unsigned)p->nsplit, 128, 0, st, p->g, p->split_tiles, q.lgnb, p->grid);
+        launch_chained(nufft_zero_tiles_kernel<DIM>, dim3(p->nsplit, q.nz), 128, 0, st, p->g, p->split_tiles, q.lgnb, p->grid);
     if (e != cudaSuccess) return e;
   }
   LaunchScope ls(HB_KERNEL_NUFFT, st);
   auto go = [&](auto kernel) {
-    return launch_chained(kernel, (unsigned)p->nitems, 32, 0, st, p->g, p->pts, p->start, p->items, p->vals, p->grid);
+    return launch_chained(kernel, dim3(p->nitems, q.nz), 32, 0, st, p->g, p->pts, p->start, p->items, p->vals, p->grid);
   };
-  if (q.lgnb == 3) return go(nufft_spread_tiles_kernel<DIM, 8>);
-  if (q.lgnb == 2) return go(nufft_spread_tiles_kernel<DIM, 4>);
-  if (q.lgnb == 1) return go(nufft_spread_tiles_kernel<DIM, 2>);
-  return go(nufft_spread_tiles_kernel<DIM, 1>);
+  if (q.nz > 1) return go(nufft_spread_tiles_kernel<DIM, 8, true>);
+  if (q.lgnb == 3) return go(nufft_spread_tiles_kernel<DIM, 8, false>);
+  if (q.lgnb == 2) return go(nufft_spread_tiles_kernel<DIM, 4, false>);
+  if (q.lgnb == 1) return go(nufft_spread_tiles_kernel<DIM, 2, false>);
+  return go(nufft_spread_tiles_kernel<DIM, 1, false>);
 }
 
 #define HB_W_DISPATCH(FN, ...)                                                                      \
@@ -168,43 +189,51 @@ long long nfine(const hb_nufft* p) { return (long long)p->g.n[0] * p->g.n[1] * p
 
 // ---- fine-grid passes (nufft_pass_kernels.cuh); axis twiddles at tw + {0, n0, n0 + n1} ----
 template <int L, bool PAD>
-cudaError_t axis_pass_l(const hb_nufft* p, int axis, int lgnb, cudaStream_t st) {
+cudaError_t axis_pass_l(const hb_nufft* p, int axis, Group q, cudaStream_t st) {
   using C = TilePassCfg<L>;
   constexpr size_t smem = C::SMEM * sizeof(float2);
   cudaError_t e = hb::fftl::allow_smem<nufft_axis_pass_kernel<L, PAD>>(smem);
   if (e != cudaSuccess) return e;
   const NufftGeom& g = p->g;
-  LaunchScope ls(HB_KERNEL_NUFFT, st);
-  if (axis == 0) {  // z: every (y, x) column
-    const long long ncols = (long long)g.n[1] * g.n[2] << lgnb;
-    return launch_chained(nufft_axis_pass_kernel<L, PAD>, dim3((unsigned)((ncols + 15) / 16), 1), C::THREADS, smem, st, p->grid,
-                          ncols, (int)ncols, 1, 1, 0, p->tw);
-  } else {  // y: the kept z planes
-    const int ncols = g.n[2] << lgnb;
-    return launch_chained(nufft_axis_pass_kernel<L, PAD>, dim3((ncols + 15) / 16, g.N[0]), C::THREADS, smem, st, p->grid, ncols,
-                          ncols, g.N[0], g.n[0], (long long)ncols * L, p->tw + g.n[0]);
+  const long long side = nfine(p) << q.lgnb;
+  if (axis == 0) {  // z: every (y, x) column of every side
+    const long long ncols = (long long)g.n[1] * g.n[2] << q.lgnb;
+    LaunchScope ls(HB_KERNEL_NUFFT, st);
+    return launch_chained(nufft_axis_pass_kernel<L, PAD>, dim3((unsigned)((ncols + 15) / 16), q.nz), C::THREADS, smem, st,
+                          p->grid, ncols, (int)ncols, q.nz, q.nz, side, p->tw);
   }
+  // y: the kept z planes; in 2-D every side is one plane
+  const int ncols = g.n[2] << q.lgnb, planes = g.N[0] > 1 ? 1 : q.nz;
+  for (int s = 0; s < q.nz; s += planes) {
+    LaunchScope ls(HB_KERNEL_NUFFT, st);
+    e = launch_chained(nufft_axis_pass_kernel<L, PAD>, dim3((ncols + 15) / 16, g.N[0] * planes), C::THREADS, smem, st,
+                       p->grid + s * side, ncols, ncols, g.N[0] * planes, g.n[0] * planes, (long long)ncols * L,
+                       p->tw + g.n[0]);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
-// to_grid: modes -> grid (type 2), else grid -> modes (type 1)
-template <int L>
-cudaError_t mode_pass_l(const hb_nufft* p, const NufftModeOp& op, Group q, float sgn, bool to_grid, cudaStream_t st) {
+// to_grid: modes -> grid (type 2), else grid -> modes (type 1); the grids from `side` on
+template <int L, bool SIDES>
+cudaError_t mode_pass_l(const hb_nufft* p, const NufftModeOp& op, Group q, int side, float sgn, bool to_grid, cudaStream_t st) {
   using C = TilePassCfg<L>;
   constexpr size_t smem = C::SMEM * sizeof(float2);
   const NufftGeom& g = p->g;
   const int nl = 16 >> q.lgnb;
-  const unsigned grid = (unsigned)((g.N[0] * g.N[1] + nl - 1) / nl);
+  const dim3 grid((unsigned)((g.N[0] * g.N[1] + nl - 1) / nl), q.nz);
+  float2* cells = p->grid + ((side * nfine(p)) << q.lgnb);
   const float2* tw = p->tw + g.n[0] + g.n[1];
   cudaError_t e;
   if (to_grid) {
-    if ((e = hb::fftl::allow_smem<nufft_modes_to_grid_kernel<L>>(smem)) != cudaSuccess) return e;
+    if ((e = hb::fftl::allow_smem<nufft_modes_to_grid_kernel<L, SIDES>>(smem)) != cudaSuccess) return e;
     LaunchScope ls(HB_KERNEL_NUFFT, st);
-    return launch_chained(nufft_modes_to_grid_kernel<L>, grid, C::THREADS, smem, st, g, op, q.lgnb, q.nact, sgn, p->corr, tw,
-                          p->grid);
+    return launch_chained(nufft_modes_to_grid_kernel<L, SIDES>, grid, C::THREADS, smem, st, g, op, q.lgnb, q.nact, sgn, p->corr,
+                          tw, cells);
   } else {
-    if ((e = hb::fftl::allow_smem<nufft_grid_to_modes_kernel<L>>(smem)) != cudaSuccess) return e;
+    if ((e = hb::fftl::allow_smem<nufft_grid_to_modes_kernel<L, SIDES>>(smem)) != cudaSuccess) return e;
     LaunchScope ls(HB_KERNEL_NUFFT, st);
-    return launch_chained(nufft_grid_to_modes_kernel<L>, grid, C::THREADS, smem, st, g, op, q.lgnb, q.nact, sgn, p->corr, tw,
-                          p->grid);
+    return launch_chained(nufft_grid_to_modes_kernel<L, SIDES>, grid, C::THREADS, smem, st, g, op, q.lgnb, q.nact, sgn, p->corr,
+                          tw, cells);
   }
 }
 
@@ -218,44 +247,46 @@ cudaError_t mode_pass_l(const hb_nufft* p, const NufftModeOp& op, Group q, float
     case 320: { constexpr int L = 320; return CALL; }                                 \
     default: return cudaErrorInvalidValue;                                            \
   }
-cudaError_t axis_pass(const hb_nufft* p, int axis, bool pad, int lgnb, cudaStream_t st) {
+cudaError_t axis_pass(const hb_nufft* p, int axis, bool pad, Group q, cudaStream_t st) {
   if (p->g.n[axis] == 1) return cudaSuccess;  // a degenerate axis of a 1-D or 2-D plan
-  HB_L_DISPATCH(p->g.n[axis], (pad ? axis_pass_l<L, true>(p, axis, lgnb, st) : axis_pass_l<L, false>(p, axis, lgnb, st)))
+  HB_L_DISPATCH(p->g.n[axis], (pad ? axis_pass_l<L, true>(p, axis, q, st) : axis_pass_l<L, false>(p, axis, q, st)))
 }
-cudaError_t mode_pass(const hb_nufft* p, const NufftModeOp& op, Group q, float sgn, bool to_grid, cudaStream_t st) {
-  HB_L_DISPATCH(p->g.n[2], (mode_pass_l<L>(p, op, q, sgn, to_grid, st)))
+cudaError_t mode_pass(const hb_nufft* p, const NufftModeOp& op, Group q, int side, float sgn, bool to_grid, cudaStream_t st) {
+  HB_L_DISPATCH(p->g.n[2], (q.nz > 1 ? mode_pass_l<L, true>(p, op, q, side, sgn, to_grid, st)
+                                    : mode_pass_l<L, false>(p, op, q, side, sgn, to_grid, st)))
 }
 
 // The passes transform forward; the other sign conjugates what enters and leaves the chain.
 float conj_sign(int isign) { return isign > 0 ? -1.f : 1.f; }
 
-// The whole grid = the spread values p->vals
+// The whole grids = the spread values p->vals
 cudaError_t spread(const hb_nufft* p, Group q, cudaStream_t st) {
   if (p->nitems > 0) return p->g.dim == 3 ? spread_tiles<3>(p, q, st) : spread_tiles<2>(p, q, st);
-  cudaError_t e = cudaMemsetAsync(p->grid, 0, ((size_t)nfine(p) << q.lgnb) * sizeof(float2), st);
+  cudaError_t e = cudaMemsetAsync(p->grid, 0, ((size_t)nfine(p) << q.lgnb) * q.nz * sizeof(float2), st);
   return e != cudaSuccess ? e : spread_reductions(p, q, st);
 }
 
-// One group of transforms: p->vals (already conjugated for isign) -> modes (op)
-int type1_from_vals(const hb_nufft* p, const NufftModeOp& op, Group q, int isign, cudaStream_t st) {
+// One group of transforms: p->vals (already conjugated for isign) -> grid, transformed along z and y
+int type1_grid(const hb_nufft* p, Group q, cudaStream_t st) {
   HB_CUDA(spread(p, q, st));
-  HB_CUDA(axis_pass(p, 0, false, q.lgnb, st));
-  HB_CUDA(axis_pass(p, 1, false, q.lgnb, st));
-  HB_CUDA(mode_pass(p, op, q, conj_sign(isign), false, st));
+  HB_CUDA(axis_pass(p, 0, false, q, st));
+  HB_CUDA(axis_pass(p, 1, false, q, st));
   return HB_OK;
 }
-// One group of transforms: samples (src) -> modes (op)
+// One group of transforms: samples (src) -> modes (op, plain)
 int type1_group(const hb_nufft* p, const SpreadSource& src, const NufftModeOp& op, Group q, int isign, cudaStream_t st) {
   HB_CUDA(gather_values(p, src, q, conj_sign(isign), st));
-  return type1_from_vals(p, op, q, isign, st);
+  if (int r = type1_grid(p, q, st)) return r;
+  HB_CUDA(mode_pass(p, op, q, 0, conj_sign(isign), false, st));
+  return HB_OK;
 }
 
 // One group of transforms: modes (op) -> samples (dst)
 int type2_group(const hb_nufft* p, const NufftModeOp& op, const InterpDest& dst, Group q, int isign, cudaStream_t st) {
   const float sgn = conj_sign(isign);
-  HB_CUDA(mode_pass(p, op, q, sgn, true, st));
-  HB_CUDA(axis_pass(p, 1, true, q.lgnb, st));
-  HB_CUDA(axis_pass(p, 0, true, q.lgnb, st));
+  HB_CUDA(mode_pass(p, op, q, 0, sgn, true, st));
+  HB_CUDA(axis_pass(p, 1, true, q, st));
+  HB_CUDA(axis_pass(p, 0, true, q, st));
   HB_CUDA(interp(p, dst, q, sgn, st));
   return HB_OK;
 }
@@ -278,12 +309,20 @@ NufftModeOp coil_modes(const void* smaps, const int64_t* coils, int64_t b0, int 
   for (int b = 0; b < n; ++b) op.maps.s[b] = (const float2*)smaps + coils[b0 + b] * nm;
   return op;
 }
-// Where the coil sum of coils [b0, b0 + n) of ncoil starts and goes.  `out` is written by the last group
-// only, so that it may be one of the call's inputs (the normal operator in place): every group has read
-// them by then.  The groups before it keep their sum in the plan.
-void coil_sum(const hb_nufft* p, NufftModeOp* op, int64_t b0, int n, int64_t ncoil, void* out, int accumulate) {
-  op->add = b0 > 0 ? p->image : accumulate ? (const float2*)out : nullptr;
-  op->out = b0 + n < ncoil ? p->image : (float2*)out;
+// Last step of the type 1 of coils [b0, b0 + q.nact) of ncoil (isign +1): grid lines -> their part of the
+// coil sum, one grid after the other.  `out` is written with the last coils only, so that it may be one
+// of the call's inputs (the normal operator in place): every group has read them by then.  The sum up to
+// there is kept in the plan.
+int coil_combine(const hb_nufft* p, const void* smaps, const int64_t* coils, int64_t b0, Group q, int64_t ncoil,
+                 void* out, int accumulate, cudaStream_t st) {
+  for (int side = 0; side < q.nz; ++side) {
+    const int first = side << q.lgnb, n = q.nact - first < 1 << q.lgnb ? q.nact - first : 1 << q.lgnb;
+    NufftModeOp op = coil_modes(smaps, coils, b0 + first, n, nmodes(p));
+    op.add = b0 + first > 0 ? p->image : accumulate ? (const float2*)out : nullptr;
+    op.out = b0 + first + n < ncoil ? p->image : (float2*)out;
+    HB_CUDA(mode_pass(p, op, {n, q.lgnb, 1}, side, conj_sign(+1), false, st));
+  }
+  return HB_OK;
 }
 
 void free_plan(hb_nufft* p) {
@@ -339,6 +378,7 @@ int create_plan(hb_nufft** out, int64_t nz, int64_t ny, int64_t nx, const float*
   p->group = maxbatch > 4 ? 8 : maxbatch > 2 ? 4 : maxbatch;
   const int nbins = g.nb[0] * g.nb[1] * g.nb[2];
   const long long vol = (long long)g.n[0] * g.n[1] * g.n[2];
+  p->sides = small_plan(g) ? (maxbatch + kNufftGroup - 1) / kNufftGroup : 1;
   const int ntiles = !tiles       ? 0
                      : g.dim == 3 ? (g.n[0] / SpreadTile<3>::T0) * (g.n[1] / SpreadTile<3>::T1) * (g.n[2] / SpreadTile<3>::T2)
                      : g.dim == 2 ? ((g.n[1] + SpreadTile<2>::T1 - 1) / SpreadTile<2>::T1) * (g.n[2] / SpreadTile<2>::T2)
@@ -356,8 +396,8 @@ int create_plan(hb_nufft** out, int64_t nz, int64_t ny, int64_t nx, const float*
     p->start = ar.take<int>(nbins + 1);
     p->corr = ar.take<float>(g.N[0] + g.N[1] + g.N[2]);
     p->tw = ar.take<float2>(g.n[0] + g.n[1] + g.n[2]);
-    p->grid = ar.take<float2>((size_t)p->group * vol);
-    p->vals = ar.take<float2>((size_t)p->group * nsamples);
+    p->grid = ar.take<float2>((size_t)p->sides * p->group * vol);
+    p->vals = ar.take<float2>((size_t)p->sides * p->group * nsamples);
     if (!external) p->image = ar.take<float2>((size_t)g.N[0] * g.N[1] * g.N[2]);
   };
   int2* bin_rank;
@@ -483,7 +523,7 @@ static int psf_in(const int* M, const float* coords, int64_t nsamples, double to
   if (int r = psf_plan(&np, M, coords, nsamples, tol, device, st, ar)) return r;
   NufftModeOp op = plain_modes(out, vol);
   op.circulant = (float)(1.0 / (double)vol);
-  const int rc = type1_group(np, {nullptr, 0, weights}, op, {1, 0}, +1, st);
+  const int rc = type1_group(np, {nullptr, 0, weights}, op, {1, 0, 1}, +1, st);
   free_plan(np);  // host state only: its arrays are the arena's
   return rc;
 }
@@ -562,11 +602,10 @@ int hb_sense_adjoint_nufft(const hb_nufft* plan, const void* kdata, const void* 
   if (ncoil == 0 && !accumulate) HB_CUDA(cudaMemsetAsync(out, 0, nm * sizeof(float2), st));
   for (int64_t b0 = 0; b0 < ncoil;) {
     const Group q = next_group(plan, ncoil - b0);
-    const int nb = q.nact;
-    NufftModeOp op = coil_modes(smaps, coils, b0, nb, nm);
-    coil_sum(plan, &op, b0, nb, ncoil, out, accumulate);
-    if (int r = type1_group(plan, {(const float2*)kdata + b0 * K, K, weights}, op, q, +1, st)) return r;
-    b0 += nb;
+    HB_CUDA(gather_values(plan, {(const float2*)kdata + b0 * K, K, weights}, q, conj_sign(+1), st));
+    if (int r = type1_grid(plan, q, st)) return r;
+    if (int r = coil_combine(plan, smaps, coils, b0, q, ncoil, out, accumulate, st)) return r;
+    b0 += q.nact;
   }
   return HB_OK;
 }
@@ -611,9 +650,9 @@ int hb_sense_normal_nufft(const hb_nufft* plan, const void* x, const void* smaps
     mid.vsgn = conj_sign(+1);
     NufftModeOp op = coil_modes(smaps, coils, b0, nb, nm);
     op.x = (const float2*)x;
-    coil_sum(plan, &op, b0, nb, ncoil, out, accumulate);
     if (int r = type2_group(plan, op, mid, q, -1, st)) return r;
-    if (int r = type1_from_vals(plan, op, q, +1, st)) return r;
+    if (int r = type1_grid(plan, q, st)) return r;
+    if (int r = coil_combine(plan, smaps, coils, b0, q, ncoil, out, accumulate, st)) return r;
     b0 += nb;
   }
   return HB_OK;

@@ -147,8 +147,8 @@ struct NufftModeOp {
 };
 
 // One CTA transforms 16 >> lgnb x-lines of NB = 1 << lgnb transforms: tile column = line * NB + b.
-// nact <= NB transforms exist; the others are zero and are not stored.  sgn = -1 conjugates
-// the modes.
+// A side has transforms side * NB + b; nact exist in all, the others are zero and are not stored.
+// sgn = -1 conjugates the modes.
 
 // Grid offset (cells) and y, z correction of the CTA's lines, once per CTA: 64-bit products and a division
 // per element cost more than the transform.
@@ -165,7 +165,7 @@ __device__ __forceinline__ void mode_lines(const NufftGeom& g, int line0, int nl
 }
 
 // type 2: grid lines = FFT along x of the corrected modes, at the kept (z, y) rows
-template <int L>
+template <int L, bool SIDES>
 __global__ void __launch_bounds__(TilePassCfg<L>::THREADS)
 nufft_modes_to_grid_kernel(NufftGeom g, const __grid_constant__ NufftModeOp op, int lgnb, int nact, float sgn, const float* corr,
                            const float2* tw, float2* grid) {
@@ -189,7 +189,7 @@ nufft_modes_to_grid_kernel(NufftGeom g, const __grid_constant__ NufftModeOp op, 
 #pragma unroll
   for (int k = 0; k < LD; ++k) {
     const int i = threadIdx.x + k * C::THREADS, i2 = i % N2, col = i / N2;
-    const int line = line0 + (col >> lgnb), b = col & (nb - 1);
+    const int line = line0 + (col >> lgnb), b = (side_index<SIDES>() << lgnb) + (col & (nb - 1));
     v[k] = w[k] = make_float2(0.f, 0.f);
     if (line < nlines && b < nact) {
       const long long m = (long long)line * N2 + i2;
@@ -210,6 +210,7 @@ nufft_modes_to_grid_kernel(NufftGeom g, const __grid_constant__ NufftModeOp op, 
   tile_team<C::S>(&col, &t);
   tile_fft<L, true>(tile, col, t, tws);
   __syncthreads();
+  grid += nufft_side(g, side_index<SIDES>(), nb);
   auto row_base = [&](int lc) { return grid + (cell_s[lc] << lgnb); };  // grid line of the CTA's mode line
   if (lgnb == 0) {
     for (int i = threadIdx.x; i < C::XT * L; i += C::THREADS) {
@@ -227,8 +228,9 @@ nufft_modes_to_grid_kernel(NufftGeom g, const __grid_constant__ NufftModeOp op, 
   }
 }
 
-// type 1: modes = correction x FFT along x of the grid lines at the kept (z, y) rows
-template <int L>
+// type 1: modes = correction x FFT along x of the grid lines at the kept (z, y) rows (coil form: one side a
+// launch, the sum runs through all coils)
+template <int L, bool SIDES>
 __global__ void __launch_bounds__(TilePassCfg<L>::THREADS)
 nufft_grid_to_modes_kernel(NufftGeom g, const __grid_constant__ NufftModeOp op, int lgnb, int nact, float sgn, const float* corr,
                            const float2* tw, const float2* grid) {
@@ -245,6 +247,7 @@ nufft_grid_to_modes_kernel(NufftGeom g, const __grid_constant__ NufftModeOp op, 
   __shared__ float scale_s[C::XT];
   mode_lines(g, line0, nl, corr, cell_s, scale_s);
   __syncthreads();
+  grid += nufft_side(g, side_index<SIDES>(), nb);
   auto row_base = [&](int lc) { return grid + (cell_s[lc] << lgnb); };
   if (lgnb == 0) {
     for (int i = threadIdx.x; i < C::XT * L; i += C::THREADS) {
@@ -276,7 +279,7 @@ nufft_grid_to_modes_kernel(NufftGeom g, const __grid_constant__ NufftModeOp op, 
     const float s = scale_s[lc] * corr2[i2];
     const long long m = (long long)line * N2 + i2;
     if (op.f) {
-      const int b = c & (nb - 1);
+      const int b = (side_index<SIDES>() << lgnb) + (c & (nb - 1));
       if (b >= nact) continue;
       float2 v = cscale(tile[tile_at(r, c)], s);
       v.y *= sgn;

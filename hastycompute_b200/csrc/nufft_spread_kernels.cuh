@@ -153,19 +153,20 @@ nufft_tile_items_kernel(NufftGeom g, int ntiles, int cap, const int* candidates,
 }
 
 // ---- per call ----
-// vals[i][b] = the value of sorted sample i for transform b (zero for b >= nact), so that a tile
+// vals[side][i][b] = the value of sorted sample i for transform side * NB + b (zero from nact on), so that a tile
 // reads a sample's NB values as one contiguous run: gathered straight from the caller's
 // [transform][sample] rows, every visit of a sample (about 11 of them at W = 7) touched NB
 // separate cache lines.
+template <bool SIDES>
 __global__ void __launch_bounds__(256) nufft_gather_values_kernel(long long K, const float4* pts,
                                                                   const __grid_constant__ SpreadSource src, int lgnb,
                                                                   int nact, float csgn, float2* vals) {
   chained_kernel_begin();
   const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int b = (int)(id & ((1 << lgnb) - 1));
+  const int side = side_index<SIDES>(), b = (side << lgnb) + (int)(id & ((1 << lgnb) - 1));
   const long long i = id >> lgnb;
   if (i >= K) return;
-  vals[id] = b < nact ? spread_value(src, b, __float_as_int(pts[i].w), csgn) : make_float2(0.f, 0.f);
+  vals[(side * K << lgnb) + id] = b < nact ? spread_value(src, b, __float_as_int(pts[i].w), csgn) : make_float2(0.f, 0.f);
 }
 
 __device__ __forceinline__ void store_cell8(float2* p, const float2* v) {  // four float2, one 32-byte store
@@ -181,6 +182,7 @@ template <int DIM>
 __global__ void __launch_bounds__(128) nufft_zero_tiles_kernel(NufftGeom g, const int* split_tiles, int lgnb, float2* grid) {
   chained_kernel_begin();
   using T = SpreadTile<DIM>;
+  grid += nufft_side(g, blockIdx.y, 1 << lgnb);
   const TileRuns<DIM> tr(g, split_tiles[blockIdx.x]);
   for (int i = threadIdx.x; i < T::T0 * T::T1 * (T::T2 << lgnb); i += 128) {
     const int q = i % (T::T2 << lgnb), y = (i / (T::T2 << lgnb)) % T::T1, z = i / ((T::T2 << lgnb) * T::T1);
@@ -189,7 +191,7 @@ __global__ void __launch_bounds__(128) nufft_zero_tiles_kernel(NufftGeom g, cons
   }
 }
 
-template <int DIM, int NB>
+template <int DIM, int NB, bool SIDES>
 __global__ void __launch_bounds__(32, NB < 4 ? 28 : NB == 4 ? 24 : DIM == 3 ? 20 : 16)
 nufft_spread_tiles_kernel(NufftGeom g, const float4* pts, const int* start, const SpreadItem* items,
                           const float2* vals, float2* grid) {
@@ -200,6 +202,9 @@ nufft_spread_tiles_kernel(NufftGeom g, const float4* pts, const int* start, cons
   __shared__ __align__(16) float w_s[kSpreadBatch][NW];
   __shared__ __align__(16) float2 c_s[kSpreadBatch][NB];
   const int lane = threadIdx.x;
+  const int side = side_index<SIDES>();
+  vals += side * g.K * NB;
+  grid += nufft_side(g, side, NB);
   const SpreadItem it = items[blockIdx.x];
   const TileRuns<DIM> tr(g, it.origin);
 

@@ -316,7 +316,8 @@ int hb_toeplitz_apply_noalloc(int64_t nz, int64_t ny, int64_t nx, const void* in
  * hb_nufft_create sorts the samples by fine-grid bin (16 bytes per sample; coords is not kept) and
  * allocates one fine grid of g interleaved transforms, the sorted values of g transforms, an image and the
  * list of spreading work, g = `maxbatch` (1..32) rounded up to 1, 2, 4 or 8 at most; it synchronises
- * `stream`.  Transforms run g at a time.  c is [ntransf][nsamples], f is
+ * `stream`.  Transforms run g at a time; 1-D and 2-D plans, and 3-D plans of up to 16^3 modes, have one
+ * such grid and set of values per 8 of maxbatch and run them together.  c is [ntransf][nsamples], f is
  * [ntransf][nz][ny][nx]. */
 typedef struct hb_nufft hb_nufft;
 int hb_nufft_create(hb_nufft** plan, int64_t nz, int64_t ny, int64_t nx, const float* coords, int64_t nsamples,

@@ -321,6 +321,33 @@ def test_sense_normal_at_coarse_tolerances(cuda, ncoil, tol):
         assert O.rel_l2(_np(out), ref) < 10 * tol
 
 
+@pytest.mark.parametrize("shape,nt,maxbatch,K", [((32, 16), 9, 16, 300), ((16, 16), 9, 16, 40000), ((16, 16), 13, 16, 40000),
+                                                 ((32, 16), 24, 16, 300), ((48, 16), 40, 32, 200), ((64,), 19, 32, 300),
+                                                 ((16,), 32, 32, 50000), ((8, 8, 8), 16, 16, 500), ((16, 16, 16), 11, 16, 300)])
+def test_batches_above_eight_transforms(cuda, shape, nt, maxbatch, K):
+    """Small plans run several grids of eight transforms at once, with the last one padded or on its own,
+    and batches beyond maxbatch.  Outputs start as NaN.  Bound as in test_every_pass_length_and_group_of_transforms."""
+    d = len(shape)
+    bound = 1e-5 + 1.41e-7 * 2 * max(shape)
+    coords = np.random.default_rng(61).uniform(-np.pi, np.pi, (d, K)).astype(np.float32)
+    plan = NufftPlan(torch.from_numpy(coords).to(cuda), shape, tol=1e-6, maxbatch=maxbatch)
+    c, fm = _rand((nt, K), 62), _rand((nt,) + shape, 63)
+    nan = complex("nan+nanj")
+    f = _np(plan.type1(_c64(c, cuda), torch.full((nt,) + shape, nan, dtype=torch.complex64, device=cuda), isign=-1))
+    y = _np(plan.type2(_c64(fm, cuda), torch.full((nt, K), nan, dtype=torch.complex64, device=cuda), isign=+1))
+    ref, ref2 = O.nudft_type1(coords, c, shape, -1), O.nudft_type2(coords, fm, +1)
+    for t in range(nt):
+        assert O.rel_l2(f[t], ref[t]) < bound and O.rel_l2(y[t], ref2[t]) < bound
+    # the coils of a SENSE operator in the same groups
+    sm, x = _rand((nt,) + shape, 64), _rand(shape, 65)
+    smt = _c64(sm, cuda)
+    k = _np(plan.sense_forward(_c64(x, cuda), smt))
+    ref = O.sense_forward(coords, x, sm)
+    for t in range(nt):
+        assert O.rel_l2(k[t], ref[t]) < bound
+    assert O.rel_l2(_np(plan.sense_adjoint(_c64(c, cuda), smt)), O.sense_adjoint(coords, c, sm)) < bound
+
+
 @pytest.mark.parametrize("shape,tol,nt", [((16, 16, 16), 1e-6, 8), ((32, 8, 48), 1e-4, 3), ((4, 4, 4), 1e-3, 2),
                                           ((16, 32, 16), 1e-9, 1), ((64, 32), 1e-6, 8), ((4, 64), 1e-3, 4),
                                           ((80, 16), 1e-5, 1)])
