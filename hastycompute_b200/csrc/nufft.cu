@@ -86,8 +86,8 @@ bool small_plan(const NufftGeom& g) { return g.dim < 3 || (long long)g.n[0] * g.
 // 1.6 times the bytes); at 3, 6 and 7, and in small plans, a second set of launches costs more than the
 // padding (type 1 of 5 transforms, 8^3 modes and 1 k samples: 22 us padded, 36 us as 4 + 1).
 // Beyond 8 transforms small plans run several grids in one set of launches: type 1 of 16 transforms, 64 x 64
-// modes and 3 k samples, tol 1e-3, 21 us against 40 us one grid after the other; 32 of 64 modes and 300 samples
-// 14 against 44 us.  The last grid may be padded, too: always from 5 transforms on, which would be padded on
+// modes and 3 k samples, tol 1e-3, 22 us against 40 us one grid after the other; 32 of 64 modes and 300 samples
+// 17 against 44 us.  The last grid may be padded, too: always from 5 transforms on, which would be padded on
 // their own as well, and below that where the padding is less work than another set of launches.  9
 // transforms, 160 x 160 modes, type 1: 52 us padded and 64 us on its own at 30 k samples, 147 and 131 us at
 // 150 k; 12: 147 and 147 us at 150 k.
@@ -138,21 +138,28 @@ cudaError_t interp_w(const hb_nufft* p, const InterpDest& dst, Group q, float cs
   return go(nufft_interp_rows_kernel<W, 1, false>, InterpCfg<W, 1>::PER_CTA);
 }
 
-// p->vals = the values to spread
-cudaError_t gather_values(const hb_nufft* p, const SpreadSource& src, Group q, float csgn, cudaStream_t st) {
-  const dim3 grid((unsigned)(((p->g.K << q.lgnb) + 255) / 256), q.nz);
+// p->vals = the values to spread, and zeros in the split tiles
+template <int DIM>
+cudaError_t gather_dim(const hb_nufft* p, const SpreadSource& src, Group q, float csgn, cudaStream_t st) {
+  const unsigned ctas = (unsigned)(((p->g.K << q.lgnb) + 255) / 256);
   LaunchScope ls(HB_KERNEL_NUFFT, st);
-  return launch_chained(q.nz > 1 ? nufft_gather_values_kernel<true> : nufft_gather_values_kernel<false>, grid, 256, 0, st, p->g.K, p->pts, src, q.lgnb, q.nact, csgn, p->vals);
+  return launch_chained(q.nz > 1 ? nufft_gather_values_kernel<DIM, true> : nufft_gather_values_kernel<DIM, false>,
+                        dim3(ctas + p->nsplit, q.nz), 256, 0, st, p->g, p->pts, src, q.lgnb, q.nact, csgn, p->vals, ctas,
+                        p->split_tiles, p->grid);
+}
+cudaError_t gather_values(const hb_nufft* p, const SpreadSource& src, Group q, float csgn, cudaStream_t st) {
+  return p->g.dim == 3 ? gather_dim<3>(p, src, q, csgn, st) : gather_dim<2>(p, src, q, csgn, st);
+}
+// Zeros in the split tiles, where interpolation has written p->vals
+cudaError_t zero_tiles(const hb_nufft* p, Group q, cudaStream_t st) {
+  if (p->nsplit == 0) return cudaSuccess;
+  LaunchScope ls(HB_KERNEL_NUFFT, st);
+  return launch_chained(p->g.dim == 3 ? nufft_zero_tiles_kernel<3> : nufft_zero_tiles_kernel<2>, dim3(p->nsplit, q.nz), 128, 0,
+                        st, p->g, p->split_tiles, q.lgnb, p->grid);
 }
 
 template <int DIM>
 cudaError_t spread_tiles(const hb_nufft* p, Group q, cudaStream_t st) {
-  if (p->nsplit > 0) {
-    LaunchScope ls(HB_KERNEL_NUFFT, st);
-    const cudaError_t e =
-        launch_chained(nufft_zero_tiles_kernel<DIM>, dim3(p->nsplit, q.nz), 128, 0, st, p->g, p->split_tiles, q.lgnb, p->grid);
-    if (e != cudaSuccess) return e;
-  }
   LaunchScope ls(HB_KERNEL_NUFFT, st);
   auto go = [&](auto kernel) {
     return launch_chained(kernel, dim3(p->nitems, q.nz), 32, 0, st, p->g, p->pts, p->start, p->items, p->vals, p->grid);
@@ -259,7 +266,7 @@ cudaError_t mode_pass(const hb_nufft* p, const NufftModeOp& op, Group q, int sid
 // The passes transform forward; the other sign conjugates what enters and leaves the chain.
 float conj_sign(int isign) { return isign > 0 ? -1.f : 1.f; }
 
-// The whole grids = the spread values p->vals
+// The whole grids = the spread values p->vals; the split tiles are zeroed
 cudaError_t spread(const hb_nufft* p, Group q, cudaStream_t st) {
   if (p->nitems > 0) return p->g.dim == 3 ? spread_tiles<3>(p, q, st) : spread_tiles<2>(p, q, st);
   cudaError_t e = cudaMemsetAsync(p->grid, 0, ((size_t)nfine(p) << q.lgnb) * q.nz * sizeof(float2), st);
@@ -651,6 +658,7 @@ int hb_sense_normal_nufft(const hb_nufft* plan, const void* x, const void* smaps
     NufftModeOp op = coil_modes(smaps, coils, b0, nb, nm);
     op.x = (const float2*)x;
     if (int r = type2_group(plan, op, mid, q, -1, st)) return r;
+    HB_CUDA(zero_tiles(plan, q, st));
     if (int r = type1_grid(plan, q, st)) return r;
     if (int r = coil_combine(plan, smaps, coils, b0, q, ncoil, out, accumulate, st)) return r;
     b0 += nb;

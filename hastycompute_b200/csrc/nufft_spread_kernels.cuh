@@ -153,20 +153,45 @@ nufft_tile_items_kernel(NufftGeom g, int ntiles, int cap, const int* candidates,
 }
 
 // ---- per call ----
+// Zeroes the cells of a tile that several pieces add into.
+template <int DIM, int THREADS>
+__device__ __forceinline__ void zero_tile(const NufftGeom& g, int origin, int lgnb, float2* grid) {
+  using T = SpreadTile<DIM>;
+  const int o0 = origin >> 20, o1 = (origin >> 10) & 1023, o2 = origin & 1023;
+  for (int i = threadIdx.x; i < T::T0 * T::T1 * (T::T2 << lgnb); i += THREADS) {
+    const int q = i % (T::T2 << lgnb), y = (i / (T::T2 << lgnb)) % T::T1, z = i / ((T::T2 << lgnb) * T::T1);
+    if (o1 + y < g.n[1])
+      grid[((((long long)(o0 + z) * g.n[1] + o1 + y) * g.n[2] + o2) << lgnb) + q] = make_float2(0.f, 0.f);
+  }
+}
+template <int DIM>
+__global__ void __launch_bounds__(128) nufft_zero_tiles_kernel(NufftGeom g, const int* split_tiles, int lgnb, float2* grid) {
+  chained_kernel_begin();
+  zero_tile<DIM, 128>(g, split_tiles[blockIdx.x], lgnb, grid + nufft_side(g, blockIdx.y, 1 << lgnb));
+}
+
 // vals[side][i][b] = the value of sorted sample i for transform side * NB + b (zero from nact on), so that a tile
 // reads a sample's NB values as one contiguous run: gathered straight from the caller's
 // [transform][sample] rows, every visit of a sample (about 11 of them at W = 7) touched NB
-// separate cache lines.
-template <bool SIDES>
-__global__ void __launch_bounds__(256) nufft_gather_values_kernel(long long K, const float4* pts,
+// separate cache lines.  CTAs from `gather_ctas` on zero a split tile each: a launch of their own costs
+// 2 us, which a type 1 of one 160 x 160 slice with 150 k samples (45 us) had lost against spreading by reductions.
+template <int DIM, bool SIDES>
+__global__ void __launch_bounds__(256) nufft_gather_values_kernel(NufftGeom g, const float4* pts,
                                                                   const __grid_constant__ SpreadSource src, int lgnb,
-                                                                  int nact, float csgn, float2* vals) {
+                                                                  int nact, float csgn, float2* vals,
+                                                                  unsigned gather_ctas, const int* split_tiles,
+                                                                  float2* grid) {
   chained_kernel_begin();
+  const int side = side_index<SIDES>();
+  if (blockIdx.x >= gather_ctas) {
+    zero_tile<DIM, 256>(g, split_tiles[blockIdx.x - gather_ctas], lgnb, grid + nufft_side(g, side, 1 << lgnb));
+    return;
+  }
   const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int side = side_index<SIDES>(), b = (side << lgnb) + (int)(id & ((1 << lgnb) - 1));
+  const int b = (side << lgnb) + (int)(id & ((1 << lgnb) - 1));
   const long long i = id >> lgnb;
-  if (i >= K) return;
-  vals[(side * K << lgnb) + id] = b < nact ? spread_value(src, b, __float_as_int(pts[i].w), csgn) : make_float2(0.f, 0.f);
+  if (i >= g.K) return;
+  vals[(side * g.K << lgnb) + id] = b < nact ? spread_value(src, b, __float_as_int(pts[i].w), csgn) : make_float2(0.f, 0.f);
 }
 
 __device__ __forceinline__ void store_cell8(float2* p, const float2* v) {  // four float2, one 32-byte store
@@ -176,19 +201,6 @@ __device__ __forceinline__ void store_cell8(float2* p, const float2* v) {  // fo
 }
 __device__ __forceinline__ void red_add4(float2* p, float2 a, float2 b) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y) : "memory");
-}
-
-template <int DIM>
-__global__ void __launch_bounds__(128) nufft_zero_tiles_kernel(NufftGeom g, const int* split_tiles, int lgnb, float2* grid) {
-  chained_kernel_begin();
-  using T = SpreadTile<DIM>;
-  grid += nufft_side(g, blockIdx.y, 1 << lgnb);
-  const TileRuns<DIM> tr(g, split_tiles[blockIdx.x]);
-  for (int i = threadIdx.x; i < T::T0 * T::T1 * (T::T2 << lgnb); i += 128) {
-    const int q = i % (T::T2 << lgnb), y = (i / (T::T2 << lgnb)) % T::T1, z = i / ((T::T2 << lgnb) * T::T1);
-    if (tr.o[1] + y < g.n[1])
-      grid[((((long long)(tr.o[0] + z) * g.n[1] + tr.o[1] + y) * g.n[2] + tr.o[2]) << lgnb) + q] = make_float2(0.f, 0.f);
-  }
 }
 
 template <int DIM, int NB, bool SIDES>
