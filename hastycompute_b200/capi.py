@@ -91,6 +91,7 @@ SIGNATURES = {
                                 c_int, c_void_p]),
     "hb_nufft_destroy": (c_int, [c_void_p]),
     "hb_nufft_width": (c_int, [c_void_p]),
+    "hb_nufft_kernel_values": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_i64, c_void_p]),
     "hb_nufft_type1": (c_int, [c_void_p, c_void_p, c_void_p, c_i64, c_int, c_void_p]),
     "hb_nufft_type2": (c_int, [c_void_p, c_void_p, c_void_p, c_i64, c_int, c_void_p]),
     "hb_sense_adjoint_nufft": (c_int, [c_void_p, c_void_p, c_void_p, P_i64, c_i64, c_void_p, c_void_p, c_int,

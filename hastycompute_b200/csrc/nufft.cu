@@ -567,6 +567,18 @@ int hb_nufft_destroy(hb_nufft* plan) {
 
 int hb_nufft_width(const hb_nufft* plan) { return plan ? plan->g.w : -1; }
 
+int hb_nufft_kernel_values(const hb_nufft* plan, const float* z, const float* s, float* phi, float* root, int64_t n,
+                           void* stream) {
+  if (!plan || !z || !s || !phi || !root || n < 1 || n > (int64_t)0x7fffffff)
+    return fail(HB_ERR_INVALID, "hb_nufft_kernel_values: null argument or n out of range");
+  DeviceGuard dg(plan->device);
+  LaunchScope ls(HB_KERNEL_NUFFT, (cudaStream_t)stream);
+  nufft_kernel_values_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(plan->g.w, plan->g.beta, z, s, phi,
+                                                                                       root, n);
+  HB_CUDA(cudaGetLastError());
+  return HB_OK;
+}
+
 int hb_nufft_type1(const hb_nufft* plan, const void* c, void* f, int64_t ntransf, int isign, void* stream) {
   if (!plan || !c || !f || ntransf < 0 || (isign != 1 && isign != -1))
     return fail(HB_ERR_INVALID, "hb_nufft_type1: null argument, negative ntransf or isign not +-1");

@@ -325,6 +325,10 @@ int hb_nufft_create(hb_nufft** plan, int64_t nz, int64_t ny, int64_t nx, const f
 int hb_nufft_destroy(hb_nufft* plan);
 /* Kernel width w (fine-grid cells) the plan uses. */
 int hb_nufft_width(const hb_nufft* plan);
+/* Tests: phi[i] = the plan's kernel at z[i] fine-grid cells from a sample, root[i] = the square root that
+ * the kernel takes of its argument, at s[i] in [1e-30, 1].  Device arrays of n. */
+int hb_nufft_kernel_values(const hb_nufft* plan, const float* z, const float* s, float* phi, float* root, int64_t n,
+                           void* stream);
 int hb_nufft_type1(const hb_nufft* plan, const void* c, void* f, int64_t ntransf, int isign, void* stream);
 int hb_nufft_type2(const hb_nufft* plan, const void* f, void* c, int64_t ntransf, int isign, void* stream);
 

@@ -348,6 +348,38 @@ def test_batches_above_eight_transforms(cuda, shape, nt, maxbatch, K):
     assert O.rel_l2(_np(plan.sense_adjoint(_c64(c, cuda), smt)), O.sense_adjoint(coords, c, sm)) < bound
 
 
+@pytest.mark.parametrize("W", [2, 4, 5, 7, 10, 16])
+def test_gridding_kernel_values_and_their_square_root(cuda, W):
+    """The kernel's own square root against FP64, s dense in [0, 1], towards 1 and down to the clamp at 1e-30: within
+    0.5 + 2^-18 ulp.  The kernel exp(beta (sqrt(1 - t^2) - 1)) against FP64: t rounded twice and s once leave s within
+    ds = 1.5 2^-22, the root within ds / sqrt(s) (at the edge sqrt(2 ds)) and two roundings, exp within 2 ulp."""
+    n = 200000
+    plan = NufftPlan(torch.from_numpy(_coords(10, 97)).to(cuda), (16, 16, 16), tol=1.01 * 10.0 ** (1 - W))
+    assert plan.width == W
+    rng = np.random.default_rng(98)
+    s = np.concatenate([rng.uniform(0, 1, n // 4), 10.0 ** rng.uniform(-30, 0, n // 4), 1 - 2.0 ** rng.uniform(-24, 0, n // 4),
+                        [1.0, 1e-30, 2.0 ** -24, 0.25]])
+    s = np.clip(np.concatenate([s, rng.uniform(0.25, 1, n - len(s))]).astype(np.float32), np.float32(1e-30), 1)
+    z = rng.uniform(-0.5 * W, 0.5 * W, n).astype(np.float32)
+    z[:4] = [0.0, 0.5 * W, -0.5 * W, 0.51 * W]
+    zt, st = torch.from_numpy(z).to(cuda), torch.from_numpy(s).to(cuda)
+    phi, root = torch.empty_like(zt), torch.empty_like(zt)
+    capi.check(plan.lib.hb_nufft_kernel_values(plan._h, zt.data_ptr(), st.data_ptr(), phi.data_ptr(), root.data_ptr(), n,
+                                               torch.cuda.current_stream(cuda).cuda_stream))
+    exact = np.sqrt(s.astype(np.float64))
+    off = np.abs(root.cpu().numpy().astype(np.float64) - exact) / np.spacing(exact.astype(np.float32))
+    assert off.max() <= 0.5 + 2.0 ** -18
+    beta = float(np.float32(2.30 * W))
+    q = np.maximum(1 - (z.astype(np.float64) / (0.5 * W)) ** 2, 0)
+    ref = np.where(q > 0, np.exp(beta * (np.sqrt(q) - 1)), 0)
+    ds = 1.5 * 2.0 ** -22
+    dr = np.where(q > ds, ds / np.sqrt(np.maximum(q, ds)), np.sqrt(2 * ds)) + 2.0 ** -23
+    rel = np.expm1(beta * dr) + beta * 2.0 ** -24 + 2.0 ** -22
+    got = phi.cpu().numpy().astype(np.float64)
+    assert (np.abs(got - ref) <= np.where(q > ds, ref * rel, np.exp(beta * (np.sqrt(2 * ds) - 1)) * (1 + rel))).all()
+    assert got[0] == 1.0 and got[3] == 0.0
+
+
 @pytest.mark.parametrize("shape,tol,nt", [((16, 16, 16), 1e-6, 8), ((32, 8, 48), 1e-4, 3), ((4, 4, 4), 1e-3, 2),
                                           ((16, 32, 16), 1e-9, 1), ((64, 32), 1e-6, 8), ((4, 64), 1e-3, 4),
                                           ((80, 16), 1e-5, 1)])
