@@ -9,8 +9,9 @@
 // it.  With M = U S V^H: soft f(s) = max(s - thresh, 0), hard keeps the `rank` largest s,
 // and the block is replaced by U f(S) V^H = M W,  W = V diag(f(s)/s) V^H  (0 where s = 0).
 // One CTA of 128 threads per block, columns padded to a multiple of four:
-//   1. G = M^H M in FP64: rows are staged in shared memory as doubles (converted once), every
-//      thread accumulates one 4 x 4 tile of G over its share of the rows in registers;
+//   1. G = M^H M in FP64: rows are staged in shared memory in single precision and converted as a
+//      thread reads them; every thread accumulates one 4 x 4 tile of G over its share of the rows (its
+//      group's) in registers, and the groups' sums are added up;
 //   2. G is diagonalised by Jacobi rotations (FP64), G = V diag(lambda) V^H, s = sqrt(lambda): a round
 //      rotates the n / 2 disjoint pairs of a round-robin tournament at once, each 2 x 2 block of
 //      A' = J^H A J by one thread, so a round takes two barriers;
@@ -96,7 +97,14 @@ struct SvtCfg {
   static constexpr int NC = 4 * NT;
   static constexpr int LD = NC + 1;                      // odd pitch in 16-byte units: rows on distinct banks
   static constexpr int TILES = NT * (NT + 1) / 2;        // upper-triangle tiles of G
-  static constexpr int GROUPS = kSvtThreads / TILES;     // row groups
+  // Row groups.  Up to 12 columns there are so many (128, 40, 20) that they are added up by shuffles within a
+  // warp before the warps' sums go to shared memory one after the other, and a warp holds whole groups: one
+  // group after the other took 20 us of a block of 4 columns (512 blocks of 8 rows x 4 columns 31 us, now 11; 18
+  // with one warp making the rotations; 64 blocks of 2560 x 4 62 -> 43, x 8 106 -> 99, x 12 170 -> 169).  From 13
+  // columns on whole groups would leave a warp's lanes idle, and there are 12 sums or fewer.
+  static constexpr bool SHUFFLE = NT <= 3;
+  static constexpr int WARP_GROUPS = 32 / TILES;  // SHUFFLE: groups in a warp
+  static constexpr int GROUPS = SHUFFLE ? kSvtThreads / 32 * WARP_GROUPS : kSvtThreads / TILES;
   static constexpr int RLD = NC + 2;                     // pitch of the staged rows
   static constexpr size_t SMEM = (size_t)2 * NC * LD * sizeof(double2) + (size_t)kSvtChunk * RLD * sizeof(float2);
   static_assert(kSvtChunk * RLD >= NC * NC, "W takes the place of the staged rows");
@@ -135,7 +143,9 @@ __global__ void __launch_bounds__(kSvtThreads, 4) svt_blocks_kernel(SvtArgs a) {
   const long long col_stride = (long long)a.d1 * a.S0 * a.S1 * a.S2;
 
   // 1. Gram matrix: thread (tile, group) accumulates G[4 ti + i][4 tj + j] over rows group, group + GROUPS, ...
-  const int tile = tid % C::TILES, group = tid / C::TILES;
+  const int wgroup = tid % 32 / C::TILES;  // SHUFFLE: the group's number in its warp
+  const int tile = (C::SHUFFLE ? tid % 32 : tid) % C::TILES;
+  const int group = !C::SHUFFLE ? tid / C::TILES : wgroup < C::WARP_GROUPS ? tid / 32 * C::WARP_GROUPS + wgroup : C::GROUPS;
   int ti = 0, tj = tile;
   while (tj >= NT - ti) {
     tj -= NT - ti;
@@ -199,9 +209,27 @@ __global__ void __launch_bounds__(kSvtThreads, 4) svt_blocks_kernel(SvtArgs a) {
     }
   }
   for (int i = tid; i < NC * LD; i += kSvtThreads) V[i] = make_double2(i / LD == i % LD ? 1.0 : 0.0, 0.0);
+  // the groups add up in a fixed order
+  if constexpr (C::SHUFFLE) {
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+      if (d >= C::WARP_GROUPS) continue;
+      const bool add = wgroup < d && wgroup + d < C::WARP_GROUPS;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const double x = __shfl_down_sync(0xffffffffu, g[i][j].x, d * C::TILES);
+          const double y = __shfl_down_sync(0xffffffffu, g[i][j].y, d * C::TILES);
+          if (add) g[i][j] = make_double2(g[i][j].x + x, g[i][j].y + y);
+        }
+    }
+  }
+  constexpr int SUMS = C::SHUFFLE ? kSvtThreads / 32 : C::GROUPS;
+  const int sum = !C::SHUFFLE ? group : wgroup == 0 ? tid / 32 : SUMS;  // this thread's, if it has one
 #pragma unroll 1
-  for (int k = 0; k < C::GROUPS; ++k) {  // groups add up in a fixed order
-    if (group == k) {
+  for (int k = 0; k < SUMS; ++k) {
+    if (sum == k) {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll

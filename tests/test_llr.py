@@ -107,3 +107,16 @@ def test_svt_odd_columns_and_rows(cuda, d0, d1, block, soft, thresh):
     xt = _c64(x, cuda)
     svt_blocks(xt, corners, block, thresh, soft)
     assert O.rel_l2(_np(xt), O.svt_blocks(x, corners, block, thresh, soft)) < 1e-5
+
+
+@pytest.mark.parametrize("d0", [2, 4, 7, 9, 10, 12])
+@pytest.mark.parametrize("d1,block", [(1, (2, 2, 2)), (2, (5, 7, 3))])
+def test_svt_few_columns(cuda, d0, d1, block):
+    """Up to 12 columns the row groups of the Gram matrix are summed within warps: fewer rows than groups, and
+    rows off their number.  Tolerance as test_svt_blocks_against_numpy_svd."""
+    S = (11, 12, 9)
+    x = _lowrank(d0, d1, S, min(2, d0), seed=70 + d0)
+    corners = [(0, 0, 0), tuple(s - b for s, b in zip(S, block))]
+    xt = _c64(x, cuda)
+    svt_blocks(xt, corners, block, 1.5, True)
+    assert O.rel_l2(_np(xt), O.svt_blocks(x, corners, block, 1.5, True)) < 1e-5
