@@ -95,9 +95,8 @@ __global__ void __launch_bounds__(THREADS_) plane_full_kernel(PassArgs a) {
     constexpr int LPZ = (M1 + NTZ - 1) / NTZ;
     const int col0 = row_of_team<SZ, NTZ, M1>(team);
     auto tcol = [&](int ky) { return T + ((long long)(ky & 1) * N1 + (ky >> 1)) * M0; };
-    constexpr bool kRegTw = EZ <= 16;
-    float2 twz[kRegTw ? EZ : 1];
-    if constexpr (kRegTw) load_lane_twiddles<M0>(twz, tw_z, t);
+    float2 twz[EZ];
+    load_lane_twiddles<M0>(twz, tw_z, t);
     float tnext[EZ];
     load_tcol<EZ, SZ>(tnext, tcol(col0 < M1 ? col0 : 0), t);
 #pragma unroll 2
@@ -111,13 +110,11 @@ __global__ void __launch_bounds__(THREADS_) plane_full_kernel(PassArgs a) {
       float2 v[EZ];
 #pragma unroll
       for (int e = 0; e < EZ / 2; ++e) v[e] = P[din_index<M0>(t, e) * LDP + cc];
-      if constexpr (kRegTw) team_fft_din_to_dout_r<M0, -1, true>(v, t, buf, twz);
-      else team_fft_din_to_dout<M0, -1, true>(v, t, buf, tw_z);
+      team_fft_din_to_dout_r<M0, -1, true>(v, t, buf, twz);
 #pragma unroll
       for (int r = 0; r < EZ; ++r) v[r] = cscale(v[r], tv[r]);
       if (it + 1 < LPZ) load_tcol<EZ, SZ>(tnext, tcol(col + NTZ < M1 ? col + NTZ : 0), t);
-      if constexpr (kRegTw) team_fft_dout_to_din_r<M0, 1, true>(v, t, buf, twz);
-      else team_fft_dout_to_din<M0, 1, true>(v, t, buf, tw_z);
+      team_fft_dout_to_din_r<M0, 1, true>(v, t, buf, twz);
       if (ok) {
 #pragma unroll
         for (int e = 0; e < EZ / 2; ++e) P[din_index<M0>(t, e) * LDP + col] = v[e];

@@ -507,10 +507,9 @@ plane_yz_kernel(PassArgs a) {
     {
       const int team = threadIdx.x / SZ, t = threadIdx.x % SZ;
       float2* buf = xbuf + team * C::TBUF_Z;
-      // this lane's z twiddles, reused by every column (registers when they are few)
-      constexpr bool kRegTw = EZ <= 16;
-      float2 twz[kRegTw ? EZ : 1];
-      if constexpr (kRegTw) load_lane_twiddles<M0>(twz, tw_z, t);
+      // this lane's z twiddles, reused by every column
+      float2 twz[EZ];
+      load_lane_twiddles<M0>(twz, tw_z, t);
       // the diagonal's columns are fetched one iteration ahead of their use
       float tnext[EZ];
       {
@@ -532,12 +531,10 @@ plane_yz_kernel(PassArgs a) {
         float2 v[EZ];
   #pragma unroll
         for (int e = 0; e < EZ / 2; ++e) v[e] = P[pos(din_index<M0>(t, e)) * LDP + colc];
-        if constexpr (kRegTw) team_fft_din_to_dout_r<M0, -1, true>(v, t, buf, twz);
-        else team_fft_din_to_dout<M0, -1, true>(v, t, buf, tw_z);
+        team_fft_din_to_dout_r<M0, -1, true>(v, t, buf, twz);
   #pragma unroll
         for (int r = 0; r < EZ; ++r) v[r] = cscale(v[r], tv[r]);
-        if constexpr (kRegTw) team_fft_dout_to_din_r<M0, 1, true>(v, t, buf, twz);
-        else team_fft_dout_to_din<M0, 1, true>(v, t, buf, tw_z);
+        team_fft_dout_to_din_r<M0, 1, true>(v, t, buf, twz);
         if (ok) {
   #pragma unroll
           for (int e = 0; e < EZ / 2; ++e) P[pos(din_index<M0>(t, e)) * LDP + col] = v[e];
@@ -753,9 +750,8 @@ plane_mod_kernel(PassArgs a) {
   {
     const int team = threadIdx.x / SZ, t = threadIdx.x % SZ;
     float2* buf = xbuf + team * C::TBUF_Z;
-    constexpr bool kRegTw = EZ <= 16;
-    float2 twz[kRegTw ? EZ : 1];
-    if constexpr (kRegTw) load_lane_twiddles<M0>(twz, tw_z, t);
+    float2 twz[EZ];
+    load_lane_twiddles<M0>(twz, tw_z, t);
     auto tcol = [&](int col) { return T + (long long)((K / 2) * col + (q >> 1)) * M0; };
     float tnext[EZ];
     load_tcol<EZ, SZ>(tnext, tcol(team < L ? team : 0), t);
@@ -772,16 +768,14 @@ plane_mod_kernel(PassArgs a) {
       float2 v[EZ];
 #pragma unroll
       for (int e = 0; e < EZ / 2; ++e) v[e] = P[din_index<M0>(t, e) * LDP + colc];
-      if constexpr (kRegTw) team_fft_din_to_dout_r<M0, -1, true>(v, t, buf, twz);
-      else team_fft_din_to_dout<M0, -1, true>(v, t, buf, tw_z);
+      team_fft_din_to_dout_r<M0, -1, true>(v, t, buf, twz);
 #pragma unroll
       for (int r = 0; r < EZ; ++r) v[r] = cscale(v[r], tv[r]);
       if (c0 + C::NTEAMS_Z < L) {
         const int cn = c0 + C::NTEAMS_Z + team;
         load_tcol<EZ, SZ>(tnext, tcol(kFull || cn < L ? cn : 0), t);
       }
-      if constexpr (kRegTw) team_fft_dout_to_din_r<M0, 1, true>(v, t, buf, twz);
-      else team_fft_dout_to_din<M0, 1, true>(v, t, buf, tw_z);
+      team_fft_dout_to_din_r<M0, 1, true>(v, t, buf, twz);
       if (ok) {
 #pragma unroll
         for (int e = 0; e < EZ / 2; ++e) P[din_index<M0>(t, e) * LDP + col] = v[e];
