@@ -315,7 +315,9 @@ const PassLauncher kLaunchC[7][2] = {HB_XROW(8, launch_c),   HB_XROW(16, launch_
 // Planes of powers of two other than 128 x 128 fit one CTA.  128 threads where 256 would leave teams without
 // a row (measured, 128 kx planes of 1 / 16 slots, us, 256 against 128 threads: 16 x 64 4.6 / 33.5
 // against 4.6 / 25.1, 32 x 16 3.3 / 19.1 against 3.3 / 14.6; 32 x 32 3.9 / 24.4 against 4.6 / 23.8,
-// 64 x 64 9.8 / 99.6 against 12.4 / 110).
+// 64 x 64 9.8 / 99.6 against 12.4 / 110).  64 x 128 and 128 x 64 planes hold an SM with one CTA of 256; 512 threads
+// fit, too, and measured 7 to 11 % less per normal operator (64 x 128 x 64, 1 / 16 / 64 coils 33.0 / 348 / 1305 us
+// against 30.9 / 309 / 1199; 128 x 64 x 64 32.2 / 340 / 1318 against 31.0 / 316 / 1228): not taken over yet.
 constexpr int full_threads(int N0, int N1) { return N0 * N1 <= (N0 < 32 ? 1024 : 512) ? 128 : 256; }
 #define HB_BROW(N0)                                                                                          \
   &launch_bfull<N0, 8, full_threads(N0, 8)>, &launch_bfull<N0, 16, full_threads(N0, 16)>,                    \

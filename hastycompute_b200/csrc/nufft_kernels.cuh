@@ -216,9 +216,11 @@ __device__ __forceinline__ int nufft_axis(const NufftGeom& g, float u, float* wt
 
 // ---- type 1 by vector reductions into a zeroed grid.  Used where the tile form
 // (nufft_spread_kernels.cuh) is not: 1-D plans (a sample has only W cells, fewer than a tile's tests
-// would cost) and the point-spread function, whose thousands of equal terms at the centre of a
-// trajectory round differently when they are summed tile by tile (2e-3 of the diagonal's rms at
-// single entries). ----
+// would cost) and the point-spread function.  There thousands of equal terms meet at the centre of a
+// trajectory, and their sum in single precision rounds by its order: by tiles, single entries of a 128^3
+// diagonal move by 2e-3 of its rms.  Whether they move towards the FP64 diagonal (hb_diag_build) entry by
+// entry has not been measured (in the L2 norm they do: 3.6e-6 from it, the reductions 1.5e-5); until then the
+// diagonals stay what they were. ----
 // 1-D, grid [n2][NB], NB = 1 << lgnb: one thread per (sample, transform), transform fastest; blockIdx.y = side
 template <int W>
 __global__ void __launch_bounds__(256) nufft_spread_line_kernel(NufftGeom g, const float4* pts, const float2* vals,
@@ -234,8 +236,8 @@ __global__ void __launch_bounds__(256) nufft_spread_line_kernel(NufftGeom g, con
   for (int m = 0; m < W; ++m) red_add(grid + (wrap(i2 + m, g.n[2]) << lgnb) + (id & ((1 << lgnb) - 1)), cscale(v, w[m]));
 }
 // 3-D, one transform: one thread per sample.  (Eight lanes per sample, each the cells of one x, take 409
-// against 1300 us for 512 k samples on 512^3; but the order of the sums decides how the equal terms at
-// the centre round, and that order moves single entries of the diagonal by 1e-3 of its rms.)
+// against 1300 us for 512 k samples on 512^3, but add in another order: see above; single entries of the
+// diagonal move by 1e-3 of its rms.)
 template <int W>
 __global__ void __launch_bounds__(256) nufft_spread_reductions_kernel(NufftGeom g, const float4* pts, const float2* vals,
                                                                       float2* grid) {
@@ -354,8 +356,13 @@ __device__ __forceinline__ void load_cells(const float2* p, float2* v) {  // V f
 // sample's rows (first y, then z), multiplies by its x weight once, and the group's lanes are added up
 // at the end.  Neighbours in the sorted order run at the same time, so most rows are in L1.
 //
-// Bound: the L1 data path (a request is served 128 bytes a cycle when its lines are aligned, and half
-// of that when every quarter of it straddles two lines).  Measured, 512 k radial samples on 256^3, one
+// Bound: latency and the L1 data path together.  A request is served 128 bytes a cycle when its lines are
+// aligned, and half of that when every quarter of it straddles two lines; at W = 7 and 8 transforms ncu
+// has that path busy 68 % of the cycles (the reads alone would take 0.35 ms of 0.66), a third of the sectors
+// missing L1, and the 24 warps per SM that 80 registers allow waiting for loads for 15 of 21 cycles.
+// From W = 11 on (tolerances below 1e-9) groups of 4 and 8 spill up to 148 bytes a thread, still
+// faster than the form with one thread per value: 64^3 modes, 40 k samples, 8 transforms W = 13 518 us against
+// 1231, W = 16 749 against 1814.  Measured, 512 k radial samples on 256^3, one
 // thread per (sample, transform) -> this form: 8 transforms, W = 7 1175 -> 663 us, W = 6 665 -> 506 us,
 // W = 5 614 -> 360 us, W = 4 328 -> 139 us; 4 transforms, W = 7 609 -> 356 us; 1 transform 253 -> 129 us.
 // One warp per sample with 16-byte loads: 738 us (1081 us without the aligned window). ----

@@ -11,9 +11,11 @@
 // cuts the candidates of such a tile into pieces of at most `cap`, which add into cells
 // zeroed beforehand (nufft_zero_tiles_kernel).
 //
-// Bound: issue (56 % of the slots in ncu, 5.6 M visits of 32 FP32x2 FMAs + about 50 other
-// instructions) with 20 warps per SM.  The reduction form it replaces issued W^3 vector
-// reductions per sample and transform.  Measured at W = 7, 512 k radial samples on a 256^3 grid:
+// Bound: the FP32 pipe, 59 % of its cycles busy in ncu (an FP32x2 FMA takes it for two), issue 56 % (5.6 M
+// visits of 32 packed FMAs + about 50 other instructions), at the 15 warps per SM that are there on average
+// of the 20 that fit: one-warp CTAs come and go, and the phases of a batch (collecting, weights, visits) of a
+// warp depend on one another.  The reduction form it replaces issued W^3 vector reductions per sample and
+// transform.  Measured at W = 7, 512 k radial samples on a 256^3 grid:
 // 8 transforms 751 us + 24 us (gathering the values) + 9 us (zeroing) against 2145 + 172 us,
 // 4: 484 us, 1: 307 us against 916 us.  Choices, 8 transforms: one warp per CTA (two: 1192 us, a
 // CTA waits for its slower warp; four: 1140 us), 96 registers (128: 825 us), long pieces first

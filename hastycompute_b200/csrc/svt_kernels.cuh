@@ -26,8 +26,9 @@
 // against 19.5 ms, 8 columns 0.74 against 2.53 ms.  On the way: rotations of a round in parallel
 // 3.26 ms, staging ahead without divisions 2.93 ms, single-precision staging and unpaired W 2.65 ms,
 // rows last to first 2.51 ms, the real products of W summed apart (a sum of 40 terms in one chain
-// rounds worse than the 20 complex products it stands for) 2.65 ms.  G by FP64 mma.sync m8n8k4 straight from global memory: 3.26 ms; 96
-// registers for five CTAs per SM 3.65 ms, 168 for three 2.87 ms.
+// rounds worse than the 20 complex products it stands for) 2.65 ms.  G by FP64 mma.sync m8n8k4 straight from global memory: 3.26 ms; At
+// 20 columns 96 registers for five CTAs per SM 3.65 ms, 168 for three 2.87 ms; the bound of 128 holds for every
+// column count, and from 21 columns on it spills 100 to 412 bytes a thread (other bounds were not measured there).
 #pragma once
 
 #include "common.cuh"

@@ -12,9 +12,8 @@ Mirrors the reference's NUFFT front end:
   the k-space manipulators of ``batch_sense.cpp:452-486``; ``sense_adjoint`` gives the CG
   right-hand side ``b = sum_c conj(S_c) NUFFT^H(y_c)``.
 
-Only 3-D transforms are compiled (the path's images are 3-D); ``2 * N`` per axis must be
-one of 8, 16, 32, 64, 128, 256, 512, 96, 160, 192, 320.  Every call runs the sm_100a kernels of
-``libhasty_b200.so``; there is no fallback.
+1-D, 2-D and 3-D plans; ``2 * N`` per axis must be one of 8, 16, 32, 64, 128, 256, 512, 96, 160,
+192, 320.  Every call runs the sm_100a kernels of ``libhasty_b200.so``; there is no fallback.
 """
 from __future__ import annotations
 
