@@ -376,6 +376,19 @@ int create_plan(hb_nufft** out, int64_t nz, int64_t ny, int64_t nx, const float*
     g.bin[a] = g.dim == 3 && a < 2 && tiles ? 4 : 8;  // every fine-grid length is a multiple of 8
     g.nb[a] = g.n[a] / g.bin[a];
   }
+  // A tile's candidates are counted in 32 bits, and on a grid smaller than its neighbourhood it meets a bin
+  // once per period.
+  if (tiles && g.dim > 1) {
+    long long most = nsamples;
+    for (int a = 3 - g.dim; a < 3; ++a) {
+      const int T = g.dim == 3 ? (a < 2 ? SpreadTile<3>::T0 : SpreadTile<3>::T2) : a == 1 ? SpreadTile<2>::T1 : SpreadTile<2>::T2;
+      const int h = (g.w + 1) / 2, met = ((T < g.n[a] ? T : g.n[a]) - 1 + h) / g.bin[a] + (h + g.bin[a] - 1) / g.bin[a] + 1;
+      most *= (met + g.nb[a] - 1) / g.nb[a];
+    }
+    if (most > 0x7fffffffLL - 4096)
+      return fail(HB_ERR_UNSUPPORTED, "hb_nufft_create: too many samples for a grid of " + std::to_string(g.n[0]) + " x " +
+                                          std::to_string(g.n[1]) + " x " + std::to_string(g.n[2]) + " cells");
+  }
   DeviceGuard dg(device);
   if (!dg.ok) return fail(HB_ERR_CUDA, "hb_nufft_create: cannot select device");
   cudaStream_t st = (cudaStream_t)stream;

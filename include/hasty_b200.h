@@ -307,6 +307,7 @@ int hb_toeplitz_apply_noalloc(int64_t nz, int64_t ny, int64_t nx, const void* in
  * Method: exponential-of-semicircle gridding kernel with upsampling 2 (the published
  * method of finufft); kernel width w = ceil(log10(1/tol)) + 1 fine-grid cells.
  * 2*N_a must be one of 8, 16, 32, 64, 128, 256, 512, 96, 160, 192, 320 and >= 2w.
+ * nsamples < 2^31 - 4096, on 2-D and 3-D grids of fewer than 32 cells along an axis divided by up to 12.
  * The order of a bin's samples and the sums of crowded tiles come from atomics, so the last bits
  * of type 1 vary from plan to plan and from run to run.
  * Lower dimensions (the reference's 1-D and 2-D plans, nufft.ixx:72-160): nz = 1 makes a

@@ -46,6 +46,16 @@ def test_sizes_and_errors_without_gpu():
     assert lib.hb_normal_workspace_bytes(None, 1, 1) == 0
 
 
+def test_nufft_sample_counts_beyond_32_bits_are_refused():
+    """A spreading tile counts its candidate samples in 32 bits and meets each bin of a small grid several
+    times (4^3 modes at w = 4: 12 times, 16 x 16 at w = 7: once): refused on the host before anything is touched."""
+    lib = capi.load()
+    h, some = ctypes.c_void_p(), ctypes.c_void_p(256)
+    for modes, tol, k in (((4, 4, 4), 1e-3, 200_000_000), ((1, 4, 4), 1e-3, 300_000_000), ((16, 16, 16), 1e-6, 2**31 - 100)):
+        assert lib.hb_nufft_create(ctypes.byref(h), *modes, some, k, tol, 1, 0, None) == capi.HB_ERR_UNSUPPORTED
+        assert b"too many samples" in lib.hb_last_error()
+
+
 def test_check_raises_with_message():
     lib = capi.load()
     code = lib.hb_plan_create(None, 16, 16, 16, 0)
